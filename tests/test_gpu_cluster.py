@@ -1,0 +1,66 @@
+"""Iterations of a small LP on one thread-block cluster against the two fused launches per
+iteration (the path that per-kernel timing, level 2, takes). Both sum every row in the same
+order and use the same elementwise arithmetic, so their iterates are equal bit for bit; where
+every row has at most 32 entries they equal the oracle's serial sums too (tests/test_gpu_parity.py
+runs config 0 there). The shapes are the edges: one entry, empty rows and columns, rows of 32 /
+33 / 256 / 257 entries (owner, warp tree, streamed), fewer chunks than CTAs, chunk counts above
+the warps of a CTA, and sizes just inside and outside the cluster's shared memory."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def lp(instances, m, n, lens, seed=0):
+    """Row i has lens[i % len(lens)] entries in distinct random columns."""
+    rng = np.random.default_rng(seed)
+    deg = np.minimum(np.resize(np.asarray(lens), m), n)
+    row = np.repeat(np.arange(m), deg)
+    col = np.concatenate([rng.choice(n, size=k, replace=False) for k in deg] or [np.zeros(0, int)])
+    val = rng.standard_normal(col.shape[0])
+    ptr, idx, val = instances._csr_from_entries(m, row, col, val)
+    return instances._finish_lp(rng, m, n, ptr, idx, val)
+
+
+def steps(inst):
+    rows = np.repeat(np.arange(inst["m"]), np.diff(inst["ptr"]))
+    rm = np.bincount(rows, np.abs(inst["val"]), inst["m"])
+    cm = np.bincount(inst["idx"], np.abs(inst["val"]), inst["n"])
+    return 0.9 / (1 + cm), 0.9 / (1 + rm)
+
+
+SHAPES = [
+    (1, 1, [1]), (3, 2, [0, 2, 1]), (40, 31, [0, 1, 31]), (257, 300, [32, 33, 0]), (64, 700, [256, 257, 300, 5]),
+    (1200, 900, [1, 40, 3]), (15, 6000, [9]), (6000, 15, [2]), (4000, 9000, [7, 3, 11]), (9000, 17500, [4]),
+    (9000, 20500, [4]),
+]
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("entry", ["lp", "with_dual", "diagonal"])
+def test_cluster_equals_launches(engine, instances, shape, entry):
+    inst = lp(instances, *shape)
+    ps, ds = steps(inst)
+    kw = dict(max_iterations=47, check_every=19, theta=0.5 if entry == "with_dual" else 1.0, tolerance=1e-13)
+    extra = {}
+    if entry == "with_dual":
+        extra = dict(primal_steps=ps, dual_steps=ds, want_dual=True)
+    else:
+        norm = np.sqrt(max((0.9 / ps - 1).max() * (0.9 / ds - 1).max(), 1e-3))
+        kw.update(tau=0.9 / norm, sigma=0.9 / norm)
+    if entry == "diagonal":
+        extra = dict(qdiag=np.random.default_rng(3).uniform(0, 2, inst["n"]))
+    A = engine.Matrix.from_instance(inst)
+    got = []
+    for level in (0, 2):
+        engine.set_timing(level)
+        try:
+            rc, x, y, r = engine.pdhg(A, inst, engine.settings(**kw), **extra)
+        finally:
+            engine.set_timing(0)
+        assert rc == 0
+        got.append((x, y, r))
+    assert np.array_equal(got[0][0], got[1][0])
+    if got[0][1] is not None:
+        assert np.array_equal(got[0][1], got[1][1])
+    assert got[0][2] == got[1][2]

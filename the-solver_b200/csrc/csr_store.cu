@@ -5,7 +5,7 @@
 // Reference behaviour followed: cuda/src/sankhya_cuda.cu:10-21 (error text),
 // :116-152 (validation order and messages, destroy-before-create, zeroed
 // handle on failure), :154-163 (destroy).
-#include "engine.cuh"
+#include "cluster.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -56,6 +56,47 @@ std::vector<int> build_tiles(int rows, const int* ptr) {
     tiles.push_back(rows);
     tiles.push_back(ptr[rows]);
     return tiles;
+}
+
+Share largest_share(const std::vector<int>& tiles) {
+    Share s;
+    const int nt = static_cast<int>(tiles.size()) / 2 - 1;
+    s.chunks = (nt + cluster::kClusterCtas - 1) / cluster::kClusterCtas;
+    for (int c = 0; c < cluster::kClusterCtas; ++c) {
+        const int t0 = std::min(nt, c * s.chunks), t1 = std::min(nt, (c + 1) * s.chunks);
+        s.rows = std::max(s.rows, tiles[2 * t1] - tiles[2 * t0]);
+        s.nnz = std::max(s.nnz, tiles[2 * t1 + 1] - tiles[2 * t0 + 1]);
+    }
+    return s;
+}
+
+bool cluster::available(const void* kernel) {
+    struct Entry { const void* k; int device; bool ok; };
+    static std::mutex mu;
+    static std::vector<Entry> cache;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Entry& e : cache)
+        if (e.k == kernel && e.device == device) return e.ok;
+    int clusters = 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kClusterCtas);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = kMaxSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kClusterCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const bool ok =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) == cudaSuccess &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+    if (!ok) (void)cudaGetLastError();
+    cache.push_back({kernel, device, ok});
+    return ok;
 }
 
 // ------------------------------------------------------------------ plans
@@ -131,6 +172,7 @@ int make_plan(const SankhyaCudaCSR* m, const int* h_ptr, const int* h_idx, const
     plan->a.val = a_val;
     plan->a.ntiles = static_cast<int>(tiles_a.size()) / 2 - 1;
     plan->a.tile = reinterpret_cast<const int2*>(plan->d_tile_a);
+    plan->a.share = largest_share(tiles_a);
     plan->at.rows = cols;
     plan->at.cols = rows;
     plan->at.nnz = nnz;
@@ -139,6 +181,7 @@ int make_plan(const SankhyaCudaCSR* m, const int* h_ptr, const int* h_idx, const
     plan->at.val = plan->d_at_val;
     plan->at.ntiles = static_cast<int>(tiles_at.size()) / 2 - 1;
     plan->at.tile = reinterpret_cast<const int2*>(plan->d_tile_at);
+    plan->at.share = largest_share(tiles_at);
     *out = std::move(plan);
     return 0;
 }

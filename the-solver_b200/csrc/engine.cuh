@@ -54,11 +54,19 @@ std::vector<int> build_tiles(int rows, const int* row_offsets);
 int device_transpose(int rows, int cols, int nnz, const int* ptr, const int* idx, const double* val, int* tptr,
                      int* tidx, double* tval, cudaStream_t stream);
 
+// Largest part of a CSR any CTA holds when the chunks of its schedule are split
+// evenly and in order over the CTAs of one cluster (cluster.cuh); chunks 0: unknown.
+struct Share {
+    int rows = 0, nnz = 0, chunks = 0;
+};
+Share largest_share(const std::vector<int>& tiles);
+
 // A CSR with its warp-chunk schedule; T is the value type (double, or float
 // for the FP32 inner iterations of the refined PDLP).
 template <class T>
 struct TileCsrT {
     int rows = 0, cols = 0, nnz = 0, ntiles = 0;
+    Share share;
     const int* ptr = nullptr;
     const int* idx = nullptr;
     const T* val = nullptr;
@@ -67,7 +75,7 @@ struct TileCsrT {
     template <class U>
     TileCsrT<U> with_values(const U* v) const {
         TileCsrT<U> o;
-        o.rows = rows; o.cols = cols; o.nnz = nnz; o.ntiles = ntiles;
+        o.rows = rows; o.cols = cols; o.nnz = nnz; o.ntiles = ntiles; o.share = share;
         o.ptr = ptr; o.idx = idx; o.val = v; o.tile = tile;
         return o;
     }
@@ -133,10 +141,12 @@ __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a,
 __device__ __forceinline__ float dadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float dmul(float a, float b) { return __fmul_rn(a, b); }
 
-// cuda/src/sankhya_cuda_lp.cu:13-17: only IEEE infinities are absent bounds.
+// cuda/src/sankhya_cuda_lp.cu:13-17: only IEEE infinities are absent bounds. The bounds
+// were validated (no lower bound of +inf, no upper one of -inf), so an infinite one never
+// compares true and needs no test of its own.
 __device__ __forceinline__ double box_ieee(double v, double lo, double hi) {
-    if (!isinf(lo) && v < lo) v = lo;
-    if (!isinf(hi) && v > hi) v = hi;
+    if (v < lo) v = lo;
+    if (v > hi) v = hi;
     return v;
 }
 // c/src/sk_solve.c:18-24: the 1e30 sentinel (SK_INFINITY) marks absent bounds.

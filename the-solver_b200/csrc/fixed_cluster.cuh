@@ -1,0 +1,147 @@
+// Fixed-step PDHG iterations of a small LP (or diagonal QP) on one cluster.
+//
+// Measured on a B200 at 1,965 MHz, us per iteration, two graph launches -> this kernel:
+// 200 x 300 (900 nonzeros) 5.5 -> 1.5; 1,000 x 2,500 (12,500) 7.0 -> 2.2; 2,000 x 5,000
+// (25,000) 7.7 -> 2.85; 4,000 x 9,000 (54,000) 7.8 -> 5.2. Of the 5,400 cycles of an
+// iteration at 2,000 x 5,000, the two exchanges take 1,500 and 1,400 (580 each of latency,
+// the rest 12.8 bytes per cycle), the rows' sums and epilogues 1,500 and the columns' 1,000:
+// a serial chain of adds (12 cycles each), one divide (137) and shared-memory latencies, with
+// the 16 SMs' shared-memory bandwidth next. Above the size that fits, the launches win anyway.
+#pragma once
+
+#include "cluster.cuh"
+#include "fixed_epi.cuh"
+
+namespace b200 {
+
+constexpr int kMaxClusterIterations = 4096;  // per launch: a few milliseconds
+
+struct FixedClusterArgs {
+    TileCsr A, AT;
+    const double *c, *cl, *cu, *tauv, *qdiag;  // tauv / sigv / qdiag may be null
+    const double *rl, *ru, *sigv;
+    double tau, sigma, theta;
+    const double *x_in, *y_in;
+    double *x_out, *y_out, *x_bar;  // x_bar: in and out
+    double* part;                   // SK: max |y_new - y| of the last iteration, one per CTA
+    int iterations;
+    unsigned int* fail;             // set when a wait gave up
+};
+
+// Shared memory of one CTA; 0 when the problem has no rows or no columns.
+inline size_t fixed_cluster_smem(const TileCsr& A, const TileCsr& AT) {
+    if (A.ntiles == 0 || AT.ntiles == 0) return 0;
+    return cluster::kClusterWarps * cluster::kProducts * 8ull + cluster::slice_bytes(A) + cluster::slice_bytes(AT) + cluster::packed_bytes<double>(A) +
+           cluster::packed_bytes<double>(AT) + cluster::send_bytes(A.share) + cluster::send_bytes(AT.share) +
+           4 * cluster::align16(8ull * A.share.rows) + 7 * cluster::align16(8ull * AT.share.rows);
+}
+
+// ONE: no CTA has more chunks of A or of A' than warps, so every chunk stays in its warp's
+// registers for the whole launch.
+template <bool SK, bool ONE>
+__global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(const __grid_constant__ FixedClusterArgs a) {
+    using namespace cluster;
+    extern __shared__ __align__(16) char smem[];
+    __shared__ double red[kClusterWarps];
+    const unsigned rank = cta_rank();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    Arena mem{smem};
+    double* sp = mem.take<double>(kClusterWarps * kProducts) + warp * kProducts;
+    if (lane < 2) sp[kChunkNnz + lane] = -0.0;
+    Slice<double> R, Q;       // rows of A, rows of A' (columns)
+    Packed<double> xv, yv;    // x_bar as R gathers it, y as Q gathers it
+    SendList xs_out, ys_out;
+    load_part(a.A, rank, mem, &R, &xv);
+    load_part(a.AT, rank, mem, &Q, &yv);
+    double* y = mem.take<double>(a.A.share.rows);    // own elements
+    double* x = mem.take<double>(a.AT.share.rows);
+    double* xb = mem.take<double>(a.AT.share.rows);
+    // the steps' constants too: a wait that acquires drops the SM's cached global lines
+    double* rl = mem.take<double>(a.A.share.rows);
+    double* ru = mem.take<double>(a.A.share.rows);
+    double* sig = mem.take<double>(a.A.share.rows);
+    double* c = mem.take<double>(a.AT.share.rows);
+    double* cl = mem.take<double>(a.AT.share.rows);
+    double* cu = mem.take<double>(a.AT.share.rows);
+    double* tau = mem.take<double>(a.AT.share.rows);
+    fill_packed(a.A, xv, a.x_bar);
+    for (int r = threadIdx.x; r < R.rows; r += blockDim.x) {
+        const int i = R.row0 + r;
+        y[r] = a.y_in[i];
+        rl[r] = a.rl[i];
+        ru[r] = a.ru[i];
+        sig[r] = a.sigv ? a.sigv[i] : a.sigma;
+    }
+    for (int r = threadIdx.x; r < Q.rows; r += blockDim.x) {
+        const int j = Q.row0 + r;
+        x[r] = a.x_in[j];
+        c[r] = a.c[j];
+        cl[r] = a.cl[j];
+        cu[r] = a.cu[j];
+        tau[r] = a.tauv ? a.tauv[j] : a.tau;
+    }
+    cluster_sync();
+    make_sends(Q.row0, Q.rows, xv, a.AT.share, mem, &xs_out);
+    make_sends(R.row0, R.rows, yv, a.A.share, mem, &ys_out);
+    cluster_sync();
+    Chunk<double, double> rc, qc;
+    if (ONE && warp < R.chunks) rc.load(R, warp, xv.v);
+    if (ONE && warp < Q.chunks) qc.load(Q, warp, yv.v);
+    double change = 0.0;
+    bool ok = true;
+    for (int it = 0; it < a.iterations && ok; ++it) {
+        const bool last = it + 1 == a.iterations;
+        for (int j = warp; j < R.chunks; j += kClusterWarps) {
+            if (!ONE) rc.load(R, j, xv.v);
+            const double act = rc.sum(R, xv.v, sp);
+            if (rc.owns) {
+                const int r = rc.r;
+                const double old = y[r];
+                const double yn = SK ? dual_step_sk(old, act, sig[r], rl[r], ru[r])
+                                     : dual_step_cuda(old, act, sig[r], rl[r], ru[r]);
+                y[r] = yn;
+                if (SK && last) change = fmax(change, fabs(dsub(yn, old)));
+            }
+        }
+        ok = exchange(ys_out, y, yv);
+        for (int j = warp; j < Q.chunks; j += kClusterWarps) {
+            if (!ONE) qc.load(Q, j, yv.v);
+            const double g = qc.sum(Q, yv.v, sp);
+            if (qc.owns) {
+                const int r = qc.r;
+                const double old = x[r], qd = a.qdiag ? __ldg(a.qdiag + Q.row0 + r) : 0.0;
+                const double xn =
+                    SK ? primal_step_sk(old, g, c[r], tau[r], cl[r], cu[r], a.qdiag != nullptr, qd, 0.0)
+                       : primal_step_cuda(old, g, c[r], tau[r], cl[r], cu[r], a.qdiag != nullptr, qd, 0.0);
+                x[r] = xn;
+                xb[r] = SK ? dsub(dmul(2.0, xn), old) : dadd(xn, dmul(a.theta, dsub(xn, old)));
+            }
+        }
+        ok = exchange(xs_out, xb, xv) && ok;
+    }
+    if (!ok && threadIdx.x == 0) *a.fail = 1u;
+    cluster_sync();
+    for (int j = threadIdx.x; j < Q.rows; j += blockDim.x) {
+        a.x_out[Q.row0 + j] = x[j];
+        a.x_bar[Q.row0 + j] = xb[j];
+    }
+    for (int i = threadIdx.x; i < R.rows; i += blockDim.x) a.y_out[R.row0 + i] = y[i];
+    if (SK) {
+        for (int o = 16; o > 0; o >>= 1) change = fmax(change, __shfl_xor_sync(0xffffffffu, change, o));
+        if (lane == 0) red[warp] = change;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < kClusterWarps; ++k) change = fmax(change, red[k]);
+            a.part[rank] = change;
+        }
+    }
+}
+
+using FixedClusterKernel = void (*)(FixedClusterArgs);
+inline FixedClusterKernel fixed_cluster_kernel(const TileCsr& A, const TileCsr& AT, bool sk) {
+    const bool one = A.share.chunks <= cluster::kClusterWarps && AT.share.chunks <= cluster::kClusterWarps;
+    return sk ? (one ? &k_fixed_cluster<true, true> : &k_fixed_cluster<true, false>)
+              : (one ? &k_fixed_cluster<false, true> : &k_fixed_cluster<false, false>);
+}
+
+}  // namespace b200

@@ -6,6 +6,30 @@
 
 namespace b200 {
 
+// cuda/src/sankhya_cuda_lp.cu:26-34, :36-52
+__device__ __forceinline__ double dual_step_cuda(double y, double act, double s, double lo, double hi) {
+    const double trial = dadd(y, dmul(s, act));
+    return dsub(trial, dmul(s, box_ieee(ddiv(trial, s), lo, hi)));
+}
+__device__ __forceinline__ double primal_step_cuda(double x, double g, double c, double t, double lo, double hi,
+                                                   bool diagonal, double curvature, double qg) {
+    double trial = dsub(x, dmul(t, dadd(dadd(c, g), qg)));
+    if (diagonal) trial = ddiv(trial, dadd(1.0, dmul(t, curvature)));  // without a diagonal: / 1, exactly
+    return box_ieee(trial, lo, hi);
+}
+
+// c/src/sk_solve.c:901-906, :908-923
+__device__ __forceinline__ double dual_step_sk(double y, double act, double s, double lo, double hi) {
+    const double trial = dadd(y, dmul(s, act));
+    return dsub(trial, dmul(s, box_sk(ddiv(trial, s), lo, hi)));
+}
+__device__ __forceinline__ double primal_step_sk(double x, double g, double c, double t, double lo, double hi,
+                                                 bool diagonal, double qd, double qx) {
+    const double xn = diagonal ? ddiv(dsub(x, dmul(t, dadd(c, g))), dadd(1.0, dmul(t, qd)))
+                               : dsub(x, dmul(t, dadd(dadd(c, qx), g)));
+    return box_sk(xn, lo, hi);
+}
+
 // cuda/src/sankhya_cuda_lp.cu:26-34
 struct DualCudaEpi {
     const double* __restrict__ y;
@@ -20,8 +44,7 @@ struct DualCudaEpi {
     };
     __device__ __forceinline__ Row load(int i) const { return Row{y[i], rl[i], ru[i], sig ? sig[i] : sigma}; }
     __device__ __forceinline__ void store(int i, double act, const Row& r, Acc&) const {
-        const double trial = dadd(r.y, dmul(r.s, act));
-        y_new[i] = dsub(trial, dmul(r.s, box_ieee(ddiv(trial, r.s), r.lo, r.hi)));
+        y_new[i] = dual_step_cuda(r.y, act, r.s, r.lo, r.hi);
     }
     __device__ __forceinline__ void finish(Acc&, double*) const {}
 };
@@ -46,8 +69,7 @@ struct PrimalCudaEpi {
         return Row{x[j], c[j], tauv ? tauv[j] : tau, cl[j], cu[j], qdiag ? qdiag[j] : 0.0, qgrad ? qgrad[j] : 0.0};
     }
     __device__ __forceinline__ void store(int j, double g, const Row& r, Acc&) const {
-        const double trial = ddiv(dsub(r.x, dmul(r.t, dadd(dadd(r.c, g), r.qg))), dadd(1.0, dmul(r.t, r.curvature)));
-        const double next = box_ieee(trial, r.lo, r.hi);
+        const double next = primal_step_cuda(r.x, g, r.c, r.t, r.lo, r.hi, qdiag != nullptr, r.curvature, r.qg);
         x_new[j] = next;
         x_bar[j] = dadd(next, dmul(theta, dsub(next, r.x)));
     }

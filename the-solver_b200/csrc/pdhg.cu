@@ -16,6 +16,7 @@
 //   SemSk    the CPU loop of c/src/sk_solve.c:849-954 (1e30 sentinel bounds,
 //            x_bar = 2 x_new - x_old, mass-based steps, 20-iteration checks)
 #include "engine.cuh"
+#include "fixed_cluster.cuh"
 #include "fixed_epi.cuh"
 
 #include <algorithm>
@@ -43,8 +44,7 @@ struct DualSkEpi {
     };
     __device__ __forceinline__ Row load(int i) const { return Row{y[i], rl[i], ru[i], sig[i]}; }
     __device__ __forceinline__ void store(int i, double act, const Row& r, Acc& acc) const {
-        const double trial = dadd(r.y, dmul(r.s, act));
-        const double yn = dsub(trial, dmul(r.s, box_sk(ddiv(trial, r.s), r.lo, r.hi)));
+        const double yn = dual_step_sk(r.y, act, r.s, r.lo, r.hi);
         y_new[i] = yn;
         acc.max(0, fabs(dsub(yn, r.y)));
     }
@@ -70,13 +70,7 @@ struct PrimalSkEpi {
         return Row{x[j], c[j], tauv[j], cl[j], cu[j], qdiag ? qdiag[j] : 0.0, qx ? qx[j] : 0.0};
     }
     __device__ __forceinline__ void store(int j, double g, const Row& r, Acc&) const {
-        double xn;
-        if (qdiag) {
-            xn = ddiv(dsub(r.x, dmul(r.t, dadd(r.c, g))), dadd(1.0, dmul(r.t, r.qd)));
-        } else {
-            xn = dsub(r.x, dmul(r.t, dadd(dadd(r.c, r.qx), g)));
-        }
-        xn = box_sk(xn, r.lo, r.hi);
+        const double xn = primal_step_sk(r.x, g, r.c, r.t, r.lo, r.hi, qdiag != nullptr, r.qd, r.qx);
         x_new[j] = xn;
         x_bar[j] = dsub(dmul(2.0, xn), r.x);
     }
@@ -202,7 +196,7 @@ struct Workspace {
     double *x[2] = {nullptr, nullptr}, *y[2] = {nullptr, nullptr};
     double *x_bar = nullptr, *qx = nullptr, *x_prev = nullptr, *act = nullptr;
     double *part_a = nullptr, *part_b = nullptr, *part_c = nullptr, *out = nullptr;
-    unsigned int* flags = nullptr;
+    unsigned int* flags = nullptr;  // right behind `out`: [0] input checks, [1] a cluster wait gave up
     int n = 0, m = 0;
 
     int allocate(int n_, int m_, int max_grid) {
@@ -235,6 +229,9 @@ static double* pinned_out() {
     if (!h.p && cudaMallocHost(reinterpret_cast<void**>(&h.p), 64 * sizeof(double)) != cudaSuccess) h.p = nullptr;
     return h.p;
 }
+
+// A checkpoint's results come back with the flags behind them (33 doubles from Workspace::out).
+static bool cluster_gave_up(const double* host_flags) { return reinterpret_cast<const unsigned int*>(host_flags)[1] != 0; }
 
 // Captured iteration graphs, keyed by everything a captured launch bakes in.
 struct GraphKey {
@@ -280,8 +277,18 @@ struct Solver {
     int launches = 0;
     GraphMap local_graphs;
     GraphMap* graphs = &local_graphs;
+    FixedClusterKernel cluster_kernel = nullptr;
+    size_t cluster_smem = 0;  // > 0: the iterations run on one cluster
+    int dual_blocks = 0;      // partials the last dual step left in part_c
 
     void setup_grids() {
+        // Rule: the LP (no explicit Hessian) fits the shared memory of one cluster, which it
+        // does up to about 100,000 nonzeros. Below that line the cluster is the faster one
+        // throughout (fixed_cluster.cuh has the figures).
+        const size_t need = Q ? 0 : fixed_cluster_smem(*A, *AT);
+        cluster_kernel = fixed_cluster_kernel(*A, *AT, sem == Sem::Sk);
+        cluster_smem = need > 0 && need <= cluster::kMaxSmem &&
+                               cluster::available(reinterpret_cast<const void*>(cluster_kernel)) ? need : 0;
         if (sem == Sem::Cuda) {
             grid_dual = tiled_grid<DualCudaEpi>(*A);
             grid_primal = tiled_grid<PrimalCudaEpi>(*AT);
@@ -290,6 +297,24 @@ struct Solver {
             grid_primal = tiled_grid<PrimalSkEpi>(*AT);
         }
         if (Q) grid_q = tiled_grid<StoreEpi>(*Q);
+        dual_blocks = A->ntiles ? grid_dual : 0;
+    }
+
+    // k iterations as cluster launches of up to kMaxClusterIterations.
+    int run_cluster(int k) {
+        while (k > 0) {
+            const int steps = std::min(k, kMaxClusterIterations), nx = cur ^ 1;
+            const FixedClusterArgs a{*A, *AT, w->c, w->cl, w->cu, has_steps ? w->tauv : nullptr,
+                                     has_qdiag ? w->qdiag : nullptr, w->rl, w->ru, has_steps ? w->sigv : nullptr,
+                                     tau, sigma, theta, w->x[cur], w->y[cur], w->x[nx], w->y[nx], w->x_bar, w->part_c,
+                                     steps, w->flags + 1};
+            B200_TRY(cluster::launch(cluster_kernel, a, cluster_smem, stream), "cluster launch");
+            ++launches;
+            cur = nx;
+            k -= steps;
+        }
+        dual_blocks = cluster::kClusterCtas;
+        return 0;
     }
 
     // One PDHG iteration from buffer cur into buffer cur^1.
@@ -346,6 +371,7 @@ struct Solver {
             for (auto& e : ev) cudaEventDestroy(e);
             return 0;
         }
+        if (cluster_smem) return run_cluster(k);
         while (k > 0) {
             const int chunk = k > 64 ? 64 : k;
             const GraphKey key{stream, Q, has_qdiag ? 1 : 0, has_steps ? 1 : 0, chunk, cur, static_cast<int>(sem),
@@ -476,7 +502,7 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
         B200_TRY(cudaMemsetAsync(w->y[0], 0, mb, stream), "zero y");
     }
     if (cols > 0) k_init_box_ieee<<<elem_grid(cols), kThreads, 0, stream>>>(cols, w->cl, w->cu, w->x[0], w->x_bar);
-    B200_TRY(cudaMemsetAsync(w->flags, 0, sizeof(unsigned int), stream), "clear flags");
+    B200_TRY(cudaMemsetAsync(w->flags, 0, 2 * sizeof(unsigned int), stream), "clear flags");
     k_validate_fixed<<<elem_grid(std::max(rows, cols)), kThreads, 0, stream>>>(
         cols, rows, w->c, w->cl, w->cu, w->rl, w->ru, pstep ? w->tauv : nullptr, dstep ? w->sigv : nullptr,
         qdiag ? w->qdiag : nullptr, w->flags);
@@ -545,8 +571,9 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
         k_combine<5, 0u><<<1, kThreads, 0, stream>>>(w->part_a, nb_rows, w->out);
         k_combine<7, 1u << 1><<<1, kThreads, 0, stream>>>(w->part_b, nb_cols, w->out + 8);
         sv.launches += 4 + (sv.Q ? 1 : 0);
-        B200_TRY(cudaMemcpyAsync(host, w->out, 16 * sizeof(double), cudaMemcpyDeviceToHost, stream), "read checkpoint");
+        B200_TRY(cudaMemcpyAsync(host, w->out, 33 * sizeof(double), cudaMemcpyDeviceToHost, stream), "read checkpoint");
         B200_TRY(cudaStreamSynchronize(stream), "checkpoint");
+        if (cluster_gave_up(host + 32)) return fail_msg("a wait inside the iteration kernel gave up");
         ts.last.checkpoint_ms += t_chk.stop();
         ts.last.checkpoints += 1;
         const double nonfinite = std::max(host[0], host[8]);
@@ -624,10 +651,10 @@ struct OwnedPair {
         std::vector<int> ta = build_tiles(rows, rp.data());
         if (tiles.alloc(ta.size() * 4, "cudaMalloc tiles")) return -1;
         B200_TRY(cudaMemcpy(tiles.p, ta.data(), tiles.bytes, cudaMemcpyHostToDevice), "upload tiles");
-        a = TileCsr{rows, cols, nnz, static_cast<int>(ta.size()) / 2 - 1, ptr.as<int>(), idx.as<int>(),
-                    val.as<double>(), tiles.as<int2>()};
-        at = TileCsr{cols, rows, nnz, static_cast<int>(tb.size()) / 2 - 1, tptr.as<int>(), tidx.as<int>(),
-                     tval.as<double>(), ttiles.as<int2>()};
+        a = TileCsr{rows, cols, nnz, static_cast<int>(ta.size()) / 2 - 1, largest_share(ta), ptr.as<int>(),
+                    idx.as<int>(), val.as<double>(), tiles.as<int2>()};
+        at = TileCsr{cols, rows, nnz, static_cast<int>(tb.size()) / 2 - 1, largest_share(tb), tptr.as<int>(),
+                     tidx.as<int>(), tval.as<double>(), ttiles.as<int2>()};
         return 0;
     }
 };
@@ -705,6 +732,7 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
         B200_TRY(cudaMemcpyAsync(w.sigv, sigv.data(), mb, cudaMemcpyHostToDevice, stream), "upload sigma");
         B200_TRY(cudaMemsetAsync(w.y[0], 0, mb, stream), "zero y");
     }
+    B200_TRY(cudaMemsetAsync(w.flags, 0, 2 * sizeof(unsigned int), stream), "clear flags");
     B200_TRY(cudaGetLastError(), "init launch");
 
     Solver sv;
@@ -717,7 +745,6 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
     sv.has_qdiag = q && diagonal;
     sv.has_steps = true;
     sv.setup_grids();
-    const int nb_dual = ap.a.ntiles ? sv.grid_dual : 0;
     const int grid_rows = tiled_grid<CheckRowsSkEpi>(ap.a);
     const int grid_cols = tiled_grid<CheckColsSkEpi>(ap.at);
     const int nb_rows = ap.a.ntiles ? grid_rows : 0, nb_cols = ap.at.ntiles ? grid_cols : 0;
@@ -738,7 +765,7 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
         it = next;
         const int cx = sv.cur;
         // dual step of the last iteration (written by every dual launch)
-        k_combine<1, 0u><<<1, kThreads, 0, stream>>>(w.part_c, nb_dual, w.out + 24);
+        k_combine<1, 0u><<<1, kThreads, 0, stream>>>(w.part_c, sv.dual_blocks, w.out + 24);
         if (time_limit > 0.0 && now_seconds() - start >= time_limit) {
             activity_is_ax = false;
             break;
@@ -755,8 +782,9 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
             if (n) k_sk_step_scale<<<grid_step, kThreads, 0, stream>>>(w.x[cx], w.x_bar, n, w.part_b);
             k_combine<2, 0u><<<1, kThreads, 0, stream>>>(w.part_b, n ? grid_step : 0, w.out + 16);
         }
-        B200_TRY(cudaMemcpyAsync(host, w.out, 32 * sizeof(double), cudaMemcpyDeviceToHost, stream), "read checkpoint");
+        B200_TRY(cudaMemcpyAsync(host, w.out, 33 * sizeof(double), cudaMemcpyDeviceToHost, stream), "read checkpoint");
         B200_TRY(cudaStreamSynchronize(stream), "checkpoint");
+        if (cluster_gave_up(host + 32)) return fail_msg("a wait inside the iteration kernel gave up");
         ts.last.checkpoints += 1;
         activity_is_ax = true;
         dual_step = host[24];
@@ -783,9 +811,10 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
     }
     if (!activity_is_ax) {
         // the reference leaves A x_bar of the last iteration in `activity`
-        B200_TRY(cudaMemcpyAsync(host, w.out + 24, sizeof(double), cudaMemcpyDeviceToHost, stream), "read dual step");
+        B200_TRY(cudaMemcpyAsync(host, w.out + 24, 9 * sizeof(double), cudaMemcpyDeviceToHost, stream), "read dual step");
         if (r) launch_tiled(ap.a, w.x_bar, StoreEpi{w.act}, stream, tiled_grid<StoreEpi>(ap.a));
         B200_TRY(cudaStreamSynchronize(stream), "activity");
+        if (cluster_gave_up(host + 8)) return fail_msg("a wait inside the iteration kernel gave up");
         dual_step = host[0];
     }
     if (n) B200_TRY(cudaMemcpyAsync(x, w.x[sv.cur], nb, cudaMemcpyDeviceToHost, stream), "download x");
