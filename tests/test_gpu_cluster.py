@@ -29,6 +29,14 @@ def steps(inst):
     return 0.9 / (1 + cm), 0.9 / (1 + rm)
 
 
+def scaled_steps(engine, **kw):
+    s = engine.pdlp_default_settings()
+    s.eps_optimal, s.ruiz_iterations = 1e-14, 10
+    for k, v in kw.items():
+        setattr(s, k, v)
+    return s
+
+
 SHAPES = [
     (1, 1, [1]), (3, 2, [0, 2, 1]), (40, 31, [0, 1, 31]), (257, 300, [32, 33, 0]), (64, 700, [256, 257, 300, 5]),
     (1200, 900, [1, 40, 3]), (15, 6000, [9]), (6000, 15, [2]), (4000, 9000, [7, 3, 11]), (9000, 17500, [4]),
@@ -64,3 +72,49 @@ def test_cluster_equals_launches(engine, instances, shape, entry):
     if got[0][1] is not None:
         assert np.array_equal(got[0][1], got[1][1])
     assert got[0][2] == got[1][2]
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("precision", ["FP64", "FP32_REFINE", "BF16_REFINE"])
+def test_adaptive_cluster_equals_launches(engine, instances, shape, precision):
+    """A QP whose diagonal Hessian is zero is the same LP on the launches: x - tau g over
+    1 + tau 0 = 1, so every step and every decision has the same bits (only the objective's
+    sums are formed differently). 150 iterations: windows of 64 and a tail of 22."""
+    inst = lp(instances, *shape, seed=5)
+    s = scaled_steps(engine, max_iterations=150, precision=getattr(engine, precision))
+    A = engine.Matrix.from_instance(inst)
+    rc, x, y, r = engine.pdlp_solve(A, inst, s)
+    rc2, x2, y2, r2 = engine.pdlp_solve_qp(A, inst, s, qdiag=np.zeros(inst["n"]))
+    assert rc == rc2 == 0
+    assert np.array_equal(x, x2) and np.array_equal(y, y2)
+    for k in ("iterations", "restarts", "rejected_steps", "final_step_size", "primal_weight"):
+        assert r[k] == r2[k], k
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}x{s[1]}")
+def test_halpern_cluster_equals_numpy(engine, instances, shape):
+    """64 anchored steps and T(z), the point the window's restart takes, against numpy FP64
+    without scaling. The anchored iteration is non-expansive, so a step's rounding (a few
+    ulps over rows of up to 300 entries) adds up at most linearly: 64 x 300 x 2^-52 = 4e-12
+    of the largest entry."""
+    inst = lp(instances, *shape, seed=9)
+    s = scaled_steps(engine, max_iterations=64, scaling=0, algorithm=engine.PDLP_HALPERN, initial_primal_weight=1.0)
+    rc, x, y, r = engine.pdlp_solve(engine.Matrix.from_instance(inst), inst, s)
+    assert rc == 0 and r["iterations"] == 64
+    import scipy.sparse as sp
+    A = sp.csr_matrix((inst["val"], inst["idx"], inst["ptr"]), shape=(inst["m"], inst["n"]))
+    eta = 0.9 / r["matrix_norm"]
+    clip = lambda v, lo, hi: np.minimum(np.maximum(v, lo), hi)
+    u, v = np.zeros(inst["n"]), np.zeros(inst["m"])
+    for k in range(65):
+        xp = clip(u - eta * (inst["c"] + A.T @ v), inst["cl"], inst["cu"])
+        w = v + eta * (A @ (2 * xp - u))
+        yp = w - eta * clip(w / eta, inst["rl"], inst["ru"])
+        if k == 64:
+            break
+        lam = (k + 1.0) / (k + 2.0)
+        u, v = lam * (2 * xp - u), lam * (2 * yp - v)
+    if r["restarts"] == 0:
+        xp, yp = u, v
+    assert np.abs(x - xp).max() <= 4e-12 * max(1.0, np.abs(xp).max())
+    assert np.abs(y - yp).max() <= 4e-12 * max(1.0, np.abs(yp).max())

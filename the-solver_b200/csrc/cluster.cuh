@@ -31,6 +31,7 @@ namespace cluster {
 constexpr int kClusterCtas = 16;       // non-portable size; checked with cudaOccupancyMaxActiveClusters
 constexpr int kClusterThreads = 512;
 constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kMaxSteps = 4096;       // iterations per launch: some ten milliseconds
 constexpr int kMaxTries = 1 << 20;    // of a wait, each of up to some microseconds
 constexpr int kMaxSmem = 226 * 1024;     // dynamic; the rest of the 227 KB holds the static arrays
 
@@ -76,6 +77,25 @@ __device__ __forceinline__ unsigned load_remote16(unsigned addr) {
 }
 
 inline size_t align16(size_t b) { return (b + 15) / 16 * 16; }
+
+// An mbarrier that one thread of the CTA arms with the bytes of an exchange.
+__device__ __forceinline__ void init_barrier(unsigned long long* bar) {
+    asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(bar))));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void expect_bytes(unsigned long long* bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(bar))), "r"(bytes) : "memory");
+}
+// False when the wait gave up.
+__device__ __forceinline__ bool wait_bytes(unsigned long long* bar, unsigned phase) {
+    unsigned done = 0;
+    for (int tries = 0; !done && tries < kMaxTries; ++tries)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done)
+                     : "r"(static_cast<unsigned>(__cvta_generic_to_shared(bar))), "r"(phase) : "memory");
+    return done != 0;
+}
 
 // ------------------------------------------------------------ one CTA's part
 
@@ -134,6 +154,17 @@ __host__ __device__ inline size_t send_bytes(const Share& s) {
     return (send_length(s) * 2ull + 15) / 16 * 16;
 }
 
+// Inclusive sums over the lanes.
+__device__ __forceinline__ int warp_scan(int v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    return v;
+}
+
 struct Arena {
     char* at;
     template <class X>
@@ -144,61 +175,84 @@ struct Arena {
     }
 };
 
-// Copies this CTA's chunks of M into shared memory and finds the elements they gather.
-// Ends with a block barrier; other CTAs may read `in` after the next cluster barrier.
+// A CTA's part of one matrix.
 template <class T, class V>
-__device__ __forceinline__ void load_part(const TileCsrT<V>& M, unsigned rank, Arena& mem, Slice<V>* out, Packed<T>* in) {
-    const Share& s = M.share;
-    const int words = (M.cols + 31) / 32;
-    out->val = mem.take<V>(s.nnz);
-    out->ptr = mem.take<int>(s.rows + 1);
-    out->first = mem.take<int>(s.chunks + 1);
-    out->idx = mem.take<unsigned short>(s.nnz);
-    in->v = mem.take<T>(packed_length(M.cols, s));
-    in->bits = mem.take<unsigned>(words);
-    in->before = mem.take<unsigned short>(words);
-    in->bar = mem.take<unsigned long long>(1);
-    in->phase = 0;
-    const int t0 = min(M.ntiles, static_cast<int>(rank) * s.chunks), t1 = min(M.ntiles, t0 + s.chunks);
-    const int2 b0 = __ldg(M.tile + t0), b1 = __ldg(M.tile + t1);
-    const int nnz = b1.y - b0.y;
-    out->row0 = b0.x;
-    out->rows = b1.x - b0.x;
-    out->chunks = t1 - t0;
-    for (int w = threadIdx.x; w < words; w += blockDim.x) in->bits[w] = 0u;
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(in->bar))));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+struct Part {
+    Slice<V> slice;
+    Packed<T> in;
+    int2 first;   // row and entry at which the slice starts
+    int nnz;
+
+    __device__ __forceinline__ void place(const TileCsrT<V>& M, unsigned rank, Arena& mem) {
+        const Share& s = M.share;
+        const int words = (M.cols + 31) / 32;
+        slice.val = mem.take<V>(s.nnz);
+        slice.ptr = mem.take<int>(s.rows + 1);
+        slice.first = mem.take<int>(s.chunks + 1);
+        slice.idx = mem.take<unsigned short>(s.nnz);
+        in.v = mem.take<T>(packed_length(M.cols, s));
+        in.bits = mem.take<unsigned>(words);
+        in.before = mem.take<unsigned short>(words);
+        in.bar = mem.take<unsigned long long>(1);
+        in.phase = 0;
+        const int t0 = min(M.ntiles, static_cast<int>(rank) * s.chunks), t1 = min(M.ntiles, t0 + s.chunks);
+        const int2 end = __ldg(M.tile + t1);
+        first = __ldg(M.tile + t0);
+        nnz = end.y - first.y;
+        slice.row0 = first.x;
+        slice.rows = end.x - first.x;
+        slice.chunks = t1 - t0;
+        for (int w = threadIdx.x; w < words; w += blockDim.x) in.bits[w] = 0u;
+        if (threadIdx.x == 0) init_barrier(in.bar);
+        for (int k = threadIdx.x; k <= slice.chunks; k += blockDim.x) slice.first[k] = __ldg(M.tile + t0 + k).x - first.x;
     }
-    __syncthreads();
-    for (int k = threadIdx.x; k <= t1 - t0; k += blockDim.x) out->first[k] = __ldg(M.tile + t0 + k).x - b0.x;
-    for (int r = threadIdx.x; r <= b1.x - b0.x; r += blockDim.x) out->ptr[r] = __ldg(M.ptr + b0.x + r) - b0.y;
-    for (int p = threadIdx.x; p < nnz; p += blockDim.x) {
-        const int j = __ldg(M.idx + b0.y + p);
-        atomicOr(in->bits + (j >> 5), 1u << (j & 31));
-        out->val[p] = M.val[b0.y + p];
+    __device__ __forceinline__ void fetch(const TileCsrT<V>& M) const {
+        for (int r = threadIdx.x; r <= slice.rows; r += blockDim.x) slice.ptr[r] = __ldg(M.ptr + first.x + r) - first.y;
+#pragma unroll 4
+        for (int p = threadIdx.x; p < nnz; p += blockDim.x) {
+            const int j = __ldg(M.idx + first.y + p);
+            const V v = M.val[first.y + p];
+            atomicOr(in.bits + (j >> 5), 1u << (j & 31));
+            slice.val[p] = v;
+        }
     }
-    __syncthreads();
-    if (threadIdx.x < 32) {
+    __device__ __forceinline__ void count(int cols) const {   // one warp
+        const int words = (cols + 31) / 32, lane = threadIdx.x & 31;
         int run = 0;
         for (int w0 = 0; w0 < words; w0 += 32) {
-            const int w = w0 + static_cast<int>(threadIdx.x), c = w < words ? __popc(in->bits[w]) : 0;
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (static_cast<int>(threadIdx.x) >= o) incl += t;
-            }
-            if (w < words) in->before[w] = static_cast<unsigned short>(run + incl - c);
+            const int w = w0 + lane, c = w < words ? __popc(in.bits[w]) : 0;
+            const int incl = warp_scan(c);
+            if (w < words) in.before[w] = static_cast<unsigned short>(run + incl - c);
             run += __shfl_sync(0xffffffffu, incl, 31);
         }
     }
-    __syncthreads();
-    in->bytes = words ? static_cast<unsigned>(sizeof(T)) * (in->before[words - 1] + __popc(in->bits[words - 1])) : 0u;
-    for (int p = threadIdx.x; p < nnz; p += blockDim.x) {
-        const int j = __ldg(M.idx + b0.y + p), w = j >> 5;
-        out->idx[p] = static_cast<unsigned short>(in->before[w] + __popc(in->bits[w] & ((1u << (j & 31)) - 1u)));
+    __device__ __forceinline__ void remap(const TileCsrT<V>& M) {
+        const int words = (M.cols + 31) / 32;
+        in.bytes = words ? static_cast<unsigned>(sizeof(T)) * (in.before[words - 1] + __popc(in.bits[words - 1])) : 0u;
+#pragma unroll 4
+        for (int p = threadIdx.x; p < nnz; p += blockDim.x) {
+            const int j = __ldg(M.idx + first.y + p), w = j >> 5;
+            slice.idx[p] = static_cast<unsigned short>(in.before[w] + __popc(in.bits[w] & ((1u << (j & 31)) - 1u)));
+        }
     }
+};
+
+// Copies this CTA's chunks of both matrices into shared memory and finds the elements they
+// gather. Ends with a block barrier; other CTAs may read `in` after the next cluster barrier.
+template <class T, class V>
+__device__ __forceinline__ void load_parts(const TileCsrT<V>& A, const TileCsrT<V>& AT, unsigned rank, Arena& mem,
+                                           Part<T, V>* a, Part<T, V>* at) {
+    a->place(A, rank, mem);
+    at->place(AT, rank, mem);
+    __syncthreads();
+    a->fetch(A);
+    at->fetch(AT);
+    __syncthreads();
+    if (threadIdx.x < 32) a->count(A.cols);
+    else if (threadIdx.x < 64) at->count(AT.cols);
+    __syncthreads();
+    a->remap(A);
+    at->remap(AT);
     __syncthreads();
 }
 
@@ -221,50 +275,58 @@ __device__ __forceinline__ void make_sends(int row0, int rows, const Packed<T>& 
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
     out->src = mem.take<unsigned short>(send_length(s));
-    const unsigned bits = remote(in.bits, c);
-    auto needs = [&](int r) {
-        const int j = row0 + r;
-        return r < rows && (load_remote(bits + 4u * (j >> 5)) >> (j & 31) & 1u);
+    // the words of the destination's bits that cover [row0, row0 + rows), a lane each
+    const int w0 = row0 >> 5, words = rows > 0 ? ((row0 + rows - 1) >> 5) - w0 + 1 : 0;
+    const unsigned bits = remote(in.bits + w0, c);
+    auto word = [&](int w) {
+        if (w >= words) return 0u;
+        unsigned b = load_remote(bits + 4u * w);
+        const int lo = row0 - 32 * (w0 + w), hi = row0 + rows - 32 * (w0 + w);   // bits [lo, hi) are ours
+        if (lo > 0) b &= ~0u << lo;
+        if (hi < 32) b &= (1u << hi) - 1u;
+        return b;
     };
     int count = 0;
-    for (int r = lane; r - lane < rows; r += 32) count += __popc(__ballot_sync(full, needs(r)));
-    __syncthreads();
+    for (int w = lane; w - lane < words; w += 32) count += __reduce_add_sync(full, __popc(word(w)));
     if (lane == 0) counts[c] = count;
     __syncthreads();
     for (int k = 0; k < c; ++k) out->src += counts[k];
     out->count = count;
     out->bar = remote(in.bar, c);
     out->at = remote(in.v, c);
-    if (count == 0) return;
-    out->at += static_cast<unsigned>(sizeof(T)) *
-               (load_remote16(remote(in.before, c) + 2u * (row0 >> 5)) +
-                __popc(load_remote(bits + 4u * (row0 >> 5)) & ((1u << (row0 & 31)) - 1u)));
-    int run = 0;
-    for (int r = lane; r - lane < rows; r += 32) {
-        const bool mine = needs(r);
-        const unsigned who = __ballot_sync(full, mine);
-        if (mine) out->src[run + __popc(who & ((1u << lane) - 1u))] = static_cast<unsigned short>(r);
-        run += __popc(who);
+    if (count > 0) {
+        out->at += static_cast<unsigned>(sizeof(T)) *
+                   (load_remote16(remote(in.before + w0, c)) + __popc(load_remote(bits) & ((1u << (row0 & 31)) - 1u)));
+        int run = 0;
+        for (int w = lane; w - lane < words; w += 32) {
+            unsigned b = word(w);
+            const int incl = warp_scan(__popc(b));
+            for (int k = run + incl - __popc(b); b; b &= b - 1u)
+                out->src[k++] = static_cast<unsigned short>(32 * (w0 + w) + __ffs(b) - 1 - row0);
+            run += __shfl_sync(full, incl, 31);
+        }
     }
-    __syncwarp();
+    __syncthreads();
 }
 
 // Sends the CTA's own elements to the CTAs that gather them, and waits until this CTA's
-// packed copy has all of its elements. False when the wait gave up.
-template <class T>
-__device__ __forceinline__ bool exchange(const SendList& s, const T* own, Packed<T>& in) {
-    const unsigned bar = static_cast<unsigned>(__cvta_generic_to_shared(in.bar));
+// packed copy has all of its elements. False when the wait gave up. `meanwhile` runs while
+// the elements are on their way.
+template <class T, class F>
+__device__ __forceinline__ bool exchange(const SendList& s, const T* own, Packed<T>& in, F meanwhile) {
     __syncthreads();   // `own` is complete
-    if (threadIdx.x == 0)
-        asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(bar), "r"(in.bytes) : "memory");
+    if (threadIdx.x == 0) expect_bytes(in.bar, in.bytes);
     for (int k = threadIdx.x & 31; k < s.count; k += 32)
         send_one(s.at + static_cast<unsigned>(sizeof(T)) * k, own[s.src[k]], s.bar);
-    unsigned done = 0;
-    for (int tries = 0; !done && tries < kMaxTries; ++tries)
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(in.phase) : "memory");
+    meanwhile();
+    const bool done = wait_bytes(in.bar, in.phase);
     in.phase ^= 1u;
-    return done != 0;
+    return done;
+}
+
+template <class T>
+__device__ __forceinline__ bool exchange(const SendList& s, const T* own, Packed<T>& in) {
+    return exchange(s, own, in, [] {});
 }
 
 // Shared-memory loads that stay where they are written: the entries of a batch are all

@@ -14,8 +14,6 @@
 
 namespace b200 {
 
-constexpr int kMaxClusterIterations = 4096;  // per launch: a few milliseconds
-
 struct FixedClusterArgs {
     TileCsr A, AT;
     const double *c, *cl, *cu, *tauv, *qdiag;  // tauv / sigv / qdiag may be null
@@ -48,11 +46,11 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
     Arena mem{smem};
     double* sp = mem.take<double>(kClusterWarps * kProducts) + warp * kProducts;
     if (lane < 2) sp[kChunkNnz + lane] = -0.0;
-    Slice<double> R, Q;       // rows of A, rows of A' (columns)
-    Packed<double> xv, yv;    // x_bar as R gathers it, y as Q gathers it
+    Part<double, double> rows, cols;   // of A and of A'
     SendList xs_out, ys_out;
-    load_part(a.A, rank, mem, &R, &xv);
-    load_part(a.AT, rank, mem, &Q, &yv);
+    load_parts(a.A, a.AT, rank, mem, &rows, &cols);
+    const Slice<double>&R = rows.slice, &Q = cols.slice;
+    Packed<double>&xv = rows.in, &yv = cols.in;    // x_bar as R gathers it, y as Q gathers it
     double* y = mem.take<double>(a.A.share.rows);    // own elements
     double* x = mem.take<double>(a.AT.share.rows);
     double* xb = mem.take<double>(a.AT.share.rows);

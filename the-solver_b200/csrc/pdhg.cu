@@ -300,10 +300,10 @@ struct Solver {
         dual_blocks = A->ntiles ? grid_dual : 0;
     }
 
-    // k iterations as cluster launches of up to kMaxClusterIterations.
+    // k iterations as cluster launches of up to cluster::kMaxSteps.
     int run_cluster(int k) {
         while (k > 0) {
-            const int steps = std::min(k, kMaxClusterIterations), nx = cur ^ 1;
+            const int steps = std::min(k, cluster::kMaxSteps), nx = cur ^ 1;
             const FixedClusterArgs a{*A, *AT, w->c, w->cl, w->cu, has_steps ? w->tauv : nullptr,
                                      has_qdiag ? w->qdiag : nullptr, w->rl, w->ru, has_steps ? w->sigv : nullptr,
                                      tau, sigma, theta, w->x[cur], w->y[cur], w->x[nx], w->y[nx], w->x_bar, w->part_c,

@@ -18,6 +18,7 @@
 //   K3  A-side chunks:  A x_cand, block sums of |dy|^2 and dy.(A dx); the last
 //       block to finish combines all partials in a fixed order and writes the
 //       new eta and the accept flag (PdlpKernels.cu:405-494).
+// A small LP's iterations run as one launch per window on a cluster instead (pdlp_cluster.cuh).
 // The window ends with a commit, the residual sums of the current and of the
 // average iterate (PdlpKernels.cu:101-209, fused into the two products), and
 // one small copy to the host, which makes the restart decision.
@@ -94,6 +95,26 @@ __device__ __forceinline__ T clampf(T v, T lo, T hi) {
 
 // ------------------------------------------------------------ iteration kernels
 
+// Dual candidate (PdlpKernels.cu:377-389). Centered: y, ax, ax_prev are deviations from an
+// FP64 center, the prox is taken of the absolute dual y_center + v in FP64.
+template <class T>
+__device__ __forceinline__ T dual_candidate(T y, T ax, T ax_prev, T sigma, T rl, T ru) {
+    const T v = y + sigma * (T(2) * ax - ax_prev);
+    return v - sigma * clampf<T>(v / sigma, rl, ru);
+}
+template <class T>
+__device__ __forceinline__ T dual_candidate_centered(T y, T ax, T ax_prev, T sigma, T rl, T ru, double y_center) {
+    const T v = y + sigma * (T(2) * ax - ax_prev);
+    const double s = static_cast<double>(sigma), vd = static_cast<double>(v);
+    const double w = (y_center + vd) / s;
+    return static_cast<T>(vd - s * clampf<double>(w, static_cast<double>(rl), static_cast<double>(ru)));
+}
+// Primal candidate of an LP (PdlpKernels.cu:391-400).
+template <class T>
+__device__ __forceinline__ T primal_candidate(T x, T aty, T tau, T c, T cl, T cu) {
+    return clampf<T>(x - tau * (c + aty), cl, cu);
+}
+
 // K1 (PdlpKernels.cu:499-518 commit, then :377-389 dual candidate). With
 // y_center (the centered FP32 loop) y, ax, ax_prev are deviations from an FP64
 // center and rl / ru the row bounds shifted by A x_center: the prox is taken of
@@ -120,17 +141,9 @@ __global__ void k_commit_dual(int n, int m, PdlpState* __restrict__ st, T* __res
             ax_prev[i] = axp;
             ax[i] = axi;
         }
-        if (make_candidate) {
-            const T v = yi + sigma * (T(2) * axi - axp);
-            if (y_center) {
-                const double s = static_cast<double>(sigma), vd = static_cast<double>(v);
-                const double w = (y_center[i] + vd) / s;
-                y_cand[i] = static_cast<T>(vd - s * clampf<double>(w, static_cast<double>(rl[i]),
-                                                                    static_cast<double>(ru[i])));
-            } else {
-                y_cand[i] = v - sigma * clampf<T>(v / sigma, rl[i], ru[i]);
-            }
-        }
+        if (make_candidate)
+            y_cand[i] = y_center ? dual_candidate_centered(yi, axi, axp, sigma, rl[i], ru[i], y_center[i])
+                                 : dual_candidate(yi, axi, axp, sigma, rl[i], ru[i]);
     }
     if (acc) {
         for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
@@ -157,13 +170,17 @@ struct StepRule {
     double limit, next;
     bool keep;
 };
-__device__ __forceinline__ StepRule step_rule(double used, double w, double dx2, double dy2, double cross, double k,
-                                              double lo, double hi) {
+// The rule's two factors at trial k: damp = 1 - (k+1)^-0.3 and boost = 1 + (k+1)^-0.6.
+__device__ __forceinline__ double step_growth(double k, bool damp) {
+    const double p = pow(k + 1.0, damp ? -0.3 : -0.6);
+    return damp ? 1.0 - p : 1.0 + p;
+}
+__device__ __forceinline__ StepRule step_rule(double used, double w, double dx2, double dy2, double cross, double damp,
+                                              double boost, double lo, double hi) {
     StepRule r;
     const double half_norm = 0.5 * (w * dx2 + dy2 / w);
     r.limit = (cross > 0.0 && half_norm > 0.0) ? half_norm / cross : hi;
     r.keep = used <= r.limit;
-    const double damp = 1.0 - pow(k + 1.0, -0.3), boost = 1.0 + pow(k + 1.0, -0.6);
     double next = fmin(damp * r.limit, boost * used);
     if (!(next > 0.0 && isfinite(next))) next = used;
     r.next = fmin(fmax(next, lo), hi);
@@ -204,7 +221,7 @@ struct PrimalCandEpi {
         T xc;
         if (QM == kQDiag) xc = clampf<T>((r.x - tau * (r.c + aty)) / (T(1) + tau * r.q), r.lo, r.hi);
         else if (QM == kQGeneral) xc = clampf<T>(r.x - tau * (r.c + r.qx + aty) / (T(1) + tau * r.q), r.lo, r.hi);
-        else xc = clampf<T>(r.x - tau * (r.c + aty), r.lo, r.hi);
+        else xc = primal_candidate(r.x, aty, tau, r.c, r.lo, r.hi);
         x_cand[j] = xc;
         const double dx = static_cast<double>(xc) - static_cast<double>(r.x);
         acc.add(0, dx * dx);
@@ -281,8 +298,8 @@ struct ProbeEpi {
         }
         if (threadIdx.x != 0) return;
         const double probe = st->updates + 1.0;
-        const StepRule rule = step_rule(st->eta, st->omega, red[0][0], red[1][0], fabs(red[2][0]), probe,
-                                        st->eta_min, st->eta_max);
+        const StepRule rule = step_rule(st->eta, st->omega, red[0][0], red[1][0], fabs(red[2][0]), step_growth(probe, true),
+                                        step_growth(probe, false), st->eta_min, st->eta_max);
         st->dx_sq = red[0][0];
         st->dy_sq = red[1][0];
         st->interaction = fabs(red[2][0]);
@@ -345,6 +362,20 @@ __device__ __forceinline__ T halpern_lambda(const PdlpState* st, int q) {
 }
 
 template <class T>
+__device__ __forceinline__ T primal_reflected(T x, T aty, T tau, T c, T cl, T cu) {
+    return T(2) * clampf<T>(x - tau * (c + aty), cl, cu) - x;
+}
+template <class T>
+__device__ __forceinline__ T dual_reflected(T y, T axb, T sigma, T rl, T ru) {
+    const T v = y + sigma * axb;
+    return T(2) * (v - sigma * clampf<T>(v / sigma, rl, ru)) - y;
+}
+template <class T>
+__device__ __forceinline__ T halpern_step(T lam, T reflected, T anchor) {
+    return lam * reflected + (T(1) - lam) * anchor;
+}
+
+template <class T>
 struct PrimalHalpernEpi {
     T* __restrict__ x;
     T* __restrict__ x_bar;
@@ -358,10 +389,9 @@ struct PrimalHalpernEpi {
     __device__ __forceinline__ void row(int j, T aty, Acc&) const {
         const T tau = static_cast<T>(st->eta / st->omega);
         const T xj = x[j];
-        const T xr = T(2) * clampf<T>(xj - tau * (c[j] + aty), cl[j], cu[j]) - xj;
-        const T lam = halpern_lambda<T>(st, q);
+        const T xr = primal_reflected(xj, aty, tau, c[j], cl[j], cu[j]);
         x_bar[j] = xr;
-        x[j] = lam * xr + (T(1) - lam) * x0[j];
+        x[j] = halpern_step(halpern_lambda<T>(st, q), xr, x0[j]);
     }
     __device__ __forceinline__ void finish(Acc&, double*) const {}
 };
@@ -377,11 +407,8 @@ struct DualHalpernEpi {
     using Acc = NoAcc;
     __device__ __forceinline__ void row(int i, T axb, Acc&) const {
         const T sigma = static_cast<T>(st->eta * st->omega);
-        const T yi = y[i];
-        const T v = yi + sigma * axb;
-        const T yr = T(2) * (v - sigma * clampf<T>(v / sigma, rl[i], ru[i])) - yi;
-        const T lam = halpern_lambda<T>(st, q);
-        y[i] = lam * yr + (T(1) - lam) * y0[i];
+        const T yr = dual_reflected(y[i], axb, sigma, rl[i], ru[i]);
+        y[i] = halpern_step(halpern_lambda<T>(st, q), yr, y0[i]);
     }
     __device__ __forceinline__ void finish(Acc&, double*) const {}
 };
@@ -449,6 +476,14 @@ __global__ void k_halpern_restart(int n, int m, const T* __restrict__ x_t, const
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) x[j] = x0[j] = x_t[j];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += stride) y[i] = y0[i] = y_t[i];
 }
+
+}  // namespace
+}  // namespace b200
+
+#include "pdlp_cluster.cuh"
+
+namespace b200 {
+namespace {
 
 // ----------------------------------------------------------- residual kernels
 // PdlpKernels.cu:101-209 split over the two products, accumulated in FP64.
@@ -1187,6 +1222,10 @@ struct LoopStats {
 // Restarted PDLP on one problem whose data (c, bounds) have type T and whose matrix
 // values have type V (T, or bf16 under fp32 iterates); iterates of type T; reductions
 // and decisions in FP64.
+// Slots of Core::res: 0..13 and 16..29 the two evaluated points, 32..35 the Halpern sums,
+// kFail set when a wait inside a cluster launch gave up.
+constexpr int kFail = 40;
+
 template <class T, class V = T>
 struct Core {
     int n = 0, m = 0, sms = 148;
@@ -1204,6 +1243,11 @@ struct Core {
     int grid_rrc = 1, grid_rcc = 1;
     int launches = 0;
     std::vector<cudaGraphExec_t> graphs;
+    // Small LPs: the iterations of a window run as one launch on one cluster
+    // (pdlp_cluster.cuh); 0 where the problem does not fit or is a QP.
+    size_t adaptive_smem = 0, halpern_smem = 0;
+    void (*adaptive_kernel)(AdaptiveClusterArgs<T, V>) = nullptr;
+    void (*halpern_kernel)(HalpernClusterArgs<T, V>) = nullptr;
     // Quadratic objective (the QP entry point): qmode kQDiag with the diagonal qd,
     // or kQGeneral with the Hessian Q and its diagonal majorant qd, whose products
     // Q x (committed point), Q x_cand and Q x_avg ride along like the A-side ones;
@@ -1277,9 +1321,26 @@ struct Core {
         grid_rcc = qmode == kQDiag ? tiled_grid<ResColsCenteredEpi<T, kQDiag>, T>(AT)
                    : qmode == kQGeneral ? tiled_grid<ResColsCenteredEpi<T, kQGeneral>, T>(AT)
                                         : tiled_grid<ResColsCenteredEpi<T>, T>(AT);
+        choose_cluster();
         for (auto g : graphs)
             if (g) cudaGraphExecDestroy(g);
         graphs.clear();
+    }
+
+    // Rule: an LP that fits one cluster's shared memory. The adaptive loop also needs one
+    // chunk per warp in the launches it stands for, so that the decision's sums keep their shape.
+    void choose_cluster() {
+        adaptive_smem = halpern_smem = 0;
+        if (qmode != kLp) return;
+        const bool one = A.share.chunks <= cluster::kClusterWarps && AT.share.chunks <= cluster::kClusterWarps;
+        adaptive_kernel = one ? &k_adaptive_cluster<T, V, true> : &k_adaptive_cluster<T, V, false>;
+        halpern_kernel = one ? &k_halpern_cluster<T, V, true> : &k_halpern_cluster<T, V, false>;
+        const size_t ad = adaptive_cluster_smem<T, V>(A, AT), ha = halpern_cluster_smem<T, V>(A, AT);
+        if (ad && ad <= cluster::kMaxSmem && A.ntiles <= grid_k3 * kWarps && AT.ntiles <= grid_k2 * kWarps &&
+            cluster::available(reinterpret_cast<const void*>(adaptive_kernel)))
+            adaptive_smem = ad;
+        if (ha && ha <= cluster::kMaxSmem && cluster::available(reinterpret_cast<const void*>(halpern_kernel)))
+            halpern_smem = ha;
     }
 
     // The QP's Hessian: a diagonal (diag, q null) or a general matrix (q, n x n, with
@@ -1372,8 +1433,35 @@ struct Core {
         launches += 2;
     }
 
-    // One window (period iterations) + window-end evaluation, as a graph.
+    // Window-end evaluation: residual sums of the current and the average iterate, to the host.
+    void window_end(bool adaptive) {
+        residuals(x, y, nullptr, nullptr, res, 0, qx);
+        k_average<T><<<eg(std::max(n, m)), kThreads, 0, stream>>>(n, m, st, adaptive ? 1 : 0, x_sum, y_sum, x_avg,
+                                                                   y_avg);
+        if (qmode == kQGeneral) {
+            launch_tiled(Q, x_avg, StoreEpiT<T>{qx_avg}, stream, grid_qs);
+            ++launches;
+        }
+        residuals(x_avg, y_avg, ax_avg, nullptr, res + 16, 1, qx_avg);
+        cudaMemcpyAsync(host, res, (kFail + 1) * sizeof(double), cudaMemcpyDeviceToHost, stream);
+        ++launches;
+    }
+
+    // One window (period iterations) + window-end evaluation: one cluster launch and the
+    // evaluation's launches, or all launches as a graph.
     int window(int period, bool adaptive, double tau, double sigma, int* graph_slot) {
+        if (adaptive && adaptive_smem) {
+            for (int done = 0; done < period; done += cluster::kMaxSteps) {
+                const AdaptiveClusterArgs<T, V> a{A, AT, x, x_sum, y, y_sum, ax, ax_prev, c, cl, cu, rl, ru,
+                                                  ctr ? ctr->yc : nullptr, st, res + kFail,
+                                                  std::min(period - done, cluster::kMaxSteps)};
+                B200_TRY(cluster::launch(adaptive_kernel, a, adaptive_smem, stream), "cluster launch");
+                ++launches;
+            }
+            window_end(true);
+            B200_TRY(cudaGetLastError(), "window launch");
+            return 0;
+        }
         cudaGraphExec_t exec = nullptr;
         if (*graph_slot >= 0) exec = graphs[static_cast<size_t>(*graph_slot)];
         if (!exec) {
@@ -1385,15 +1473,7 @@ struct Core {
                 else fixed_iteration(static_cast<T>(tau), static_cast<T>(sigma));
             }
             if (adaptive) adaptive_iteration(false);  // commit the last probe
-            residuals(x, y, nullptr, nullptr, res, 0, qx);
-            k_average<T><<<eg(std::max(n, m)), kThreads, 0, stream>>>(n, m, st, adaptive ? 1 : 0, x_sum, y_sum, x_avg,
-                                                                       y_avg);
-            if (qmode == kQGeneral) {
-                launch_tiled(Q, x_avg, StoreEpiT<T>{qx_avg}, stream, grid_qs);
-                ++launches;
-            }
-            residuals(x_avg, y_avg, ax_avg, nullptr, res + 16, 1, qx_avg);
-            cudaMemcpyAsync(host, res, 32 * sizeof(double), cudaMemcpyDeviceToHost, stream);
+            window_end(adaptive);
             B200_TRY(cudaStreamEndCapture(stream, &g), "end capture");
             cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
             cudaGraphDestroy(g);
@@ -1442,11 +1522,33 @@ struct Core {
         ++launches;
     }
 
+    // T at a Halpern window's end, its residual sums and relative KKT, to the host.
+    void halpern_window_end() {
+        launch_tiled(AT, y, PrimalTEpi<T>{x, x_bar, x_cand, x_restart, c, cl, cu, st, part_c}, stream, grid_pt);
+        k_combine<2, 3u><<<1, kThreads, 0, stream>>>(part_c, AT.ntiles ? grid_pt : 0, res + 32);
+        launch_tiled(A, x_bar, DualTEpi<T>{y, y_cand, y_restart, rl, ru, st, part_d}, stream, grid_dt);
+        k_combine<2, 3u><<<1, kThreads, 0, stream>>>(part_d, A.ntiles ? grid_dt : 0, res + 34);
+        residuals(x_cand, y_cand, nullptr, nullptr, res, 0);
+        cudaMemcpyAsync(host, res, (kFail + 1) * sizeof(double), cudaMemcpyDeviceToHost, stream);
+        launches += 4;
+    }
+
     // One Halpern window: `period` anchored steps, then T at the window's end
     // (into x_cand / y_cand), its residual sums (res[32..35]) and the relative KKT of
     // T(z) (res[0..13]); x_restart / y_restart hold the anchor. A graph per (period,
     // tau, sigma); the anchor offset comes from the device state.
     int halpern_window(int period, int* graph_slot) {
+        if (halpern_smem) {
+            for (int done = 0; done < period; done += cluster::kMaxSteps) {
+                const HalpernClusterArgs<T, V> a{A, AT, x, y, x_restart, y_restart, c, cl, cu, rl, ru, st, res + kFail,
+                                                 done, std::min(period - done, cluster::kMaxSteps)};
+                B200_TRY(cluster::launch(halpern_kernel, a, halpern_smem, stream), "cluster launch");
+                ++launches;
+            }
+            halpern_window_end();
+            B200_TRY(cudaGetLastError(), "window launch");
+            return 0;
+        }
         cudaGraphExec_t exec = nullptr;
         if (*graph_slot >= 0) exec = graphs[static_cast<size_t>(*graph_slot)];
         if (!exec) {
@@ -1457,12 +1559,7 @@ struct Core {
                 launch_tiled(AT, y, PrimalHalpernEpi<T>{x, x_bar, x_restart, c, cl, cu, st, q}, stream, grid_ph);
                 launch_tiled(A, x_bar, DualHalpernEpi<T>{y, y_restart, rl, ru, st, q}, stream, grid_dh);
             }
-            launch_tiled(AT, y, PrimalTEpi<T>{x, x_bar, x_cand, x_restart, c, cl, cu, st, part_c}, stream, grid_pt);
-            k_combine<2, 3u><<<1, kThreads, 0, stream>>>(part_c, AT.ntiles ? grid_pt : 0, res + 32);
-            launch_tiled(A, x_bar, DualTEpi<T>{y, y_cand, y_restart, rl, ru, st, part_d}, stream, grid_dt);
-            k_combine<2, 3u><<<1, kThreads, 0, stream>>>(part_d, A.ntiles ? grid_dt : 0, res + 34);
-            residuals(x_cand, y_cand, nullptr, nullptr, res, 0);
-            cudaMemcpyAsync(host, res, 40 * sizeof(double), cudaMemcpyDeviceToHost, stream);
+            halpern_window_end();
             B200_TRY(cudaStreamEndCapture(stream, &g), "end capture");
             cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
             cudaGraphDestroy(g);
@@ -1500,6 +1597,7 @@ struct Core {
             omega = std::min(kMaxWeight, std::max(kMinWeight, lp.cost_norm / lp.bound_norm));
         if (lp.omega0 > 0.0) omega = lp.omega0;
         k_init_state<<<1, 1, 0, stream>>>(st, eta, omega, eta, eta);
+        B200_TRY(cudaMemsetAsync(res + kFail, 0, sizeof(double), stream), "zero");
         B200_TRY(cudaGetLastError(), "Halpern setup");
         long long iteration = 0, since_restart = 0;
         double r_restart = std::numeric_limits<double>::infinity(), r_previous = r_restart;
@@ -1512,6 +1610,7 @@ struct Core {
             k_set_halpern<<<1, 1, 0, stream>>>(st, static_cast<double>(since_restart));
             if (halpern_window(period, slot)) return -1;
             B200_TRY(cudaStreamSynchronize(stream), "Halpern window");
+            if (host[kFail] != 0.0) return fail_msg("a wait inside the iteration kernel gave up");
             ++out->syncs;
             iteration += period;
             since_restart += period;
@@ -1591,6 +1690,7 @@ struct Core {
         if (lp.omega0 > 0.0) omega = lp.omega0;
         const double eta_start = lp.eta0 > 0.0 ? std::min(std::max(lp.eta0, eta_min), eta_max) : eta_global;
         k_init_state<<<1, 1, 0, stream>>>(st, eta_start, omega, eta_min, eta_max);
+        B200_TRY(cudaMemsetAsync(res + kFail, 0, sizeof(double), stream), "zero");
         B200_TRY(cudaGetLastError(), "PDLP setup");
 
         long long iteration = 0;
@@ -1616,6 +1716,7 @@ struct Core {
             *baked = omega;
             if (window(period, lp.adaptive, tau, sigma, slot)) return -1;
             B200_TRY(cudaStreamSynchronize(stream), "PDLP window");
+            if (host[kFail] != 0.0) return fail_msg("a wait inside the iteration kernel gave up");
             ++out->syncs;
             iteration += period;
             iterations_since_restart += period;
