@@ -247,7 +247,7 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     DevBuf blob;
     // 8 n-vectors + the column segment map, 7 m-vectors + the row segment map,
     // 12 per-LP slots, counters
-    if (blob.alloc(9 * nb + 8 * mb + 12 * kb + 4096, "cudaMalloc batch workspace")) return -1;
+    if (blob.alloc_on(stream, 9 * nb + 8 * mb + 12 * kb + 4096, "cudaMalloc batch workspace")) return -1;
     char* p = blob.as<char>();
     auto take = [&](size_t b) { char* r = p; p += b; return r; };
     double *dc = reinterpret_cast<double*>(take(nb)), *dcl = reinterpret_cast<double*>(take(nb)),
@@ -296,12 +296,8 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     if (m) k_steps_and_max<<<elem_grid(m), kThreads, 0, stream>>>(m, rmass, d_rseg, sig, rmax);
     if (n) k_init_box<<<elem_grid(n), kThreads, 0, stream>>>(n, dcl, dcu, xb0, xbar);
     B200_TRY(cudaGetLastError(), "batch setup");
-    unsigned int* host_counters = nullptr;
-    B200_TRY(cudaMallocHost(reinterpret_cast<void**>(&host_counters), 64), "cudaMallocHost");
-    struct Free {
-        unsigned int* p;
-        ~Free() { cudaFreeHost(p); }
-    } free_host{host_counters};
+    unsigned int* host_counters = reinterpret_cast<unsigned int*>(pinned_slot());
+    if (!host_counters) return fail_msg("cudaMallocHost counters");
     B200_TRY(cudaMemcpyAsync(host_counters, counters, 8, cudaMemcpyDeviceToHost, stream), "read");
     B200_TRY(cudaStreamSynchronize(stream), "batch setup");
     if (host_counters[1]) return fail_msg("matrix is not block-diagonal over the given segments");

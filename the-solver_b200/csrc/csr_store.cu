@@ -312,6 +312,42 @@ int grid_for(const void* kernel, int ntiles, int dynamic_smem) {
     return std::max(1, std::min(ntiles, resident));
 }
 
+cudaMemPool_t solve_pool() {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    static bool asked[64] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!asked[device]) {
+        asked[device] = true;
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        unsigned long long keep = kPoolBytes;
+        int no = 0;   // concurrent solves of several threads do not wait for one another's memory
+        if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
+            cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no) == cudaSuccess)
+            pools[device] = pool;
+        else
+            (void)cudaGetLastError();
+    }
+    return pools[device];
+}
+
+double* pinned_slot() {
+    struct Holder {
+        double* p = nullptr;
+        ~Holder() { if (p) cudaFreeHost(p); }
+    };
+    thread_local Holder h;
+    if (!h.p && cudaMallocHost(reinterpret_cast<void**>(&h.p), kPinnedSlot * sizeof(double)) != cudaSuccess) h.p = nullptr;
+    return h.p;
+}
+
 TimingState& timing() {
     thread_local TimingState state;
     return state;

@@ -199,14 +199,16 @@ struct Workspace {
     unsigned int* flags = nullptr;  // right behind `out`: [0] input checks, [1] a cluster wait gave up
     int n = 0, m = 0;
 
-    int allocate(int n_, int m_, int max_grid) {
+    // From the solve pool on *on, or (null) for longer than a call.
+    int allocate(int n_, int m_, int max_grid, const cudaStream_t* on) {
         n = n_;
         m = m_;
         const size_t nb = (static_cast<size_t>(n) * 8 + 255) / 256 * 256;
         const size_t mb = (static_cast<size_t>(m) * 8 + 255) / 256 * 256;
         const size_t pb = (static_cast<size_t>(max_grid) * 8 * 8 + 255) / 256 * 256;
         const size_t total = 11 * nb + 6 * mb + 3 * pb + 512;
-        if (blob.alloc(total, "cudaMalloc PDHG workspace")) return -1;
+        const char* what = "cudaMalloc PDHG workspace";
+        if (on ? blob.alloc_on(*on, total, what) : blob.alloc(total, what)) return -1;
         char* p = blob.as<char>();
         auto take = [&](size_t b) { double* r = reinterpret_cast<double*>(p); p += b; return r; };
         c = take(nb); cl = take(nb); cu = take(nb); qdiag = take(nb); tauv = take(nb);
@@ -218,17 +220,6 @@ struct Workspace {
         return 0;
     }
 };
-
-// A host-visible pinned slot for checkpoint results, one per thread.
-static double* pinned_out() {
-    struct Holder {
-        double* p = nullptr;
-        ~Holder() { if (p) cudaFreeHost(p); }
-    };
-    thread_local Holder h;
-    if (!h.p && cudaMallocHost(reinterpret_cast<void**>(&h.p), 64 * sizeof(double)) != cudaSuccess) h.p = nullptr;
-    return h.p;
-}
 
 // A checkpoint's results come back with the flags behind them (33 doubles from Workspace::out).
 static bool cluster_gave_up(const double* host_flags) { return reinterpret_cast<const unsigned int*>(host_flags)[1] != 0; }
@@ -477,12 +468,12 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
         if (!cache || cache->w.n != cols || cache->w.m != rows) {
             plan->solve_cache.reset();
             cache = std::make_shared<FixedCache>();
-            if (cache->w.allocate(cols, rows, sms * 8)) return -1;
+            if (cache->w.allocate(cols, rows, sms * 8, nullptr)) return -1;
             plan->solve_cache = cache;
         }
     } else {
         cache = std::make_shared<FixedCache>();
-        if (cache->w.allocate(cols, rows, sms * 8)) return -1;
+        if (cache->w.allocate(cols, rows, sms * 8, &stream)) return -1;
     }
     Workspace* w = &cache->w;
 
@@ -508,7 +499,7 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
         qdiag ? w->qdiag : nullptr, w->flags);
     B200_TRY(cudaGetLastError(), "init launch");
     {
-        unsigned int* hflags = reinterpret_cast<unsigned int*>(pinned_out() + 48);
+        unsigned int* hflags = reinterpret_cast<unsigned int*>(pinned_slot() + 48);
         B200_TRY(cudaMemcpyAsync(hflags, w->flags, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream), "flags");
         B200_TRY(cudaStreamSynchronize(stream), "validation");
         const unsigned int f = *hflags;
@@ -538,7 +529,7 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     const int grid_rows = tiled_grid<CheckRowsCudaEpi>(plan->a);
     const int grid_cols = tiled_grid<CheckColsCudaEpi>(plan->at);
     const int nb_rows = plan->a.ntiles ? grid_rows : 0, nb_cols = plan->at.ntiles ? grid_cols : 0;
-    double* host = pinned_out();
+    double* host = pinned_slot();
     if (!host) return fail_msg("cudaMallocHost checkpoint slot");
 
     bool have_prev = false;
@@ -628,29 +619,30 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
 struct OwnedPair {
     DevBuf ptr, idx, val, tiles, tptr, tidx, tval, ttiles;
     TileCsr a, at;
-    int upload_csc(int rows, int cols, const int* p, const int* i, const double* x) {
+    int upload_csc(int rows, int cols, const int* p, const int* i, const double* x, cudaStream_t s) {
         const int nnz = p[cols];
         const size_t nz = static_cast<size_t>(nnz > 0 ? nnz : 1);
         std::vector<int> tb = build_tiles(cols, p);
-        if (ptr.alloc((static_cast<size_t>(rows) + 1) * 4, "cudaMalloc A") || idx.alloc(nz * 4, "cudaMalloc A") ||
-            val.alloc(nz * 8, "cudaMalloc A") || tptr.alloc((static_cast<size_t>(cols) + 1) * 4, "cudaMalloc A^T") ||
-            tidx.alloc(nz * 4, "cudaMalloc A^T") || tval.alloc(nz * 8, "cudaMalloc A^T") ||
-            ttiles.alloc(tb.size() * 4, "cudaMalloc tiles"))
+        if (ptr.alloc_on(s, (static_cast<size_t>(rows) + 1) * 4, "cudaMalloc A") || idx.alloc_on(s, nz * 4, "cudaMalloc A") ||
+            val.alloc_on(s, nz * 8, "cudaMalloc A") || tptr.alloc_on(s, (static_cast<size_t>(cols) + 1) * 4, "cudaMalloc A^T") ||
+            tidx.alloc_on(s, nz * 4, "cudaMalloc A^T") || tval.alloc_on(s, nz * 8, "cudaMalloc A^T") ||
+            ttiles.alloc_on(s, tb.size() * 4, "cudaMalloc tiles"))
             return -1;
-        B200_TRY(cudaMemcpy(tptr.p, p, tptr.bytes, cudaMemcpyHostToDevice), "upload A^T");
+        B200_TRY(cudaMemcpyAsync(tptr.p, p, tptr.bytes, cudaMemcpyHostToDevice, s), "upload A^T");
         if (nnz) {
-            B200_TRY(cudaMemcpy(tidx.p, i, static_cast<size_t>(nnz) * 4, cudaMemcpyHostToDevice), "upload A^T");
-            B200_TRY(cudaMemcpy(tval.p, x, static_cast<size_t>(nnz) * 8, cudaMemcpyHostToDevice), "upload A^T");
+            B200_TRY(cudaMemcpyAsync(tidx.p, i, static_cast<size_t>(nnz) * 4, cudaMemcpyHostToDevice, s), "upload A^T");
+            B200_TRY(cudaMemcpyAsync(tval.p, x, static_cast<size_t>(nnz) * 8, cudaMemcpyHostToDevice, s), "upload A^T");
         }
-        B200_TRY(cudaMemcpy(ttiles.p, tb.data(), ttiles.bytes, cudaMemcpyHostToDevice), "upload tiles");
+        B200_TRY(cudaMemcpyAsync(ttiles.p, tb.data(), ttiles.bytes, cudaMemcpyHostToDevice, s), "upload tiles");
         if (device_transpose(cols, rows, nnz, tptr.as<int>(), tidx.as<int>(), tval.as<double>(), ptr.as<int>(),
-                             idx.as<int>(), val.as<double>(), nullptr))
+                             idx.as<int>(), val.as<double>(), s))
             return -1;
         std::vector<int> rp(static_cast<size_t>(rows) + 1);
-        B200_TRY(cudaMemcpy(rp.data(), ptr.p, rp.size() * 4, cudaMemcpyDeviceToHost), "read A offsets");
+        B200_TRY(cudaMemcpyAsync(rp.data(), ptr.p, rp.size() * 4, cudaMemcpyDeviceToHost, s), "read A offsets");
+        B200_TRY(cudaStreamSynchronize(s), "read A offsets");
         std::vector<int> ta = build_tiles(rows, rp.data());
-        if (tiles.alloc(ta.size() * 4, "cudaMalloc tiles")) return -1;
-        B200_TRY(cudaMemcpy(tiles.p, ta.data(), tiles.bytes, cudaMemcpyHostToDevice), "upload tiles");
+        if (tiles.alloc_on(s, ta.size() * 4, "cudaMalloc tiles")) return -1;
+        B200_TRY(cudaMemcpyAsync(tiles.p, ta.data(), tiles.bytes, cudaMemcpyHostToDevice, s), "upload tiles");
         a = TileCsr{rows, cols, nnz, static_cast<int>(ta.size()) / 2 - 1, largest_share(ta), ptr.as<int>(),
                     idx.as<int>(), val.as<double>(), tiles.as<int2>()};
         at = TileCsr{cols, rows, nnz, static_cast<int>(tb.size()) / 2 - 1, largest_share(tb), tptr.as<int>(),
@@ -711,12 +703,12 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     OwnedPair ap;
-    if (ap.upload_csc(r, n, m->A.p, m->A.i, m->A.x)) return -1;
+    if (ap.upload_csc(r, n, m->A.p, m->A.i, m->A.x, stream)) return -1;
     OwnedPair qp;
     const bool explicit_q = q && !diagonal;
-    if (explicit_q && qp.upload_csc(n, n, q->p, q->i, q->x)) return -1;
+    if (explicit_q && qp.upload_csc(n, n, q->p, q->i, q->x, stream)) return -1;
     Workspace w;
-    if (w.allocate(n, r, sms * 8)) return -1;
+    if (w.allocate(n, r, sms * 8, &stream)) return -1;
     const size_t nb = sizeof(double) * static_cast<size_t>(n), mb = sizeof(double) * static_cast<size_t>(r);
     if (n) {
         B200_TRY(cudaMemcpyAsync(w.c, m->c, nb, cudaMemcpyHostToDevice, stream), "upload c");
@@ -749,7 +741,7 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
     const int grid_cols = tiled_grid<CheckColsSkEpi>(ap.at);
     const int nb_rows = ap.a.ntiles ? grid_rows : 0, nb_cols = ap.at.ntiles ? grid_cols : 0;
     const int grid_step = elem_grid(n);
-    double* host = pinned_out();
+    double* host = pinned_slot();
     if (!host) return fail_msg("cudaMallocHost checkpoint slot");
     TimingState& ts = timing();
     ts.last = SankhyaB200Timing{};

@@ -1058,8 +1058,8 @@ struct Scaled {
         const size_t nb = (static_cast<size_t>(n) * 8 + 255) / 256 * 256;
         const size_t mb = (static_cast<size_t>(m) * 8 + 255) / 256 * 256;
         const size_t pb = (static_cast<size_t>(sms) * 8 * 8 * 8 + 255) / 256 * 256;
-        if (blob.alloc(8 * nb + 7 * mb + 4 * pb + 1024, "cudaMalloc PDLP model")) return -1;
-        if (vals.alloc(static_cast<size_t>(plan.a.nnz) * 16 + 1024, "cudaMalloc scaled values")) return -1;
+        if (blob.alloc_on(stream, 8 * nb + 7 * mb + 4 * pb + 1024, "cudaMalloc PDLP model")) return -1;
+        if (vals.alloc_on(stream, static_cast<size_t>(plan.a.nnz) * 16 + 1024, "cudaMalloc scaled values")) return -1;
         char* p = blob.as<char>();
         auto take = [&](size_t b) { double* r = reinterpret_cast<double*>(p); p += b; return r; };
         c = take(nb); cl = take(nb); cu = take(nb); Cs = take(nb); tmp_n = take(nb); tmp2_n = take(nb);
@@ -1279,7 +1279,7 @@ struct Core {
         const size_t nb = (static_cast<size_t>(n) * sizeof(T) + 255) / 256 * 256;
         const size_t mb = (static_cast<size_t>(m) * sizeof(T) + 255) / 256 * 256;
         const size_t pb = (static_cast<size_t>(sms) * 8 * 8 * 8 + 255) / 256 * 256;
-        if (blob.alloc(7 * nb + 9 * mb + 4 * pb + 2048, "cudaMalloc PDLP iterates")) return -1;
+        if (blob.alloc_on(stream, 7 * nb + 9 * mb + 4 * pb + 2048, "cudaMalloc PDLP iterates")) return -1;
         char* p = blob.as<char>();
         auto take = [&](size_t b) { char* r = p; p += b; return r; };
         x = reinterpret_cast<T*>(take(nb)); x_cand = reinterpret_cast<T*>(take(nb));
@@ -1356,7 +1356,7 @@ struct Core {
         qmode = kQGeneral;
         Q = *q;
         const size_t nb = (static_cast<size_t>(n) * sizeof(T) + 255) / 256 * 256;
-        if (qblob.alloc(3 * nb, "cudaMalloc Hessian products")) return -1;
+        if (qblob.alloc_on(stream, 3 * nb, "cudaMalloc Hessian products")) return -1;
         qx = qblob.as<T>();
         qx_cand = reinterpret_cast<T*>(qblob.as<char>() + nb);
         qx_avg = reinterpret_cast<T*>(qblob.as<char>() + 2 * nb);
@@ -1791,11 +1791,6 @@ struct Core {
     }
 };
 
-struct HostSlot {
-    double* p = nullptr;
-    ~HostSlot() { if (p) cudaFreeHost(p); }
-};
-
 }  // namespace
 
 }  // namespace b200
@@ -1842,7 +1837,7 @@ int run_polished(const Scaled& sc, Core<double>& hi, const LoopParams& lp, const
     const size_t mb = sizeof(double) * static_cast<size_t>(std::max(m, 1));
     const size_t nd = (nb + 255) / 256 * 256, md = (mb + 255) / 256 * 256;
     DevBuf buf;
-    if (buf.alloc(5 * nd + 4 * md, "cudaMalloc polishing data")) return -1;
+    if (buf.alloc_on(stream, 5 * nd + 4 * md, "cudaMalloc polishing data")) return -1;
     char* base = buf.as<char>();
     double* zero_c = reinterpret_cast<double*>(base);
     double* cl0 = reinterpret_cast<double*>(base + nd);
@@ -2087,12 +2082,12 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
     const double t_start = now_s();
     std::shared_ptr<Plan> plan;
     if (get_plan(matrix, &plan)) return -1;
-    HostSlot hs;
-    B200_TRY(cudaMallocHost(reinterpret_cast<void**>(&hs.p), 64 * sizeof(double)), "cudaMallocHost");
+    double* slot = pinned_slot();
+    if (!slot) return fail_msg("cudaMallocHost result slot");
     cudaStream_t stream = engine_stream();
     Scaled sc;
     sc.stream = stream;
-    sc.host = hs.p;
+    sc.host = slot;
     if (sc.allocate(*plan)) return -1;
     const size_t nb = sizeof(double) * static_cast<size_t>(n), mb = sizeof(double) * static_cast<size_t>(m);
     if (n) {
@@ -2139,7 +2134,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
     if (hessian) {
         if (get_plan(hessian, &qplan)) return -1;
         const size_t qv = (static_cast<size_t>(qplan->a.nnz) * 8 + 255) / 256 * 256;
-        if (qbuf.alloc(qv + static_cast<size_t>(n) * 8 + 256, "cudaMalloc scaled Hessian")) return -1;
+        if (qbuf.alloc_on(stream, qv + static_cast<size_t>(n) * 8 + 256, "cudaMalloc scaled Hessian")) return -1;
         Qs = qplan->a;
         Qs.val = qbuf.as<double>();
         qd_s = reinterpret_cast<double*>(qbuf.as<char>() + qv);
@@ -2149,7 +2144,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
         k_abs_row_sums<<<wg, kThreads, 0, stream>>>(n, qplan->a.ptr, Qs.val, qd_s);
         launches += 2;
     } else if (qdiag) {
-        if (qbuf.alloc(static_cast<size_t>(n) * 8 + 256, "cudaMalloc scaled Hessian diagonal")) return -1;
+        if (qbuf.alloc_on(stream, static_cast<size_t>(n) * 8 + 256, "cudaMalloc scaled Hessian diagonal")) return -1;
         qd_s = qbuf.as<double>();
         if (n) B200_TRY(cudaMemcpyAsync(qd_s, qdiag, nb, cudaMemcpyHostToDevice, stream), "upload diagonal");
         k_scale_diag<<<eg(n), kThreads, 0, stream>>>(n, qd_s, sc.Cs, qd_s);
@@ -2159,7 +2154,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
     // FP64 point of the scaled problem (x^, y^): starts at zeros or the warm start
     Core<double> hi;
     hi.stream = stream;
-    hi.host = hs.p;
+    hi.host = slot;
     if (hi.allocate(n, m, sc.sms)) return -1;
     if (hi.set_hessian(qd_s, hessian ? &Qs : nullptr)) return -1;
     hi.set_problem(sc.A, sc.AT, sc.c, sc.cl, sc.cu, sc.rl, sc.ru);
@@ -2175,7 +2170,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
         lp.cost_norm = cost_norm;
         lp.bound_norm = bound_norm;
         if (polishing) {
-            if (run_polished(sc, hi, lp, s, ps, hs.p, &stats, polish_result, &launches)) return -1;
+            if (run_polished(sc, hi, lp, s, ps, slot, &stats, polish_result, &launches)) return -1;
         } else if (hi.run(lp, &stats)) {
             return -1;
         }
@@ -2188,7 +2183,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
         const size_t nnz = static_cast<size_t>(plan->a.nnz);
         const bool bf16 = s.precision == SANKHYA_B200_BF16_REFINE;
         const size_t vbytes = bf16 ? 2 : 4;
-        if (vals32.alloc(nnz * 2 * vbytes + 1024, "cudaMalloc narrowed values")) return -1;
+        if (vals32.alloc_on(stream, nnz * 2 * vbytes + 1024, "cudaMalloc narrowed values")) return -1;
         float* a32 = nullptr;
         float* at32 = nullptr;
         __nv_bfloat16* a16 = nullptr;
@@ -2208,8 +2203,8 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
         const size_t mf = (static_cast<size_t>(m) * 4 + 255) / 256 * 256;
         const size_t nd = (static_cast<size_t>(n) * 8 + 255) / 256 * 256;
         const size_t md = (static_cast<size_t>(m) * 8 + 255) / 256 * 256;
-        if (blob32.alloc(3 * nf + 2 * mf + 256, "cudaMalloc FP32 frame")) return -1;
-        if (cbuf.alloc(3 * nd + md + 256, "cudaMalloc FP64 center products")) return -1;
+        if (blob32.alloc_on(stream, 3 * nf + 2 * mf + 256, "cudaMalloc FP32 frame")) return -1;
+        if (cbuf.alloc_on(stream, 3 * nd + md + 256, "cudaMalloc FP64 center products")) return -1;
         char* base = blob32.as<char>();
         Centered ctr;
         ctr.A = sc.A;
@@ -2240,13 +2235,13 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
             ctr.grid_q = tiled_grid<StoreEpi>(Qs);
             const size_t qnnz = static_cast<size_t>(Qs.nnz);
             const size_t qv32 = (qnnz * 4 + 255) / 256 * 256;
-            if (q32buf.alloc(qv32 + static_cast<size_t>(n) * 4 + 256, "cudaMalloc FP32 Hessian")) return -1;
+            if (q32buf.alloc_on(stream, qv32 + static_cast<size_t>(n) * 4 + 256, "cudaMalloc FP32 Hessian")) return -1;
             k_narrow<<<sc.sms * 8, kThreads, 0, stream>>>(static_cast<long long>(qnnz), Qs.val, q32buf.as<float>());
             Q32 = Qs.with_values<float>(q32buf.as<float>());
             qd32 = reinterpret_cast<float*>(q32buf.as<char>() + qv32);
             k_narrow<<<eg(n), kThreads, 0, stream>>>(n, qd_s, qd32);
         } else if (qdiag) {
-            if (q32buf.alloc(static_cast<size_t>(n) * 4 + 256, "cudaMalloc FP32 Hessian diagonal")) return -1;
+            if (q32buf.alloc_on(stream, static_cast<size_t>(n) * 4 + 256, "cudaMalloc FP32 Hessian diagonal")) return -1;
             qd32 = q32buf.as<float>();
             k_narrow<<<eg(n), kThreads, 0, stream>>>(n, qd_s, qd32);
         }
@@ -2256,7 +2251,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
         lp.bound_norm = bound_norm;
         auto run_lo = [&](auto& lo, const auto& av, const auto& atv) -> int {
             lo.stream = stream;
-            lo.host = hs.p;
+            lo.host = slot;
             if (lo.allocate(n, m, sc.sms)) return -1;
             if (lo.set_hessian(qd32, hessian ? &Q32 : nullptr)) return -1;
             lo.set_problem(av, atv, ctr.c32, ctr.cl32, ctr.cu32, ctr.rl32, ctr.ru32);
@@ -2277,14 +2272,14 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
         // ------------- Halpern or fixed-step loop: FP32 iterations, then an FP64 finish
         DevBuf vals32, blob32;
         const size_t nnz = static_cast<size_t>(plan->a.nnz);
-        if (vals32.alloc(nnz * 8 + 1024, "cudaMalloc FP32 values")) return -1;
+        if (vals32.alloc_on(stream, nnz * 8 + 1024, "cudaMalloc FP32 values")) return -1;
         float* a32 = vals32.as<float>();
         float* at32 = a32 + (nnz + 63) / 64 * 64;
         k_narrow<<<sc.sms * 8, kThreads, 0, stream>>>(static_cast<long long>(nnz), sc.A.val, a32);
         k_narrow<<<sc.sms * 8, kThreads, 0, stream>>>(static_cast<long long>(nnz), sc.AT.val, at32);
         const size_t nf = (static_cast<size_t>(n) * 4 + 255) / 256 * 256;
         const size_t mf = (static_cast<size_t>(m) * 4 + 255) / 256 * 256;
-        if (blob32.alloc(3 * nf + 2 * mf + 256, "cudaMalloc FP32 model")) return -1;
+        if (blob32.alloc_on(stream, 3 * nf + 2 * mf + 256, "cudaMalloc FP32 model")) return -1;
         char* base = blob32.as<char>();
         float* c32 = reinterpret_cast<float*>(base);
         float* cl32 = reinterpret_cast<float*>(base + nf);
@@ -2299,7 +2294,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
         k_narrow<<<gv, kThreads, 0, stream>>>(m, sc.ru, ru32);
         Core<float> lo;
         lo.stream = stream;
-        lo.host = hs.p;
+        lo.host = slot;
         if (lo.allocate(n, m, sc.sms)) return -1;
         lo.set_problem(sc.A.with_values<float>(a32), sc.AT.with_values<float>(at32), c32, cl32, cu32, rl32, ru32);
         k_narrow<<<gv, kThreads, 0, stream>>>(n, hi.x, lo.x);
@@ -2423,9 +2418,9 @@ extern "C" int sankhya_b200_scale_factors(const SankhyaCudaCSR* matrix, int scal
     if (get_plan(matrix, &plan)) return -1;
     Scaled sc;
     sc.stream = engine_stream();
-    HostSlot hs;
-    B200_TRY(cudaMallocHost(reinterpret_cast<void**>(&hs.p), 64 * sizeof(double)), "cudaMallocHost");
-    sc.host = hs.p;
+    double* slot = pinned_slot();
+    if (!slot) return fail_msg("cudaMallocHost result slot");
+    sc.host = slot;
     if (sc.allocate(*plan)) return -1;
     const int n = matrix->cols, m = matrix->rows;
     const size_t nb = sizeof(double) * static_cast<size_t>(n), mb = sizeof(double) * static_cast<size_t>(m);

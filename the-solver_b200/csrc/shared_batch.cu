@@ -468,7 +468,7 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
     const size_t total = 6 * NB + (c_per_lp ? NB : nb) + 3 * MB + (row_bounds_per_lp ? 2 * MB : 2 * mb) + 2 * nb +
                          2 * mb + 12 * kb + stage + 4096;
     DevBuf blob;
-    if (blob.alloc(total, "cudaMalloc shared batch workspace")) return -1;
+    if (blob.alloc_on(stream, total, "cudaMalloc shared batch workspace")) return -1;
     char* p = blob.as<char>();
     auto take = [&](size_t b) { char* r = p; p += b; return reinterpret_cast<double*>(r); };
     double *xb0 = take(NB), *xb1 = take(NB), *xbar = take(NB), *dcl = take(NB), *dcu = take(NB), *tune = take(NB);
@@ -536,12 +536,8 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
     k_multi_init<<<elem_grid(static_cast<int>(std::min<size_t>(n * bp, 1u << 30))), kThreads, 0, stream>>>(
         n * bp, dcl, dcu, xb0, xbar);
     B200_TRY(cudaGetLastError(), "shared batch setup");
-    unsigned int* host_counters = nullptr;
-    B200_TRY(cudaMallocHost(reinterpret_cast<void**>(&host_counters), 64), "cudaMallocHost");
-    struct Free {
-        unsigned int* p;
-        ~Free() { cudaFreeHost(p); }
-    } free_host{host_counters};
+    unsigned int* host_counters = reinterpret_cast<unsigned int*>(pinned_slot());
+    if (!host_counters) return fail_msg("cudaMallocHost counters");
 
     int shape = s.schedule - 1;
     if (s.schedule == 0) {

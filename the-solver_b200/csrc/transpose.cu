@@ -197,7 +197,7 @@ int device_transpose(int rows, int cols, int nnz, const int* ptr, const int* idx
     auto al = [](long long b) { return (b + 255) / 256 * 256; };
     const long long n4 = al(4LL * std::max(nnz, 1));
     DevBuf buf;
-    if (buf.alloc(static_cast<size_t>(5 * n4 + al(4LL * (cols + 1)) + 2 * al(4LL * (hist_len + 1)) + al(4 * scan_tmp) +
+    if (buf.alloc_on(st, static_cast<size_t>(5 * n4 + al(4LL * (cols + 1)) + 2 * al(4LL * (hist_len + 1)) + al(4 * scan_tmp) +
                                       256),
                   "cudaMalloc transpose scratch"))
         return -1;
