@@ -112,3 +112,36 @@ def test_every_warp_schedule_gives_the_same_bits(engine, instances):
     s.schedule = 4
     rc, *_ = _shared(engine, nodes, s)
     assert rc == -1 and "settings" in engine.last_error()
+
+
+@pytest.mark.parametrize("batch", [1, 2, 31, 33, 63, 65, 130])
+@pytest.mark.parametrize("bounds", ["shared", "per_lp"])
+def test_widths_and_row_lengths(engine, instances, batch, bounds):
+    """Batch widths around a slab (32) and a warp's group (64), and rows of 0 to 14 entries
+    (every remainder of the gather depths), shared column bounds and bounds that differ in
+    some slabs only, against the block-diagonal batch, bit for bit."""
+    rng = np.random.default_rng(batch)
+    m, n = 45, 60
+    deg = np.arange(m) % 15
+    row = np.repeat(np.arange(m), deg)
+    col = np.concatenate([rng.choice(n, size=k, replace=False) for k in deg])
+    ptr, idx, val = instances._csr_from_entries(m, row, col, rng.standard_normal(row.shape[0]))
+    base = instances._finish_lp(rng, m, n, ptr, idx, val)
+    cl, cu = np.tile(base["cl"], (batch, 1)), np.tile(base["cu"], (batch, 1))
+    if bounds == "per_lp":
+        for k in range(0, batch, 40):
+            cl[k, k % n] = cu[k, k % n] = 1.5
+            cu[k, (k + 7) % n] = 1e30
+    nodes = [dict(base, cl=cl[k], cu=cu[k]) for k in range(batch)]
+    blk, rseg, cseg = engine.block_diagonal(nodes)
+    for schedule in (0, 1, 2, 3):
+        s = _settings(engine, 70, 1e-12, 1e-12)
+        s.schedule, s.check_every = schedule, 33
+        box = (cl, cu) if bounds == "per_lp" else (base["cl"], base["cu"])
+        A = engine.Matrix.from_instance(base)
+        rc, x, y, res = engine.shared_batch_pdhg(A, batch, base["c"], base["rl"], base["ru"], *box, s, want_dual=True)
+        assert rc == 0, engine.last_error()
+        rc2, xb, yb, resb = engine.batch_pdhg(engine.Matrix.from_instance(blk), blk, rseg, cseg, s, want_dual=True)
+        assert rc2 == 0, engine.last_error()
+        assert np.array_equal(x.ravel(), xb) and np.array_equal(y.ravel(), yb)
+        assert [r["iterations"] for r in res] == [r["iterations"] for r in resb]

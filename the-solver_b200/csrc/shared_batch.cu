@@ -7,13 +7,21 @@
 //
 // Layout. The per-LP vectors live batch-minor on the device: element j of LP k
 // at j * bp + k, bp = batch rounded up to 32. A row of the shared matrix is read
-// once per iteration for all LPs; its "gathers" become contiguous 256-byte
-// loads of 32 LPs' values (one slab), and a warp carries a few slabs through
-// the row, one LP per lane and slab. Each LP's row sum runs over
+// once per iteration for all LPs; its "gathers" become contiguous 512-byte
+// loads of 64 LPs' values, two LPs a lane. Each LP's row sum runs over
 // the row's entries in stored order with unfused products and adds, the order
 // and rounding of sk_solve's serial CSC loops (and of the single-LP kernels'
 // short-row path), so every LP's iterates equal a separate solve's bit for bit.
-// Costs and row bounds may be given once for all LPs (kept as one vector).
+// Costs and row bounds may be given once for all LPs (kept as one vector). Column bounds
+// are kept per (column, slab of 32 LPs): nodes fix a few variables each, so nearly every
+// slab has one box, and 16 bytes stand for 512. Iterates are updated in place.
+//
+// Measured on a B200 at 1,965 MHz, us per iteration of all LPs: 256 nodes of 5,000 x 10,000
+// (60,000 nonzeros) 57.0 -> 38.0; 32 nodes of it 18.1 -> 16.0; 160 of 2,000 x 4,003 22.1 ->
+// 20.0; 256 of 300 x 600 11.4 -> 10.5. The larger share came from instructions (the shuffles
+// that handed out a row's entries, under tests of whether each exists, were three quarters
+// of them), the rest from the boxes and the in-place update, which keep the working set
+// (50 MB at 256 nodes) in L2. 24 to 32 warps per SM at half of the issue slots remain.
 #include "batch_common.cuh"
 
 #include <algorithm>
@@ -34,89 +42,85 @@ using batch::sk_inf;
 using batch::sk_neg_inf;
 using batch::slot_value;
 
-// Warp shapes: S 32-LP slabs carried by one warp, gathers of A row entries issued
-// together. Every shape sums each LP in stored order, so all give the same bits;
-// the fastest for a (matrix, batch width) is picked by timing (schedule 0) or
-// fixed by the caller (schedule 1..3).
-struct Shape {
-    int slabs, ahead;
-};
-constexpr Shape kShapes[3] = {{1, 8}, {2, 4}, {4, 4}};
+// Gathers a warp has in flight for one row (times 64 LPs). Every depth sums each LP in
+// stored order, so all give the same bits; the fastest for a (matrix, batch width) is
+// picked by timing (schedule 0) or fixed by the caller (schedule 1..3).
+constexpr int kAhead[3] = {3, 4, 6};
 
-// Each epilogue prefetches its per-(row, LP) data into L1 before the gathers
-// (prefetch: no registers held), reads it after them (load) and finishes the step
-// with the row sum (store).
+// The epilogues work on two LPs, k and k + 1 (k even), of one row or column: load reads
+// what they need (before the gathers), store finishes the step with the row sums.
+
+__device__ __forceinline__ double2 ld2(const double* p) { return *reinterpret_cast<const double2*>(p); }
+__device__ __forceinline__ void st2(double* p, double a, double b) { *reinterpret_cast<double2*>(p) = make_double2(a, b); }
+__device__ __forceinline__ double2 both(double v) { return make_double2(v, v); }
 
 // sk_solve.c:901-906 per (row, LP), with LP freezing
 struct MultiDualEpi {
-    const double* __restrict__ y;
+    const double* y;   // may be y_new: each element is read and written by one thread
     const double* __restrict__ rl;
     const double* __restrict__ ru;
     const double* __restrict__ sig;
     const int* __restrict__ done;
-    double* __restrict__ y_new;
+    double* y_new;
     int bp, rows_per_lp;
     struct Row {
-        double y, lo, hi;
-        int frozen;
+        double2 y, lo, hi;
+        double s;
+        int2 frozen;
     };
     __device__ __forceinline__ Row load(int i, int k) const {
-        const size_t e = static_cast<size_t>(i) * bp + k, b = rows_per_lp ? e : static_cast<size_t>(i);
-        return Row{y[e], rl[b], ru[b], done[k]};
-    }
-    __device__ __forceinline__ void prefetch(int i, int k) const {
-        const size_t e = static_cast<size_t>(i) * bp + k, b = rows_per_lp ? e : static_cast<size_t>(i);
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(y + e));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(rl + b));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(ru + b));
-    }
-    __device__ __forceinline__ void store(int i, int k, double act, const Row& r) const {
         const size_t e = static_cast<size_t>(i) * bp + k;
-        if (r.frozen) {
-            y_new[e] = r.y;
-            return;
-        }
-        const double s = sig[i];
-        const double trial = dadd(r.y, dmul(s, act));
-        y_new[e] = dsub(trial, dmul(s, box_sk(ddiv(trial, s), r.lo, r.hi)));
+        return Row{ld2(y + e), rows_per_lp ? ld2(rl + e) : both(__ldg(rl + i)), rows_per_lp ? ld2(ru + e) : both(__ldg(ru + i)),
+                   __ldg(sig + i), *reinterpret_cast<const int2*>(done + k)};
+    }
+    static __device__ __forceinline__ double step(double y, double act, double s, double lo, double hi, int frozen) {
+        const double trial = dadd(y, dmul(s, act));
+        const double next = dsub(trial, dmul(s, box_sk(ddiv(trial, s), lo, hi)));
+        return frozen ? y : next;
+    }
+    __device__ __forceinline__ void store(int i, int k, double2 act, const Row& r) const {
+        st2(y_new + static_cast<size_t>(i) * bp + k, step(r.y.x, act.x, r.s, r.lo.x, r.hi.x, r.frozen.x),
+            step(r.y.y, act.y, r.s, r.lo.y, r.hi.y, r.frozen.y));
     }
 };
 
 // sk_solve.c:918-923 (LP, no Q) per (column, LP), with LP freezing
 struct MultiPrimalEpi {
-    const double* __restrict__ x;
+    const double* x;   // may be x_new
     const double* __restrict__ c;
     const double* __restrict__ tau;
-    const double* __restrict__ cl;
+    const double2* __restrict__ box;   // (lower, upper) per column and slab
+    const double* __restrict__ cl;     // per LP, where a slab's box differs (its lower is NaN)
     const double* __restrict__ cu;
     const int* __restrict__ done;
-    double* __restrict__ x_new;
-    double* __restrict__ x_bar;
+    double* x_new;
+    double* x_bar;
     int bp, c_per_lp;
     struct Row {
-        double x, c, lo, hi;
-        int frozen;
+        double2 x, c, box;
+        double t;
+        int2 frozen;
     };
     __device__ __forceinline__ Row load(int j, int k) const {
         const size_t e = static_cast<size_t>(j) * bp + k;
-        return Row{x[e], c[c_per_lp ? e : static_cast<size_t>(j)], cl[e], cu[e], done[k]};
+        return Row{ld2(x + e), c_per_lp ? ld2(c + e) : both(__ldg(c + j)),
+                   __ldg(box + static_cast<size_t>(j) * (bp >> 5) + (k >> 5)), __ldg(tau + j),
+                   *reinterpret_cast<const int2*>(done + k)};
     }
-    __device__ __forceinline__ void prefetch(int j, int k) const {
-        const size_t e = static_cast<size_t>(j) * bp + k;
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(x + e));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(cl + e));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(cu + e));
+    static __device__ __forceinline__ double step(double x, double g, double c, double t, double lo, double hi) {
+        return box_sk(dsub(x, dmul(t, dadd(dadd(c, 0.0), g))), lo, hi);
     }
-    __device__ __forceinline__ void store(int j, int k, double g, const Row& r) const {
+    __device__ __forceinline__ void store(int j, int k, double2 g, const Row& r) const {
         const size_t e = static_cast<size_t>(j) * bp + k;
-        if (r.frozen) {
-            x_new[e] = r.x;
-            return;
+        double2 lo = both(r.box.x), hi = both(r.box.y);
+        if (isnan(r.box.x)) {   // tested here, behind the gathers, where the box has arrived
+            lo = ld2(cl + e);
+            hi = ld2(cu + e);
         }
-        double xn = dsub(r.x, dmul(tau[j], dadd(dadd(r.c, 0.0), g)));
-        xn = box_sk(xn, r.lo, r.hi);
-        x_new[e] = xn;
-        x_bar[e] = dsub(dmul(2.0, xn), r.x);
+        const double a = step(r.x.x, g.x, r.c.x, r.t, lo.x, hi.x), b = step(r.x.y, g.y, r.c.y, r.t, lo.y, hi.y);
+        st2(x_new + e, r.frozen.x ? r.x.x : a, r.frozen.y ? r.x.y : b);
+        if (!r.frozen.x) x_bar[e] = dsub(dmul(2.0, a), r.x.x);
+        if (!r.frozen.y) x_bar[e + 1] = dsub(dmul(2.0, b), r.x.y);
     }
 };
 
@@ -125,65 +129,90 @@ struct MultiStoreEpi {
     int bp;
     struct Row {};
     __device__ __forceinline__ Row load(int, int) const { return {}; }
-    __device__ __forceinline__ void prefetch(int, int) const {}
-    __device__ __forceinline__ void store(int i, int k, double s, const Row&) const {
-        out[static_cast<size_t>(i) * bp + k] = s;
+    __device__ __forceinline__ void store(int i, int k, double2 s, const Row&) const {
+        st2(out + static_cast<size_t>(i) * bp + k, s.x, s.y);
     }
 };
 
-// One warp per (row, group of 32 S LPs): out(r, k) = sum_p a_p v[col_p, k] in
-// stored order for every LP k of the group. The gathers of AH entries are issued
-// before their products are added, in order, to each LP's sum.
-template <class Epi, int S, int AH>
-__global__ void __launch_bounds__(kThreads) k_multi(int rows, int groups, int bp, const int* __restrict__ ptr,
-                                                    const int* __restrict__ idx, const double* __restrict__ val,
-                                                    const double* __restrict__ v, Epi epi) {
-    const unsigned full = 0xffffffffu;
+// One warp per (row, group of 64 LPs), two LPs a lane: out(r, k) = sum_p a_p v[col_p, k] in
+// stored order for every LP k of the group. The gathers of AH entries go out together; the
+// epilogue's data goes out before them and the entries of the warp's next unit are pulled
+// into L1 meanwhile, so that a unit's chain is one or two gather latencies. All lanes read
+// the entries themselves (one broadcast load each): shuffles under the tests of whether an
+// entry exists took three times the instructions.
+// Off: unsigned while an element's offset fits 32 bits.
+template <class Epi, int AH, class Off>
+__global__ void __launch_bounds__(kThreads, AH <= 4 ? 4 : 3) k_multi(int rows, int groups, int bp,
+                                                                      const int* __restrict__ ptr,
+                                                                      const int* __restrict__ idx,
+                                                                      const double* __restrict__ val,
+                                                                      const double* __restrict__ v, Epi epi) {
     const int lane = threadIdx.x & 31;
-    const long long units = static_cast<long long>(rows) * groups;
-    const long long nw = static_cast<long long>(gridDim.x) * kWarps;
-    for (long long u = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5); u < units; u += nw) {
-        const int r = static_cast<int>(u / groups), g = static_cast<int>(u % groups);
-        const int k0 = g * 32 * S;
-        const int ns = min(S, (bp - k0) >> 5);
+    const int nw = gridDim.x * kWarps, u = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const int dr = nw / groups, dg = nw % groups;
+    int r = u / groups, g = u % groups;
+    if (r >= rows) return;
+    int p0 = __ldg(ptr + r), p1 = __ldg(ptr + r + 1);
+    for (;;) {
+        int rn = r + dr, gn = g + dg;
+        if (gn >= groups) {
+            gn -= groups;
+            ++rn;
+        }
+        int n0 = 0, n1 = 0;
+        if (rn < rows) {
+            n0 = __ldg(ptr + rn);
+            n1 = __ldg(ptr + rn + 1);
+        }
+        const int k = 64 * g + 2 * lane;
+        const bool live = k < bp;
+        const double* vk = v + (live ? k : 0);
+        typename Epi::Row pre{};
+        if (live) pre = epi.load(r, k);
+        double2 acc = make_double2(0.0, 0.0);
+        int p = p0;
+        for (; p + AH <= p1; p += AH) {
+            Off at[AH];
+            double a[AH];
+            double2 w[AH];
 #pragma unroll
-        for (int s = 0; s < S; ++s)
-            if (s < ns) epi.prefetch(r, k0 + 32 * s + lane);
-        double acc[S];
+            for (int q = 0; q < AH; ++q) at[q] = static_cast<Off>(__ldg(idx + p + q)) * static_cast<Off>(bp);
 #pragma unroll
-        for (int s = 0; s < S; ++s) acc[s] = 0.0;
-        const int p0 = __ldg(ptr + r), p1 = __ldg(ptr + r + 1);
-        for (int pb = p0; pb < p1; pb += 32) {
-            const int cnt = min(32, p1 - pb);
-            int ci = 0;
-            double ai = 0.0;
-            if (lane < cnt) {
-                ci = __ldg(idx + pb + lane);
-                ai = __ldg(val + pb + lane);
-            }
-            for (int e0 = 0; e0 < cnt; e0 += AH) {
-                double g8[AH][S];
+            for (int q = 0; q < AH; ++q) w[q] = __ldg(reinterpret_cast<const double2*>(vk + at[q]));
 #pragma unroll
-                for (int q = 0; q < AH; ++q) {
-                    const int col = __shfl_sync(full, ci, min(e0 + q, 31));
-                    const double* src = v + static_cast<size_t>(col) * bp + k0 + lane;
+            for (int q = 0; q < AH; ++q) a[q] = __ldg(val + p + q);
 #pragma unroll
-                    for (int s = 0; s < S; ++s)
-                        g8[q][s] = (e0 + q < cnt && s < ns) ? __ldg(src + 32 * s) : 0.0;
-                }
-#pragma unroll
-                for (int q = 0; q < AH; ++q) {
-                    const double a = __shfl_sync(full, ai, min(e0 + q, 31));
-                    if (e0 + q < cnt) {
-#pragma unroll
-                        for (int s = 0; s < S; ++s) acc[s] = dadd(acc[s], dmul(a, g8[q][s]));
-                    }
-                }
+            for (int q = 0; q < AH; ++q) {
+                acc.x = dadd(acc.x, dmul(a[q], w[q].x));
+                acc.y = dadd(acc.y, dmul(a[q], w[q].y));
             }
         }
+        if (p < p1) {
+            double a[AH];
+            double2 w[AH];
 #pragma unroll
-        for (int s = 0; s < S; ++s)
-            if (s < ns) epi.store(r, k0 + 32 * s + lane, acc[s], epi.load(r, k0 + 32 * s + lane));
+            for (int q = 0; q + 1 < AH; ++q)
+                if (p + q < p1) {
+                    a[q] = __ldg(val + p + q);
+                    w[q] = __ldg(reinterpret_cast<const double2*>(vk + static_cast<Off>(__ldg(idx + p + q)) * static_cast<Off>(bp)));
+                }
+#pragma unroll
+            for (int q = 0; q + 1 < AH; ++q)
+                if (p + q < p1) {
+                    acc.x = dadd(acc.x, dmul(a[q], w[q].x));
+                    acc.y = dadd(acc.y, dmul(a[q], w[q].y));
+                }
+        }
+        if (n0 + 16 * lane < n1) {   // a line of values (and of indices) per 16 entries
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(idx + n0 + 16 * lane));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(val + n0 + 16 * lane));
+        }
+        if (live) epi.store(r, k, acc, pre);
+        if (rn >= rows) return;
+        r = rn;
+        g = gn;
+        p0 = n0;
+        p1 = n1;
     }
 }
 
@@ -216,12 +245,42 @@ __global__ void k_from_batch_minor(int len, int batch, int bp, const double* __r
     }
 }
 
+// The boxes of every column by slab: the bounds its 32 LPs share, bit for bit (LPs past the
+// batch aside), or NaN for the lower where they differ. One warp per (column, slab).
+__global__ void k_slab_boxes(int n, int batch, int bp, const double* __restrict__ cl, const double* __restrict__ cu,
+                             double2* __restrict__ box) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, slabs = bp >> 5;
+    const long long units = static_cast<long long>(n) * slabs;
+    for (long long u = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5); u < units;
+         u += static_cast<long long>(gridDim.x) * kWarps) {
+        const int k = static_cast<int>(u % slabs) * 32 + lane;
+        const size_t e = static_cast<size_t>(u / slabs) * bp + k;
+        const double lo = cl[e], hi = cu[e], lo0 = __shfl_sync(full, lo, 0), hi0 = __shfl_sync(full, hi, 0);
+        const bool same = k >= batch || (__double_as_longlong(lo) == __double_as_longlong(lo0) &&
+                                         __double_as_longlong(hi) == __double_as_longlong(hi0));
+        if (__all_sync(full, same) ? lane == 0 : false) box[u] = make_double2(lo0, hi0);
+        else if (lane == 0) box[u] = make_double2(__longlong_as_double(0x7ff8000000000000ll), 0.0);
+    }
+}
+
+// The same for bounds shared by all LPs.
+__global__ void k_shared_boxes(int n, int slabs, const double* __restrict__ cl, const double* __restrict__ cu,
+                               double2* __restrict__ box) {
+    const long long units = static_cast<long long>(n) * slabs;
+    for (long long u = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; u < units;
+         u += static_cast<long long>(blockDim.x) * gridDim.x)
+        box[u] = make_double2(cl[u / slabs], cu[u / slabs]);
+}
+
 // Initial point of every LP (sk_solve.c:882-884): x = box(0), x_bar = x.
-__global__ void k_multi_init(size_t total, const double* __restrict__ cl, const double* __restrict__ cu,
-                             double* __restrict__ x, double* __restrict__ x_bar) {
+__global__ void k_multi_init(size_t total, int bp, const double2* __restrict__ box, const double* __restrict__ cl,
+                             const double* __restrict__ cu, double* __restrict__ x, double* __restrict__ x_bar) {
     for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < total;
          e += static_cast<size_t>(blockDim.x) * gridDim.x) {
-        const double v = box_sk(0.0, cl[e], cu[e]);
+        double2 b = box[e >> 5];   // (column, slab) of element (column, LP): bp is a multiple of 32
+        if (isnan(b.x)) b = make_double2(cl[e], cu[e]);
+        const double v = box_sk(0.0, b.x, b.y);
         x[e] = v;
         x_bar[e] = v;
     }
@@ -349,22 +408,26 @@ __global__ void k_mark_padding(int batch, int bp, int* __restrict__ done) {
     if (k < bp) done[k] = 1;
 }
 
-template <class Epi, int S, int AH>
-void launch_shape(int rows, int bp, const TileCsr& M, const double* v, const Epi& epi, cudaStream_t st) {
+template <class Epi, int AH, class Off>
+void launch_ahead(int rows, int bp, const TileCsr& M, const double* v, const Epi& epi, cudaStream_t st) {
     if (rows == 0) return;
-    const int groups = (bp + 32 * S - 1) / (32 * S);
+    const int groups = (bp + 63) / 64;
     const long long blocks = (static_cast<long long>(rows) * groups + kWarps - 1) / kWarps;
-    const int grid = grid_for(reinterpret_cast<const void*>(&k_multi<Epi, S, AH>),
+    const int grid = grid_for(reinterpret_cast<const void*>(&k_multi<Epi, AH, Off>),
                               static_cast<int>(std::min<long long>(blocks, 1 << 30)), 0);
-    k_multi<Epi, S, AH><<<grid, kThreads, 0, st>>>(rows, groups, bp, M.ptr, M.idx, M.val, v, epi);
+    k_multi<Epi, AH, Off><<<grid, kThreads, 0, st>>>(rows, groups, bp, M.ptr, M.idx, M.val, v, epi);
 }
 
 template <class Epi>
 void launch_multi(int shape, int rows, int bp, const TileCsr& M, const double* v, const Epi& epi, cudaStream_t st) {
+    if (static_cast<long long>(M.cols) * bp > 0xffffffffll) {
+        launch_ahead<Epi, kAhead[1], size_t>(rows, bp, M, v, epi, st);
+        return;
+    }
     switch (shape) {
-        case 0: launch_shape<Epi, kShapes[0].slabs, kShapes[0].ahead>(rows, bp, M, v, epi, st); break;
-        case 1: launch_shape<Epi, kShapes[1].slabs, kShapes[1].ahead>(rows, bp, M, v, epi, st); break;
-        default: launch_shape<Epi, kShapes[2].slabs, kShapes[2].ahead>(rows, bp, M, v, epi, st); break;
+        case 0: launch_ahead<Epi, kAhead[0], unsigned>(rows, bp, M, v, epi, st); break;
+        case 1: launch_ahead<Epi, kAhead[1], unsigned>(rows, bp, M, v, epi, st); break;
+        default: launch_ahead<Epi, kAhead[2], unsigned>(rows, bp, M, v, epi, st); break;
     }
 }
 
@@ -463,15 +526,19 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
     const size_t nb = al(sizeof(double) * n), mb = al(sizeof(double) * static_cast<size_t>(m));
     const size_t kb = al(sizeof(double) * bp);
     const size_t stage = std::max(NB, MB);
-    // batch-minor: x[2], x_bar, cl, cu, (c); y[2], act, (rl, ru); shared: tau, cmass,
-    // sig, rmass, (c), (rl, ru); per-LP slots; staging for the layout changes
-    const size_t total = 6 * NB + (c_per_lp ? NB : nb) + 3 * MB + (row_bounds_per_lp ? 2 * MB : 2 * mb) + 2 * nb +
+    const bool tuned = s.schedule == 0;
+    const size_t CB = col_bounds_per_lp ? NB : nb;
+    // batch-minor: x, x_bar, (cl, cu), (c); y[2], act, (rl, ru); shared: boxes, tau, cmass,
+    // sig, rmass, (c), (cl, cu), (rl, ru); per-LP slots; staging for the layout changes
+    const size_t total = 2 * NB + 2 * CB + (tuned ? NB : 0) + al(bp / 32 * n * sizeof(double2)) +
+                         (c_per_lp ? NB : nb) + 3 * MB + (row_bounds_per_lp ? 2 * MB : 2 * mb) + 2 * nb +
                          2 * mb + 12 * kb + stage + 4096;
     DevBuf blob;
     if (blob.alloc_on(stream, total, "cudaMalloc shared batch workspace")) return -1;
     char* p = blob.as<char>();
     auto take = [&](size_t b) { char* r = p; p += b; return reinterpret_cast<double*>(r); };
-    double *xb0 = take(NB), *xb1 = take(NB), *xbar = take(NB), *dcl = take(NB), *dcu = take(NB), *tune = take(NB);
+    double *x = take(NB), *xbar = take(NB), *dcl = take(CB), *dcu = take(CB), *tune = take(tuned ? NB : 0);
+    double2* box = reinterpret_cast<double2*>(take(al(bp / 32 * n * sizeof(double2))));
     double* dc = take(c_per_lp ? NB : nb);
     double *yb0 = take(MB), *yb1 = take(MB), *act = take(MB);
     double* drl = take(row_bounds_per_lp ? MB : mb);
@@ -503,23 +570,14 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
         k_to_batch_minor<<<dim3((len + 31) / 32, bpi / 32), tblock, 0, stream>>>(len, batch, bpi, staging, dst);
         return 0;
     };
-    // a shared vector replicated into every LP's slot (column bounds are per LP inside)
-    auto upload_replicated = [&](const double* host, int len, double* dst) -> int {
-        if (len == 0) return 0;
-        std::vector<double> rep(static_cast<size_t>(batch) * len);
-        for (int k = 0; k < batch; ++k) std::memcpy(rep.data() + static_cast<size_t>(k) * len, host, sizeof(double) * len);
-        B200_TRY(cudaMemcpyAsync(staging, rep.data(), sizeof(double) * rep.size(), cudaMemcpyHostToDevice, stream),
-                 "upload");
-        k_to_batch_minor<<<dim3((len + 31) / 32, bpi / 32), tblock, 0, stream>>>(len, batch, bpi, staging, dst);
-        B200_TRY(cudaStreamSynchronize(stream), "upload");
-        return 0;
-    };
     if (upload(c, n, c_per_lp != 0, dc)) return -1;
-    if (col_bounds_per_lp) {
-        if (upload(clow, n, true, dcl) || upload(cupp, n, true, dcu)) return -1;
-    } else {
-        if (upload_replicated(clow, n, dcl) || upload_replicated(cupp, n, dcu)) return -1;
-    }
+    if (upload(clow, n, col_bounds_per_lp != 0, dcl) || upload(cupp, n, col_bounds_per_lp != 0, dcu)) return -1;
+    const int slabs = bpi / 32;
+    if (col_bounds_per_lp)
+        k_slab_boxes<<<elem_grid(static_cast<int>(std::min<size_t>(n * bp, 1u << 30))), kThreads, 0, stream>>>(
+            n, batch, bpi, dcl, dcu, box);
+    else
+        k_shared_boxes<<<elem_grid(n), kThreads, 0, stream>>>(n, slabs, dcl, dcu, box);
     if (upload(rlow, m, row_bounds_per_lp != 0, drl) || upload(rupp, m, row_bounds_per_lp != 0, dru)) return -1;
     if (m) B200_TRY(cudaMemsetAsync(yb0, 0, MB, stream), "zero y");
     B200_TRY(cudaMemsetAsync(viol, 0, 6 * kb, stream), "zero slots");
@@ -534,7 +592,7 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
     k_mass_steps<<<elem_grid(n), kThreads, 0, stream>>>(n, cmass, tau);
     if (m) k_mass_steps<<<elem_grid(m), kThreads, 0, stream>>>(m, rmass, sig);
     k_multi_init<<<elem_grid(static_cast<int>(std::min<size_t>(n * bp, 1u << 30))), kThreads, 0, stream>>>(
-        n * bp, dcl, dcu, xb0, xbar);
+        n * bp, bpi, box, dcl, dcu, x, xbar);
     B200_TRY(cudaGetLastError(), "shared batch setup");
     unsigned int* host_counters = reinterpret_cast<unsigned int*>(pinned_slot());
     if (!host_counters) return fail_msg("cudaMallocHost counters");
@@ -545,30 +603,31 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
         // the staging buffer and the tuning buffer; iterates untouched
         shape = autotuned_shape(A, AT, bpi,
                                 MultiDualEpi{yb0, drl, dru, sig, done, act, bpi, row_bounds_per_lp ? 1 : 0}, xbar,
-                                MultiPrimalEpi{xb0, dc, tau, dcl, dcu, done, staging, tune, bpi, c_per_lp ? 1 : 0},
+                                MultiPrimalEpi{x, dc, tau, box, dcl, dcu, done, staging, tune, bpi, c_per_lp ? 1 : 0},
                                 yb0, stream);
         B200_TRY(cudaGetLastError(), "shared batch schedule");
     }
     const dim3 check_rows(static_cast<unsigned>(std::max(1, std::min((m + 7) / 8, 4 * 148 * 8 * 32 / bpi))), bpi / 32);
     const dim3 check_cols(static_cast<unsigned>(std::max(1, std::min((n + 7) / 8, 4 * 148 * 8 * 32 / bpi))), bpi / 32);
-    double* xb[2] = {xb0, xb1};
     double* yb[2] = {yb0, yb1};
-    std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
+    std::map<std::tuple<int, int, bool>, cudaGraphExec_t> graphs;
     struct Graphs {
-        std::map<std::pair<int, int>, cudaGraphExec_t>* g;
+        std::map<std::tuple<int, int, bool>, cudaGraphExec_t>* g;
         ~Graphs() {
             for (auto& kv : *g)
                 if (kv.second) cudaGraphExecDestroy(kv.second);
         }
     } graphs_guard{&graphs};
     int cur = 0, it = 0, launches = 0;
-    auto iterate = [&]() {
-        const int nx = cur ^ 1;
+    // In place, so that x, x_bar and y (50 MB at 256 LPs of 5,000 x 10,000) stay in L2; only
+    // the iteration before a check keeps the y it started from.
+    auto iterate = [&](bool keep) {
+        const int nx = keep ? cur ^ 1 : cur;
         launch_multi(shape, m, bpi, A, xbar, MultiDualEpi{yb[cur], drl, dru, sig, done, yb[nx], bpi,
                                                            row_bounds_per_lp ? 1 : 0},
                      stream);
         launch_multi(shape, n, bpi, AT, yb[nx],
-                     MultiPrimalEpi{xb[cur], dc, tau, dcl, dcu, done, xb[nx], xbar, bpi, c_per_lp ? 1 : 0}, stream);
+                     MultiPrimalEpi{x, dc, tau, box, dcl, dcu, done, x, xbar, bpi, c_per_lp ? 1 : 0}, stream);
         cur = nx;
     };
     bool timed_out = false;
@@ -579,13 +638,14 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
         int k = next - it;
         while (k > 0) {
             const int chunk = std::min(k, 64);
-            auto key = std::make_pair(chunk, cur);
+            const bool last = chunk == k;   // ends at the check
+            auto key = std::make_tuple(chunk, cur, last);
             auto g = graphs.find(key);
             if (g == graphs.end()) {
                 const int saved = cur;
                 cudaGraph_t graph;
                 B200_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-                for (int i = 0; i < chunk; ++i) iterate();
+                for (int i = 0; i < chunk; ++i) iterate(last && i + 1 == chunk);
                 B200_TRY(cudaStreamEndCapture(stream, &graph), "end capture");
                 cudaGraphExec_t exec;
                 cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
@@ -596,7 +656,7 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
             }
             B200_TRY(cudaGraphLaunch(g->second, stream), "graph launch");
             launches += (m ? 2 : 1) * chunk;
-            cur ^= (chunk & 1);
+            if (last) cur ^= 1;
             k -= chunk;
         }
         it = next;
@@ -604,11 +664,11 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
         ++checks;
         B200_TRY(cudaMemsetAsync(counters, 0, 4, stream), "zero counter");
         if (m) {
-            launch_multi(shape, m, bpi, A, xb[cur], MultiStoreEpi{act, bpi}, stream);
+            launch_multi(shape, m, bpi, A, x, MultiStoreEpi{act, bpi}, stream);
             k_multi_rows_check<<<check_rows, tblock, 0, stream>>>(m, bpi, row_bounds_per_lp ? 1 : 0, act, yb[cur],
                                                                   yb[cur ^ 1], drl, dru, done, viol, dstep);
         }
-        k_multi_cols_check<<<check_cols, tblock, 0, stream>>>(n, bpi, xb[cur], xbar, done, scale, step);
+        k_multi_cols_check<<<check_cols, tblock, 0, stream>>>(n, bpi, x, xbar, done, scale, step);
         k_multi_gate<<<elem_grid(batch), kThreads, 0, stream>>>(batch, it, last ? 1 : 0, s.primal_tol, s.dual_tol,
                                                                 viol, dstep, scale, step, massmax, done, iters,
                                                                 report, counters);
@@ -624,7 +684,7 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
     const double loop_ms = loop_events.stop(stream);
     std::vector<int> h_done(static_cast<size_t>(batch)), h_iters(static_cast<size_t>(batch));
     std::vector<double> h_report(static_cast<size_t>(batch) * 4);
-    k_from_batch_minor<<<dim3((n + 31) / 32, bpi / 32), tblock, 0, stream>>>(n, batch, bpi, xb[cur], staging);
+    k_from_batch_minor<<<dim3((n + 31) / 32, bpi / 32), tblock, 0, stream>>>(n, batch, bpi, x, staging);
     B200_TRY(cudaMemcpyAsync(x_out, staging, sizeof(double) * static_cast<size_t>(batch) * n, cudaMemcpyDeviceToHost,
                              stream),
              "download x");
