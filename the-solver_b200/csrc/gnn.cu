@@ -17,9 +17,10 @@
 // tensor cores, tcgen05.mma with a TMEM accumulator (tc_gemm.cuh), and so are
 // the weight gradients of the 128-wide layers, which reduce over all nodes in
 // fixed node slices; the 16-wide input layers' weight gradients and any operand
-// that is not 16-byte aligned take an mma.sync m16n8k16 kernel. They are
-// HBM-bound streams of the activations, not tensor-throughput-bound. Aggregations are fp32 gathers over the stored A
-// and A' (warp per node, 64 channels, entries in stored order). Every reduction
+// that is not 16-byte aligned take mma.sync m16n8k16 kernels. They are HBM-bound
+// streams of the activations, not tensor-throughput-bound. Aggregations are fp32
+// gathers over the stored A and A' (warp per node, 64 channels, entries in stored
+// order). Every reduction
 // (weight gradients split over K, bias sums, head sums, loss) has a fixed order,
 // so a training run is reproducible bit for bit.
 #include "batch_common.cuh"
@@ -29,6 +30,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -45,6 +47,7 @@ constexpr int kF = 16;          // input features per node
 constexpr int kX = 2 * kH;      // row width of a layer input [H | aggregation]
 constexpr int kGemmThreads = 128;
 constexpr int kRedBlocks = 296; // partial sums per reduction (2 per SM)
+constexpr int kInputSlices = 296; // partial sums of an input layer's gradients (2 per SM)
 
 // ----------------------------------------------------------------- GEMM
 
@@ -193,16 +196,23 @@ void sum_slices(int count, int slices, long long stride, const float* part, floa
 // --------------------------------------------------------- aggregation
 
 // out[r][c] (+)= post[r] sum_p a_p pre[col_p] in[col_p][c], c < 64: one warp per
-// row, two channels per lane, entries in stored order.
+// row, two channels per lane, entries in stored order. What bounds it is the 256 bytes
+// gathered per entry, from L2 (7.5 TB/s at 1M entries). With `h` (backward) the sum, with
+// what `prev` holds, goes through the relu of the layer that produced h and is stored as
+// the dense dz [rows x 64]: a pass of its own for that took 15 us a layer at 100,000 rows.
 __global__ void __launch_bounds__(kThreads) k_spmm64(int rows, const int* __restrict__ ptr, const int* __restrict__ idx,
                                                      const double* __restrict__ val, const float* __restrict__ in,
                                                      int sin, const float* __restrict__ pre,
                                                      const float* __restrict__ post, float* __restrict__ out, int sout,
-                                                     int accumulate) {
+                                                     const float* __restrict__ prev, const float* __restrict__ h) {
     const int lane = threadIdx.x & 31;
     for (long long r = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5); r < rows;
          r += static_cast<long long>(gridDim.x) * kWarps) {
-        float2 acc = make_float2(0.f, 0.f);
+        float2 acc = make_float2(0.f, 0.f), was = acc, act = acc;
+        if (h) {
+            was = *reinterpret_cast<const float2*>(prev + r * kX + 2 * lane);
+            act = *reinterpret_cast<const float2*>(h + r * kX + 2 * lane);
+        }
         const int p1 = ptr[r + 1];
         for (int p = ptr[r]; p < p1; ++p) {
             const int col = idx[p];
@@ -216,38 +226,81 @@ __global__ void __launch_bounds__(kThreads) k_spmm64(int rows, const int* __rest
             acc.x *= post[r];
             acc.y *= post[r];
         }
-        float2* o = reinterpret_cast<float2*>(out + r * sout + 2 * lane);
-        if (accumulate) {
-            const float2 prev = *o;
-            acc.x += prev.x;
-            acc.y += prev.y;
+        if (h) {
+            acc.x = act.x > 0.f ? acc.x + was.x : 0.f;
+            acc.y = act.y > 0.f ? acc.y + was.y : 0.f;
         }
-        *o = acc;
+        *reinterpret_cast<float2*>(out + r * sout + 2 * lane) = acc;
     }
 }
 
-// dz[i][c] = dh[i][c] where h[i][c] > 0, else 0 (relu backward).
-__global__ void k_relu_mask(int rows, const float* __restrict__ dh, int sdh, const float* __restrict__ h, int sh,
-                            float* __restrict__ dz) {
-    const long long total = static_cast<long long>(rows) * kH;
-    for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
-         e += static_cast<long long>(blockDim.x) * gridDim.x) {
-        const long long i = e / kH;
-        const int c = static_cast<int>(e % kH);
-        dz[e] = h[i * sh + c] > 0.f ? dh[i * sdh + c] : 0.f;
-    }
-}
+// Gradients of an input layer (16 features): part[b][f * 64 + c] = sum over block b's nodes
+// of F[i][f] dz[i][c], operands in bf16 and sums in fp32, and part[b][16 * 64 + c] = the
+// fp32 sum of dz[i][c]; dz = dh where h > 0 (h null: dh). One pass over dh in place of a
+// relu pass, a bias pass and a 64 x 64 tile kernel that filled a quarter of its tile (45 us
+// at 100,000 nodes); bounded by reading dh and h. A warp takes 16 nodes a step as the K of
+// eight m16n8k16 products (features x 8 channels each), its operands loaded straight in
+// fragment order: a load covers 4 nodes x 8 consecutive channels, whole sectors.
+constexpr int kInputOut = kF * kH + kH;
 
-// Per-block column sums of dz [rows x 64] (block b: rows b, b + gridDim.x, ...,
-// four row phases reduced in order): part[b][c].
-__global__ void k_colsum64(int rows, const float* __restrict__ dz, float* __restrict__ part) {
-    __shared__ float s[4][kH];
-    const int c = threadIdx.x & (kH - 1), q = threadIdx.x >> 6;
-    float acc = 0.f;
-    for (long long i = blockIdx.x * 4LL + q; i < rows; i += 4LL * gridDim.x) acc += dz[i * kH + c];
-    s[q][c] = acc;
+__global__ void __launch_bounds__(kThreads) k_input_grad(int rows, const float* __restrict__ F,
+                                                         const float* __restrict__ dh, int sdh,
+                                                         const float* __restrict__ h, float* __restrict__ part) {
+    __shared__ float red[kWarps][kInputOut];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g4 = lane >> 2, t4 = lane & 3;
+    float acc[8][4], bias[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        bias[j] = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+    }
+    auto pair = [](float lo, float hi) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<const unsigned*>(&v);
+    };
+    for (int i0 = (blockIdx.x * kWarps + warp) * 16; i0 < rows; i0 += gridDim.x * kWarps * 16) {
+        float f[4][2], z[8][4];   // nodes 2 t4, 2 t4 + 1, 2 t4 + 8, 2 t4 + 9
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const long long i = i0 + 2 * t4 + (q & 1) + 8 * (q >> 1);
+            const bool live = i < rows;
+            f[q][0] = live ? F[i * kF + g4] : 0.f;
+            f[q][1] = live ? F[i * kF + g4 + 8] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) z[j][q] = live ? dh[i * sdh + 8 * j + g4] : 0.f;
+        }
+        if (h) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const long long i = i0 + 2 * t4 + (q & 1) + 8 * (q >> 1);
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (!(i < rows && h[i * kX + 8 * j + g4] > 0.f)) z[j][q] = 0.f;
+            }
+        }
+        const unsigned a0 = pair(f[0][0], f[1][0]), a1 = pair(f[0][1], f[1][1]);
+        const unsigned a2 = pair(f[2][0], f[3][0]), a3 = pair(f[2][1], f[3][1]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            bias[j] += (z[j][0] + z[j][1]) + (z[j][2] + z[j][3]);
+            mma_bf16(acc[j], a0, a1, a2, a3, pair(z[j][0], z[j][1]), pair(z[j][2], z[j][3]));
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        bias[j] += __shfl_xor_sync(0xffffffffu, bias[j], 1);
+        bias[j] += __shfl_xor_sync(0xffffffffu, bias[j], 2);
+        if (t4 == 0) red[warp][kF * kH + 8 * j + g4] = bias[j];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) red[warp][(g4 + 8 * (e >> 1)) * kH + 8 * j + 2 * t4 + (e & 1)] = acc[j][e];
+    }
     __syncthreads();
-    if (q == 0) part[blockIdx.x * kH + c] = ((s[0][c] + s[1][c]) + s[2][c]) + s[3][c];
+    for (int e = threadIdx.x; e < kInputOut; e += kThreads) {
+        float t = red[0][e];
+        for (int w = 1; w < kWarps; ++w) t += red[w][e];
+        part[static_cast<long long>(blockIdx.x) * kInputOut + e] = t;
+    }
 }
 
 // ------------------------------------------------------------ features
@@ -354,7 +407,8 @@ __global__ void k_features(int m, int n, const double* __restrict__ c, const dou
 // ---------------------------------------------------------------- heads
 
 // Warp per node. s = h . w + b (fp32, lanes' two channels then an xor tree).
-// With a target: loss term, dh = ds w into dh (row stride sdh), and per-block
+// With a target: loss term, dh = ds w (through the relu that produced h, on request) into
+// dh (row stride sdh), and per-block
 // partials part[b][0..63] = sum ds h, part[b][64] = sum ds, part[b][65] = loss.
 struct HeadArgs {
     int rows;
@@ -371,56 +425,88 @@ struct HeadArgs {
     float* dh;
     int sdh;
     float* part;
+    int relu;               // dh masked by h > 0
 };
+
+// Eight rows of a warp at a time: their loads and their sums' shuffles overlap, and lane q
+// does the FP64 part (a sigmoid) of row q; one row at a time every lane repeated it and the
+// warp waited out each step (51 us at 100,000 rows). The partial sums keep the row order.
+constexpr int kHeadRows = 8;
 
 __global__ void __launch_bounds__(kThreads) k_head(HeadArgs a) {
     __shared__ float red[kWarps][kH + 2];
+    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float w0 = a.w[2 * lane], w1 = a.w[2 * lane + 1], wb = a.w[kH];
     float g0 = 0.f, g1 = 0.f, gb = 0.f, gl = 0.f;
     const double inv_count = 1.0 / static_cast<double>(max(a.rows, 1));
     const double bs = a.is_x ? *a.bs : 1.0;
-    for (long long r = static_cast<long long>(blockIdx.x) * kWarps + warp; r < a.rows;
-         r += static_cast<long long>(gridDim.x) * kWarps) {
-        const float2 hv = *reinterpret_cast<const float2*>(a.h + r * a.sh + 2 * lane);
-        float s = hv.x * w0 + hv.y * w1;
+    const long long stride = static_cast<long long>(gridDim.x) * kWarps;
+    for (long long r0 = static_cast<long long>(blockIdx.x) * kWarps + warp; r0 < a.rows; r0 += kHeadRows * stride) {
+        float2 hv[kHeadRows];
+        float s[kHeadRows];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        const double sd = static_cast<double>(s + wb);
-        double pred, ds_dpred = 1.0, width = 1.0;
-        if (a.is_x) {
-            const double lo = a.lo[r], hi = a.hi[r];
-            const bool hl = present(lo), hu = present(hi);
-            if (hl && hu) {
-                const double sig = 1.0 / (1.0 + exp(-sd));
-                pred = lo + (hi - lo) * sig;
-                ds_dpred = (hi - lo) * sig * (1.0 - sig);
-                width = fmax(hi - lo, 1e-12);
-            } else {
-                const double lin = bs * sd;
-                pred = lin;
-                bool inside = true;
-                if (hl && lin <= lo) { pred = lo; inside = false; }
-                if (hu && lin >= hi) { pred = hi; inside = false; }
-                ds_dpred = inside ? bs : 0.0;
-                width = bs;
-            }
-        } else {
-            pred = a.ys * sd;
-            ds_dpred = a.ys;
-            width = a.ys;
+        for (int q = 0; q < kHeadRows; ++q) {
+            const long long r = r0 + q * stride;
+            hv[q] = r < a.rows ? *reinterpret_cast<const float2*>(a.h + r * a.sh + 2 * lane) : make_float2(0.f, 0.f);
         }
-        if (lane == 0) a.out[r] = pred;
-        if (a.target) {
-            const double e = (pred - a.target[r]) / width;
-            const double ds = 2.0 * e / width * inv_count * ds_dpred;
-            const float dsf = static_cast<float>(ds);
-            *reinterpret_cast<float2*>(a.dh + r * a.sdh + 2 * lane) = make_float2(dsf * w0, dsf * w1);
-            g0 += dsf * hv.x;
-            g1 += dsf * hv.y;
+#pragma unroll
+        for (int q = 0; q < kHeadRows; ++q) s[q] = hv[q].x * w0 + hv[q].y * w1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < kHeadRows; ++q) s[q] += __shfl_xor_sync(full, s[q], o);
+        float mine = s[0];
+#pragma unroll
+        for (int q = 1; q < kHeadRows; ++q) mine = lane == q ? s[q] : mine;
+        const long long r = r0 + lane * stride;
+        float dsf = 0.f, lossf = 0.f;
+        if (lane < kHeadRows && r < a.rows) {
+            const double sd = static_cast<double>(mine + wb);
+            double pred, ds_dpred = 1.0, width = 1.0;
+            if (a.is_x) {
+                const double lo = a.lo[r], hi = a.hi[r];
+                const bool hl = present(lo), hu = present(hi);
+                if (hl && hu) {
+                    const double sig = 1.0 / (1.0 + exp(-sd));
+                    pred = lo + (hi - lo) * sig;
+                    ds_dpred = (hi - lo) * sig * (1.0 - sig);
+                    width = fmax(hi - lo, 1e-12);
+                } else {
+                    const double lin = bs * sd;
+                    pred = lin;
+                    bool inside = true;
+                    if (hl && lin <= lo) { pred = lo; inside = false; }
+                    if (hu && lin >= hi) { pred = hi; inside = false; }
+                    ds_dpred = inside ? bs : 0.0;
+                    width = bs;
+                }
+            } else {
+                pred = a.ys * sd;
+                ds_dpred = a.ys;
+                width = a.ys;
+            }
+            a.out[r] = pred;
+            if (a.target) {
+                const double e = (pred - a.target[r]) / width;
+                dsf = static_cast<float>(2.0 * e / width * inv_count * ds_dpred);
+                lossf = static_cast<float>(e * e * inv_count);
+            }
+        }
+        if (!a.target) continue;
+#pragma unroll
+        for (int q = 0; q < kHeadRows; ++q) {
+            const long long rq = r0 + q * stride;
+            const float d = __shfl_sync(full, dsf, q), l = __shfl_sync(full, lossf, q);
+            if (rq >= a.rows) break;
+            float2 dh = make_float2(d * w0, d * w1);
+            if (a.relu) dh = make_float2(hv[q].x > 0.f ? dh.x : 0.f, hv[q].y > 0.f ? dh.y : 0.f);
+            *reinterpret_cast<float2*>(a.dh + rq * a.sdh + 2 * lane) = dh;
+            g0 += d * hv[q].x;
+            g1 += d * hv[q].y;
             if (lane == 0) {
-                gb += dsf;
-                gl += static_cast<float>(e * e * inv_count);
+                gb += d;
+                gl += l;
             }
         }
     }
@@ -548,7 +634,7 @@ int ensure_workspace(SankhyaB200Gnn* g, int m, int n) {
     const long long nx = al(4LL * n * kX), mx = al(4LL * m * kX);
     const long long nh = al(4LL * n * kH), mh = al(4LL * m * kH);
     const long long nf = al(4LL * n * kF), mf = al(4LL * m * kF);
-    const long long part_floats = std::max<long long>(148LL * 2 * kX * kH, static_cast<long long>(kRedBlocks) * (kH + 2));
+    const long long part_floats = std::max<long long>(148LL * 2 * tc::WgPipeShape<3>::kOut, static_cast<long long>(kInputSlices) * kInputOut);
     const long long total = 6 * nd + 5 * md + 256 + nf + mf + al(4LL * n) + al(4LL * m) + (R + 1) * (nx + mx) + nx +
                             mx + nh + mh + al(4 * part_floats) + 256 + al(sizeof(FeatureSlots));
     g->m = g->n = -1;
@@ -597,17 +683,31 @@ bool tc_fits(const void* a, int lda, const void* c, int ldc) {
            lda % 4 == 0 && ldc % 4 == 0;
 }
 
+// CTAs per SM of a kernel with this much dynamic shared memory, asked (and the kernel's
+// attribute set) once per kernel and device.
+int resident(const void* fn, int threads, int smem) {
+    struct Entry { const void* fn; int device, per_sm; };
+    static std::mutex mu;
+    static std::vector<Entry> cache;
+    int device = 0, per_sm = 1;
+    cudaGetDevice(&device);
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Entry& e : cache)
+        if (e.fn == fn && e.device == device) return e.per_sm;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
+    cache.push_back({fn, device, std::max(1, per_sm)});
+    return cache.back().per_sm;
+}
+
 // K = 64 / 128: the cp.async-pipelined kernel, one CTA per SM (its shared memory).
 template <int N, int K, int ST>
 void gemm_tc_pipe(SankhyaB200Gnn* s, cudaStream_t st, int M, const float* A, int lda, const __nv_bfloat16* B, int sbk,
                   int sbn, const float* bias, int relu, float* C, int ldc) {
     using S = tc::TcPipeShape<N, K, ST>;
     const void* fn = reinterpret_cast<const void*>(&tc::k_gemm_tc_pipe<N, K, ST>);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, S::kThreads, S::kSmem);
     const int tiles = (M + S::kM - 1) / S::kM;
-    const int grid = std::max(1, std::min(tiles, s->sms * std::max(1, per_sm)));
+    const int grid = std::max(1, std::min(tiles, s->sms * resident(fn, S::kThreads, S::kSmem)));
     tc::k_gemm_tc_pipe<N, K, ST><<<grid, S::kThreads, S::kSmem, st>>>(M, A, lda, B, sbk, sbn, bias, relu, C, ldc,
                                                                        s->tc_flag.as<unsigned int>());
 }
@@ -624,7 +724,7 @@ void gemm_tc(SankhyaB200Gnn* s, cudaStream_t st, int M, const float* A, int lda,
     }
     using S = tc::TcShape<N, K>;
     const void* fn = reinterpret_cast<const void*>(&tc::k_gemm_tc<N, K>);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
+    resident(fn, 128, S::kSmem);
     const int tiles = (M + S::kM - 1) / S::kM;
     const int grid = std::max(1, std::min(tiles, s->sms * std::min(4, 512 / S::kCols)));
     tc::k_gemm_tc<N, K><<<grid, 128, S::kSmem, st>>>(M, A, lda, B, sbk, sbn, bias, relu, C, ldc,
@@ -666,47 +766,43 @@ int check_tc(SankhyaB200Gnn* s, cudaStream_t st) {
     return fail_msg("a tensor-core GEMM's wait for its MMAs gave up");
 }
 
-// dW [K x 64] = X^T dZ over `rows` nodes (X fp32 [rows x K] with row stride ldx),
-// split over nodes into fixed slices, summed in slice order into out.
-void gemm_weight_grad(SankhyaB200Gnn* s, cudaStream_t st, int rows, const float* X, int ldx, int K, const float* dz,
-                      float* out) {
+// Gradients of a 128-wide layer over `rows` nodes, into out: dW [128 x 64] = X^T dZ and,
+// behind it, the bias gradient [64]; X fp32 [rows x 128], dz fp32 [rows x 64], both 16-byte
+// aligned. One slice (a whole number of 64-node stages) per resident CTA, summed in order.
+void layer_grads(SankhyaB200Gnn* s, cudaStream_t st, int rows, const float* X, const float* dz, float* out) {
+    using W = tc::WgPipeShape<3>;
     if (rows == 0) {
-        cudaMemsetAsync(out, 0, sizeof(float) * K * kH, st);
+        cudaMemsetAsync(out, 0, sizeof(float) * W::kOut, st);
         return;
     }
-    if (K == kX && tc_fits(X, ldx, dz, kH)) {
-        // tensor-core path: one slice (a whole number of 64-node stages) per resident CTA
-        using W = tc::WgPipeShape<3>;
-        const void* fn = reinterpret_cast<const void*>(&tc::k_wgrad_tc_pipe<kX, 3>);
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, W::kSmem);
-        int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, W::kThreads, W::kSmem);
-        const int want = std::max(1, std::min({148 * 2, s->sms * std::max(1, per_sm), (rows + W::kNodes - 1) / W::kNodes}));
-        const int chunk = ((rows + want - 1) / want + W::kNodes - 1) / W::kNodes * W::kNodes;
-        const int slices = (rows + chunk - 1) / chunk;
-        tc::k_wgrad_tc_pipe<kX, 3><<<slices, W::kThreads, W::kSmem, st>>>(rows, chunk, X, ldx, dz, s->part,
-                                                                           s->tc_flag.as<unsigned int>());
-        sum_slices(K * kH, slices, static_cast<long long>(K) * kH, s->part, out, st);
-        return;
-    }
-    const int slices = std::max(1, std::min(148 * 2, (rows + 255) / 256));
-    const int chunk = (rows + slices - 1) / slices;
-    Gemm<float> g{K, kH, rows, X, 1, ldx, dz, kH, 1, s->part, kH, 1, static_cast<long long>(K) * kH, chunk, nullptr, 0};
-    k_gemm_bf16<float><<<dim3((K + 63) / 64, 1, slices), kGemmThreads, 0, st>>>(g);
-    sum_slices(K * kH, slices, static_cast<long long>(K) * kH, s->part, out, st);
+    const void* fn = reinterpret_cast<const void*>(&tc::k_wgrad_tc_pipe<kX, 3>);
+    const int want = std::max(1, std::min({148 * 2, s->sms * resident(fn, W::kThreads, W::kSmem),
+                                           (rows + W::kNodes - 1) / W::kNodes}));
+    const int chunk = ((rows + want - 1) / want + W::kNodes - 1) / W::kNodes * W::kNodes;
+    const int slices = (rows + chunk - 1) / chunk;
+    tc::k_wgrad_tc_pipe<kX, 3><<<slices, W::kThreads, W::kSmem, st>>>(rows, chunk, X, kX, dz, s->part,
+                                                                       s->tc_flag.as<unsigned int>());
+    sum_slices(W::kOut, slices, W::kOut, s->part, out, st);
 }
 
-void bias_grad(SankhyaB200Gnn* s, cudaStream_t st, int rows, const float* dz, float* out) {
-    const int blocks = kRedBlocks;
-    k_colsum64<<<blocks, 4 * kH, 0, st>>>(rows, dz, s->part);
-    sum_slices(kH, blocks, kH, s->part, out, st);
+// Gradients of an input layer: dW [16 x 64] and the bias gradient, from dh through the
+// relu of h (null: dh is masked already).
+void input_grads(SankhyaB200Gnn* s, cudaStream_t st, int rows, const float* F, const float* dh, int sdh, const float* h,
+                 float* out) {
+    if (rows == 0) {
+        cudaMemsetAsync(out, 0, sizeof(float) * kInputOut, st);
+        return;
+    }
+    const int slices = std::max(1, std::min(kInputSlices, (rows + 16 * kWarps - 1) / (16 * kWarps)));
+    k_input_grad<<<slices, kThreads, 0, st>>>(rows, F, dh, sdh, h, s->part);
+    sum_slices(kInputOut, slices, kInputOut, s->part, out, st);
 }
 
 void spmm(cudaStream_t st, const TileCsr& M, const float* in, int sin, const float* pre, const float* post, float* out,
-          int sout, int accumulate) {
+          int sout, const float* prev, const float* h) {
     if (M.rows == 0) return;
     const int blocks = static_cast<int>(std::min<long long>((M.rows + kWarps - 1) / kWarps, 148LL * 8));
-    k_spmm64<<<blocks, kThreads, 0, st>>>(M.rows, M.ptr, M.idx, M.val, in, sin, pre, post, out, sout, accumulate);
+    k_spmm64<<<blocks, kThreads, 0, st>>>(M.rows, M.ptr, M.idx, M.val, in, sin, pre, post, out, sout, prev, h);
 }
 
 int upload_instance(SankhyaB200Gnn* g, const Plan& plan, const double* c, const double* rl, const double* ru,
@@ -738,9 +834,9 @@ void forward(SankhyaB200Gnn* g, const Plan& plan, cudaStream_t st) {
     gemm_forward(g, st, n, kF, g->fv, kF, g->params_h + o.Ev, g->params + o.bev, g->xv[0], kX);
     gemm_forward(g, st, m, kF, g->fc, kF, g->params_h + o.Ec, g->params + o.bec, g->xc[0], kX);
     for (int t = 0; t < R; ++t) {
-        spmm(st, plan.a, g->xv[t], kX, nullptr, g->inv_row, g->xc[t] + kH, kX, 0);
+        spmm(st, plan.a, g->xv[t], kX, nullptr, g->inv_row, g->xc[t] + kH, kX, nullptr, nullptr);
         gemm_forward(g, st, m, kX, g->xc[t], kX, g->params_h + o.Wc[t], g->params + o.bc[t], g->xc[t + 1], kX);
-        spmm(st, plan.at, g->xc[t + 1], kX, nullptr, g->inv_col, g->xv[t] + kH, kX, 0);
+        spmm(st, plan.at, g->xc[t + 1], kX, nullptr, g->inv_col, g->xv[t] + kH, kX, nullptr, nullptr);
         gemm_forward(g, st, n, kX, g->xv[t], kX, g->params_h + o.Wv[t], g->params + o.bv[t], g->xv[t + 1], kX);
     }
 }
@@ -751,7 +847,7 @@ void heads(SankhyaB200Gnn* g, const Plan& plan, cudaStream_t st, bool with_targe
     const Offsets& o = g->off;
     const int blocks = kRedBlocks;
     HeadArgs hx{n, g->xv[R], kX, g->params + o.wx, g->cl, g->cu, g->bs, 1.0, 1, g->x_hat,
-                with_target ? g->x_t : nullptr, g->gv, kX, g->part};
+                with_target ? g->x_t : nullptr, g->zv, kH, g->part, 1};
     k_head<<<blocks, kThreads, 0, st>>>(hx);
     if (with_target) {
         sum_slices(kH + 1, blocks, kH + 2, g->part, g->grad + o.wx, st);
@@ -759,7 +855,7 @@ void heads(SankhyaB200Gnn* g, const Plan& plan, cudaStream_t st, bool with_targe
     }
     if (m) {
         HeadArgs hy{m, g->xc[R], kX, g->params + o.wy, nullptr, nullptr, nullptr, g->settings.y_scale, 0, g->y_hat,
-                    with_target ? g->y_t : nullptr, g->gc, kX, g->part};
+                    with_target ? g->y_t : nullptr, g->gc, kX, g->part, 0};
         k_head<<<blocks, kThreads, 0, st>>>(hy);
         if (with_target) {
             sum_slices(kH + 1, blocks, kH + 2, g->part, g->grad + o.wy, st);
@@ -771,40 +867,20 @@ void heads(SankhyaB200Gnn* g, const Plan& plan, cudaStream_t st, bool with_targe
     }
 }
 
+// zv holds the column head's gradient, through its layer's relu; gc [.., :64] the row head's.
 void backward(SankhyaB200Gnn* g, const Plan& plan, cudaStream_t st) {
     const int m = plan.a.rows, n = plan.a.cols, R = g->settings.rounds;
     const Offsets& o = g->off;
     for (int t = R - 1; t >= 0; --t) {
-        k_relu_mask<<<elem_blocks(static_cast<long long>(n) * kH), kThreads, 0, st>>>(n, g->gv, kX, g->xv[t + 1], kX,
-                                                                                     g->zv);
-        gemm_weight_grad(g, st, n, g->xv[t], kX, kX, g->zv, g->grad + o.Wv[t]);
-        bias_grad(g, st, n, g->zv, g->grad + o.bv[t]);
+        layer_grads(g, st, n, g->xv[t], g->zv, g->grad + o.Wv[t]);
         gemm_input_grad(g, st, n, g->zv, g->params_h + o.Wv[t], kX, g->gv, kX);
-        spmm(st, plan.a, g->gv + kH, kX, g->inv_col, nullptr, g->gc, kX, 1);
-        if (m) {
-            k_relu_mask<<<elem_blocks(static_cast<long long>(m) * kH), kThreads, 0, st>>>(m, g->gc, kX, g->xc[t + 1],
-                                                                                         kX, g->zc);
-        }
-        gemm_weight_grad(g, st, m, g->xc[t], kX, kX, g->zc, g->grad + o.Wc[t]);
-        if (m) {
-            bias_grad(g, st, m, g->zc, g->grad + o.bc[t]);
-            gemm_input_grad(g, st, m, g->zc, g->params_h + o.Wc[t], kX, g->gc, kX);
-        } else {
-            cudaMemsetAsync(g->grad + o.bc[t], 0, sizeof(float) * kH, st);
-        }
-        spmm(st, plan.at, g->gc + kH, kX, g->inv_row, nullptr, g->gv, kX, 1);
+        spmm(st, plan.a, g->gv + kH, kX, g->inv_col, nullptr, g->zc, kH, g->gc, g->xc[t + 1]);
+        layer_grads(g, st, m, g->xc[t], g->zc, g->grad + o.Wc[t]);
+        gemm_input_grad(g, st, m, g->zc, g->params_h + o.Wc[t], kX, g->gc, kX);
+        spmm(st, plan.at, g->gc + kH, kX, g->inv_row, nullptr, g->zv, kH, g->gv, g->xv[t]);
     }
-    k_relu_mask<<<elem_blocks(static_cast<long long>(n) * kH), kThreads, 0, st>>>(n, g->gv, kX, g->xv[0], kX, g->zv);
-    gemm_weight_grad(g, st, n, g->fv, kF, kF, g->zv, g->grad + o.Ev);
-    bias_grad(g, st, n, g->zv, g->grad + o.bev);
-    if (m) {
-        k_relu_mask<<<elem_blocks(static_cast<long long>(m) * kH), kThreads, 0, st>>>(m, g->gc, kX, g->xc[0], kX,
-                                                                                     g->zc);
-        bias_grad(g, st, m, g->zc, g->grad + o.bec);
-    } else {
-        cudaMemsetAsync(g->grad + o.bec, 0, sizeof(float) * kH, st);
-    }
-    gemm_weight_grad(g, st, m, g->fc, kF, kF, g->zc, g->grad + o.Ec);
+    input_grads(g, st, n, g->fv, g->zv, kH, nullptr, g->grad + o.Ev);
+    input_grads(g, st, m, g->fc, g->gc, kX, g->xc[0], g->grad + o.Ec);
 }
 
 int check_model(SankhyaB200Gnn* g) {

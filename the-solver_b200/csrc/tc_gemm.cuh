@@ -517,9 +517,11 @@ __global__ void __launch_bounds__(256, 1) k_gemm_tc_pipe(int M, const float* __r
 //
 // part[z][f * 64 + n] = sum over the nodes k of slice z of X[k][f] dZ[k][n]: the
 // weight gradient dW = X^T dZ of a 128-wide layer input (f < 128) against the 64
-// channels of dZ, over the node slice [z chunk, min(rows, (z + 1) chunk)). The fixed
-// slices are summed afterwards in slice order, so the result does not depend on
-// timing.
+// channels of dZ, over the node slice [z chunk, min(rows, (z + 1) chunk)); behind them,
+// part[z][128 * 64 + n] = the slice's sum of dZ[k][n], the bias gradient, from the FP32
+// values as they are converted (a pass of its own over dZ took 13 us at 100,000 nodes, and
+// 5 more to sum its partials). The fixed slices are summed afterwards in slice order, so
+// the result does not depend on timing.
 //
 // The node index is the MMA's K: A = X^T (128 x nodes) and B = dZ (nodes x 64) are
 // both MN-major, so one 32-byte piece of a row of X or dZ (8 features or channels of
@@ -546,6 +548,7 @@ struct WgPipeShape {
     static constexpr int kBuf = kABytes + kBBytes;
     static constexpr int kSmem = ST * kStage + 2 * kBuf + 64 + 128;
     static constexpr int kCols = 64;
+    static constexpr int kOut = 128 * 64 + 64;            // floats of one slice
 };
 
 template <int F, int ST>
@@ -563,9 +566,9 @@ __global__ void __launch_bounds__(256) k_wgrad_tc_pipe(int rows, int chunk, cons
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int k0 = blockIdx.x * chunk, k1 = min(rows, k0 + chunk);
     const int nst = k1 > k0 ? (k1 - k0 + S::kNodes - 1) / S::kNodes : 0;
-    float* out = part + static_cast<long long>(blockIdx.x) * (128 * 64);
+    float* out = part + static_cast<long long>(blockIdx.x) * S::kOut;
     if (nst == 0) {
-        for (int e = tid; e < 128 * 64; e += S::kThreads) out[e] = 0.f;
+        for (int e = tid; e < S::kOut; e += S::kThreads) out[e] = 0.f;
         return;
     }
     auto issue = [&](int st) {
@@ -608,6 +611,7 @@ __global__ void __launch_bounds__(256) k_wgrad_tc_pipe(int rows, int chunk, cons
     const uint32_t idesc = instr_desc_bf16_mn(128, 64);
     bool failed = false;
     int issued = 0;
+    float bias[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // channels 8 ((tid / 8) mod 8) + i of this thread's nodes
     for (int st = 0; st < nst; ++st) {
         const int b = st & 1;
         issue(st + ST - 1);
@@ -636,6 +640,8 @@ __global__ void __launch_bounds__(256) k_wgrad_tc_pipe(int rows, int chunk, cons
             const float4 lo = *reinterpret_cast<const float4*>(row + ((c ^ (k & 7)) << 4));
             const float4 hi = *reinterpret_cast<const float4*>(row + (((c + 1) ^ (k & 7)) << 4));
             *reinterpret_cast<uint4*>(sB + u * 16) = pack8(lo, hi);
+            bias[0] += lo.x; bias[1] += lo.y; bias[2] += lo.z; bias[3] += lo.w;
+            bias[4] += hi.x; bias[5] += hi.y; bias[6] += hi.z; bias[7] += hi.w;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
@@ -682,6 +688,19 @@ __global__ void __launch_bounds__(256) k_wgrad_tc_pipe(int rows, int chunk, cons
                 *reinterpret_cast<float4*>(row + c0 + 4 * q) =
                     make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]),
                                 __uint_as_float(v[4 * q + 3]));
+        }
+        // the 32 threads of a channel block (node lane tid mod 8, quarter tid / 64), in order
+        float (*sums)[64] = reinterpret_cast<float (*)[64]>(stages);   // no copy is in flight: the last stages were empty
+        const int who = (tid & 7) + 8 * (tid >> 6), c = 8 * ((tid >> 3) & 7);
+        cp_async_wait<0>();
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sums[who][c + i] = bias[i];
+        __syncthreads();
+        if (tid < 64) {
+            float t = 0.f;
+            for (int w = 0; w < 32; ++w) t += sums[w][tid];
+            out[128 * 64 + tid] = t;
         }
     } else {
         if (tid == 0) atomicOr(err, 1u);
