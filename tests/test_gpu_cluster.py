@@ -1,10 +1,11 @@
-"""Iterations of a small LP on one thread-block cluster against the two fused launches per
-iteration (the path that per-kernel timing, level 2, takes). Both sum every row in the same
+"""Iterations of a small LP on one thread-block cluster, and of a mid-size one in one
+cooperative launch, against the two fused launches per iteration (the path that per-kernel
+timing, level 2, takes). Both sum every row in the same
 order and use the same elementwise arithmetic, so their iterates are equal bit for bit; where
 every row has at most 32 entries they equal the oracle's serial sums too (tests/test_gpu_parity.py
 runs config 0 there). The shapes are the edges: one entry, empty rows and columns, rows of 32 /
-33 / 256 / 257 entries (owner, warp tree, streamed), fewer chunks than CTAs, chunk counts above
-the warps of a CTA, and sizes just inside and outside the cluster's shared memory."""
+33 / 256 / 257 entries (owner, warp tree, streamed), fewer chunks than CTAs, chunk counts at and
+above the cluster's 256, more chunks than the cooperative launch has warps, and long rows there."""
 import numpy as np
 import pytest
 
@@ -40,7 +41,7 @@ def scaled_steps(engine, **kw):
 SHAPES = [
     (1, 1, [1]), (3, 2, [0, 2, 1]), (40, 31, [0, 1, 31]), (257, 300, [32, 33, 0]), (64, 700, [256, 257, 300, 5]),
     (1200, 900, [1, 40, 3]), (15, 6000, [9]), (6000, 15, [2]), (4000, 9000, [7, 3, 11]), (9000, 17500, [4]),
-    (9000, 20500, [4]),
+    (9000, 20500, [4]), (8192, 8192, [1]), (8193, 5000, [6]), (500, 7000, [300, 12, 0, 64]), (42000, 30000, [5, 17, 0, 9]),
 ]
 
 

@@ -6,6 +6,7 @@
 // :116-152 (validation order and messages, destroy-before-create, zeroed
 // handle on failure), :154-163 (destroy).
 #include "cluster.cuh"
+#include "flow.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -67,6 +68,7 @@ Share largest_share(const std::vector<int>& tiles) {
         s.rows = std::max(s.rows, tiles[2 * t1] - tiles[2 * t0]);
         s.nnz = std::max(s.nnz, tiles[2 * t1 + 1] - tiles[2 * t0 + 1]);
     }
+    for (int t = 0; t < nt; ++t) s.long_rows += tiles[2 * t + 3] - tiles[2 * t + 1] > kChunkNnz;
     return s;
 }
 
@@ -97,6 +99,26 @@ bool cluster::available(const void* kernel) {
     if (!ok) (void)cudaGetLastError();
     cache.push_back({kernel, device, ok});
     return ok;
+}
+
+int flow::resident_ctas(const void* kernel, int threads, size_t smem) {
+    struct Entry { const void* k; int device, ctas; };
+    static std::mutex mu;
+    static std::vector<Entry> cache;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Entry& e : cache)
+        if (e.k == kernel && e.device == device) return e.ctas;
+    int cooperative = 0, sms = 0, per_sm = 0;
+    const bool ok =
+        cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && cooperative &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) == cudaSuccess && per_sm > 0;
+    if (!ok) (void)cudaGetLastError();
+    cache.push_back({kernel, device, ok ? sms : 0});
+    return cache.back().ctas;
 }
 
 // ------------------------------------------------------------------ plans

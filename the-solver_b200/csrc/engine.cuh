@@ -58,6 +58,7 @@ int device_transpose(int rows, int cols, int nnz, const int* ptr, const int* idx
 // evenly and in order over the CTAs of one cluster (cluster.cuh); chunks 0: unknown.
 struct Share {
     int rows = 0, nnz = 0, chunks = 0;
+    int long_rows = 0;   // rows beyond kChunkNnz entries in the whole matrix
 };
 Share largest_share(const std::vector<int>& tiles);
 

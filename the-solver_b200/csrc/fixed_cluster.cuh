@@ -2,11 +2,12 @@
 //
 // Measured on a B200 at 1,965 MHz, us per iteration, two graph launches -> this kernel:
 // 200 x 300 (900 nonzeros) 5.5 -> 1.5; 1,000 x 2,500 (12,500) 7.0 -> 2.2; 2,000 x 5,000
-// (25,000) 7.7 -> 2.85; 4,000 x 9,000 (54,000) 7.8 -> 5.2. Of the 5,400 cycles of an
+// (25,000) 7.7 -> 2.85; 3,000 x 7,000 (42,000) 7.7 -> 3.8. Of the 5,400 cycles of an
 // iteration at 2,000 x 5,000, the two exchanges take 1,500 and 1,400 (580 each of latency,
 // the rest 12.8 bytes per cycle), the rows' sums and epilogues 1,500 and the columns' 1,000:
 // a serial chain of adds (12 cycles each), one divide (137) and shared-memory latencies, with
-// the 16 SMs' shared-memory bandwidth next. Above the size that fits, the launches win anyway.
+// the 16 SMs' shared-memory bandwidth next. With more than one chunk a warp (4,000 x 9,000,
+// 54,000) it took 5.2 where the cooperative launch of fixed_flow.cuh takes 3.9, so it ends there.
 #pragma once
 
 #include "cluster.cuh"
@@ -26,17 +27,18 @@ struct FixedClusterArgs {
     unsigned int* fail;             // set when a wait gave up
 };
 
-// Shared memory of one CTA; 0 when the problem has no rows or no columns.
+// Shared memory of one CTA; 0 when the problem has no rows or no columns, or a CTA would
+// have more chunks than warps (each stays in its warp's registers for the whole launch).
 inline size_t fixed_cluster_smem(const TileCsr& A, const TileCsr& AT) {
-    if (A.ntiles == 0 || AT.ntiles == 0) return 0;
+    if (A.ntiles == 0 || AT.ntiles == 0 ||
+        std::max(A.share.chunks, AT.share.chunks) > cluster::kClusterWarps)
+        return 0;
     return cluster::kClusterWarps * cluster::kProducts * 8ull + cluster::slice_bytes(A) + cluster::slice_bytes(AT) + cluster::packed_bytes<double>(A) +
            cluster::packed_bytes<double>(AT) + cluster::send_bytes(A.share) + cluster::send_bytes(AT.share) +
            4 * cluster::align16(8ull * A.share.rows) + 7 * cluster::align16(8ull * AT.share.rows);
 }
 
-// ONE: no CTA has more chunks of A or of A' than warps, so every chunk stays in its warp's
-// registers for the whole launch.
-template <bool SK, bool ONE>
+template <bool SK>
 __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(const __grid_constant__ FixedClusterArgs a) {
     using namespace cluster;
     extern __shared__ __align__(16) char smem[];
@@ -83,14 +85,13 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
     make_sends(R.row0, R.rows, yv, a.A.share, mem, &ys_out);
     cluster_sync();
     Chunk<double, double> rc, qc;
-    if (ONE && warp < R.chunks) rc.load(R, warp, xv.v);
-    if (ONE && warp < Q.chunks) qc.load(Q, warp, yv.v);
+    if (warp < R.chunks) rc.load(R, warp, xv.v);
+    if (warp < Q.chunks) qc.load(Q, warp, yv.v);
     double change = 0.0;
     bool ok = true;
     for (int it = 0; it < a.iterations && ok; ++it) {
         const bool last = it + 1 == a.iterations;
-        for (int j = warp; j < R.chunks; j += kClusterWarps) {
-            if (!ONE) rc.load(R, j, xv.v);
+        if (warp < R.chunks) {
             const double act = rc.sum(R, xv.v, sp);
             if (rc.owns) {
                 const int r = rc.r;
@@ -102,8 +103,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
             }
         }
         ok = exchange(ys_out, y, yv);
-        for (int j = warp; j < Q.chunks; j += kClusterWarps) {
-            if (!ONE) qc.load(Q, j, yv.v);
+        if (warp < Q.chunks) {
             const double g = qc.sum(Q, yv.v, sp);
             if (qc.owns) {
                 const int r = qc.r;
@@ -133,13 +133,6 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
             a.part[rank] = change;
         }
     }
-}
-
-using FixedClusterKernel = void (*)(FixedClusterArgs);
-inline FixedClusterKernel fixed_cluster_kernel(const TileCsr& A, const TileCsr& AT, bool sk) {
-    const bool one = A.share.chunks <= cluster::kClusterWarps && AT.share.chunks <= cluster::kClusterWarps;
-    return sk ? (one ? &k_fixed_cluster<true, true> : &k_fixed_cluster<true, false>)
-              : (one ? &k_fixed_cluster<false, true> : &k_fixed_cluster<false, false>);
 }
 
 }  // namespace b200

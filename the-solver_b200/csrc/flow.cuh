@@ -1,0 +1,206 @@
+// Mid-size LPs: many PDHG iterations in one cooperative launch, without barriers.
+//
+// Above the size that fits one cluster (cluster.cuh) and up to about a million nonzeros an
+// iteration's launches are still mostly latency: 8.8 us for two at 8,000 x 16,000 with
+// 128,000 nonzeros, where the gathers take 0.5 us each. Here every warp keeps its chunks
+// of A and A' for a window of iterations, and an iterate's element travels as one aligned
+// access (16 bytes in FP64, 8 in FP32) that holds the value and the number of its
+// iteration: whoever gathers it reads until the number is the one it needs. So a step of
+// the whole grid costs a store's way to L2 and a load's way back (2,300 cycles), where a
+// grid barrier takes 2,400 and the gathers come on top, and the matrix stays in L1, which
+// a barrier's acquire would empty. A read that comes too early makes the store's line
+// travel again, so a lane first waits for its first entry alone.
+//
+// No element is overwritten before it has been read: a row's owner stores its next y only
+// after it has gathered x from all the columns of the row, and those columns' owners have
+// stored that x after they gathered this y (A and A' have the same entries). All CTAs are
+// resident (cooperative launch), so every wait ends; each is bounded all the same.
+//
+// Row sums keep k_tiled's order, so every iterate has the same bits.
+//
+// Measured on a B200 at 1,965 MHz, us per fixed-step iteration, launches -> this: 8,000 x
+// 16,000 with 128,000 nonzeros 8.7 -> 4.3; 15,000 x 30,000 (300,000) 10.9 -> 5.6; 30,000 x
+// 60,000 (480,000) 13.1 -> 7.1; 50,000 x 100,000 (1M) 17.8 -> 13.4; 120,000 x 250,000 (2M)
+// 31.9 -> 25.2; 300,000 x 600,000 (4.8M) 67.3 -> 66.7. With columns of up to 1,000 entries:
+// 128,000 9.6 -> 5.1; 480,000 13.3 -> 12.9; 1.2M 22.8 -> 25.2. Below some 45,000 nonzeros the
+// cluster is ahead (25,000: 2.8 against 3.8; 42,000: 3.8 against 3.9).
+#pragma once
+
+#include "engine.cuh"
+
+namespace b200 {
+namespace flow {
+
+constexpr int kMaxPolls = 1 << 22;    // loads of one wait, some seconds
+
+// An element and the iteration it belongs to, read and written as one access.
+template <class T>
+struct Tagged;
+template <>
+struct alignas(16) Tagged<double> {
+    double value;
+    unsigned long long tag;
+};
+template <>
+struct alignas(8) Tagged<float> {
+    float value;
+    unsigned tag;
+};
+
+__device__ __forceinline__ Tagged<double> load_tagged(const Tagged<double>* p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    return Tagged<double>{__longlong_as_double(static_cast<long long>(lo)), hi};
+}
+__device__ __forceinline__ Tagged<float> load_tagged(const Tagged<float>* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return Tagged<float>{__uint_as_float(static_cast<unsigned>(v)), static_cast<unsigned>(v >> 32)};
+}
+__device__ __forceinline__ void store_tagged(Tagged<double>* p, double v, unsigned long long tag) {
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"(tag) : "memory");
+}
+__device__ __forceinline__ void store_tagged(Tagged<float>* p, float v, unsigned tag) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p),
+                 "l"(static_cast<unsigned long long>(__float_as_uint(v)) | static_cast<unsigned long long>(tag) << 32)
+                 : "memory");
+}
+
+template <class T>
+struct TagOf { using type = unsigned long long; };
+template <>
+struct TagOf<float> { using type = unsigned; };
+
+// Waits for the element of iteration `want`. `left` counts down over all of a thread's
+// waits of an iteration; at 0 nothing is waited for any more.
+template <class T>
+__device__ __forceinline__ T wait_element(const Tagged<T>* p, typename TagOf<T>::type want, int* left) {
+    Tagged<T> e = load_tagged(p);
+    while (e.tag != want && --*left > 0) e = load_tagged(p);
+    return e.value;
+}
+
+template <class T, class V>
+__device__ __forceinline__ T value_at(const V* p) { return static_cast<T>(__ldg(p)); }
+template <>
+__device__ __forceinline__ float value_at<float, __nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(__ldg(p)); }
+
+// A chunk as one warp sees it: its bounds and the row of each lane.
+struct ChunkRows {
+    int p0, p1;        // entries
+    int row, q0, len;  // this lane's row and its entries within the chunk; len 0 without one
+    bool owns;
+};
+template <class V>
+__device__ __forceinline__ ChunkRows chunk_rows(const TileCsrT<V>& A, int t) {
+    const int2 b0 = __ldg(A.tile + t), b1 = __ldg(A.tile + t + 1);
+    ChunkRows c;
+    c.p0 = b0.y;
+    c.p1 = b1.y;
+    c.row = b0.x + static_cast<int>(threadIdx.x & 31);
+    c.owns = c.row < b1.x;
+    c.q0 = c.owns ? __ldg(A.ptr + c.row) - b0.y : 0;
+    c.len = c.owns ? __ldg(A.ptr + c.row + 1) - b0.y - c.q0 : 0;
+    return c;
+}
+
+// The sum of this lane's row (whole warps), in k_tiled's order, of the elements of
+// iteration `want` of v. `sp`: the warp's kChunkNnz products. (The row beyond a chunk waits
+// entry by entry on purpose: requesting eight at a time there costs the common path its
+// registers, 5 to 40 % of an iteration.)
+template <class T, class V>
+__device__ __forceinline__ T chunk_sum(const TileCsrT<V>& A, const ChunkRows& c, const Tagged<T>* v,
+                                       typename TagOf<T>::type want, T* sp, int* left) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (c.p1 - c.p0 > kChunkNnz) {   // one row longer than a chunk
+        auto get = [&](int j) { return wait_element(v + j, want, left); };
+        T s0 = T(0), s1 = T(0);
+        int p = c.p0 + lane;
+        for (; p + 32 < c.p1; p += 64) {
+            s0 = fma(value_at<T>(A.val + p), get(__ldg(A.idx + p)), s0);
+            s1 = fma(value_at<T>(A.val + p + 32), get(__ldg(A.idx + p + 32)), s1);
+        }
+        if (p < c.p1) s0 = fma(value_at<T>(A.val + p), get(__ldg(A.idx + p)), s0);
+        return warp_sum(s0 + s1);
+    }
+    int col[kPerLane];
+    T a[kPerLane], g[kPerLane];
+#pragma unroll
+    for (int k = 0; k < kPerLane; ++k) {
+        const int p = c.p0 + 32 * k + lane;
+        col[k] = -1;
+        a[k] = g[k] = T(0);
+        if (p < c.p1) {
+            col[k] = __ldg(A.idx + p);
+            a[k] = value_at<T>(A.val + p);
+        }
+    }
+    if (col[0] >= 0) g[0] = wait_element(v + col[0], want, left);
+    __syncwarp();
+    unsigned missing = 0;
+#pragma unroll
+    for (int k = 1; k < kPerLane; ++k)
+        if (col[k] >= 0) missing |= 1u << k;
+    while (missing && --*left > 0) {
+        Tagged<T> e[kPerLane];
+#pragma unroll
+        for (int k = 1; k < kPerLane; ++k)
+            if (missing >> k & 1u) e[k] = load_tagged(v + col[k]);
+#pragma unroll
+        for (int k = 1; k < kPerLane; ++k)
+            if ((missing >> k & 1u) && e[k].tag == want) {
+                g[k] = e[k].value;
+                missing &= ~(1u << k);
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < kPerLane; ++k)
+        if (col[k] >= 0) sp[32 * k + lane] = dmul(a[k], g[k]);
+    __syncwarp();
+    T s = T(0);
+    if (c.len <= kShortRow) {
+        int q = c.q0;
+        const int q1 = c.q0 + c.len;
+        for (; q + 4 <= q1; q += 4) {
+            const T e0 = sp[q], e1 = sp[q + 1], e2 = sp[q + 2], e3 = sp[q + 3];
+            s = dadd(dadd(dadd(dadd(s, e0), e1), e2), e3);
+        }
+        for (; q < q1; ++q) s = dadd(s, sp[q]);
+    }
+    unsigned long_rows = __ballot_sync(full, c.len > kShortRow);
+    while (long_rows) {
+        const int l = __ffs(long_rows) - 1;
+        long_rows &= long_rows - 1;
+        const int a0 = __shfl_sync(full, c.q0, l), al = __shfl_sync(full, c.len, l);
+        T t = T(0);
+        for (int q = lane; q < al; q += 32) t = dadd(t, sp[a0 + q]);
+        t = warp_sum(t);
+        if (lane == l) s = t;
+    }
+    __syncwarp();
+    return s;
+}
+
+// Where this beats the launches (figures above): up to 3M nonzeros, or 400,000 where a row
+// or column is longer than a chunk (its warp waits for 64 entries at a time).
+template <class V>
+inline bool flow_pays(const TileCsrT<V>& A, const TileCsrT<V>& AT) {
+    const bool has_long = A.share.long_rows + AT.share.long_rows > 0;
+    return A.ntiles > 0 && AT.ntiles > 0 && A.nnz <= (has_long ? 400000 : 3000000);
+}
+
+// CTAs of `threads` threads the current device holds at a time with one per SM, 0 where
+// the kernel cannot be launched cooperatively (asked once per kernel and device).
+int resident_ctas(const void* kernel, int threads, size_t smem);
+
+template <class Args>
+inline cudaError_t launch(void (*kernel)(Args), const Args& args, int ctas, int threads, size_t smem, cudaStream_t stream) {
+    void* p[] = {const_cast<Args*>(&args)};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(ctas), dim3(threads), p, smem, stream);
+}
+
+}  // namespace flow
+}  // namespace b200

@@ -18,6 +18,7 @@
 #include "engine.cuh"
 #include "fixed_cluster.cuh"
 #include "fixed_epi.cuh"
+#include "fixed_flow.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -195,6 +196,8 @@ struct Workspace {
     double *qdiag = nullptr, *tauv = nullptr, *sigv = nullptr;
     double *x[2] = {nullptr, nullptr}, *y[2] = {nullptr, nullptr};
     double *x_bar = nullptr, *qx = nullptr, *x_prev = nullptr, *act = nullptr;
+    flow::Tagged<double>*xt = nullptr, *yt = nullptr;  // x_bar and y by iteration (fixed_flow.cuh)
+    unsigned long long epoch = 0;                       // iterations numbered so far; 0: not cleared yet
     double *part_a = nullptr, *part_b = nullptr, *part_c = nullptr, *out = nullptr;
     unsigned int* flags = nullptr;  // right behind `out`: [0] input checks, [1] a cluster wait gave up
     int n = 0, m = 0;
@@ -206,15 +209,17 @@ struct Workspace {
         const size_t nb = (static_cast<size_t>(n) * 8 + 255) / 256 * 256;
         const size_t mb = (static_cast<size_t>(m) * 8 + 255) / 256 * 256;
         const size_t pb = (static_cast<size_t>(max_grid) * 8 * 8 + 255) / 256 * 256;
-        const size_t total = 11 * nb + 6 * mb + 3 * pb + 512;
+        const size_t total = 10 * nb + 6 * mb + 2 * nb + 2 * mb + 3 * pb + 512;
         const char* what = "cudaMalloc PDHG workspace";
         if (on ? blob.alloc_on(*on, total, what) : blob.alloc(total, what)) return -1;
         char* p = blob.as<char>();
         auto take = [&](size_t b) { double* r = reinterpret_cast<double*>(p); p += b; return r; };
         c = take(nb); cl = take(nb); cu = take(nb); qdiag = take(nb); tauv = take(nb);
         x[0] = take(nb); x[1] = take(nb); x_bar = take(nb); qx = take(nb); x_prev = take(nb);
-        take(nb);
         rl = take(mb); ru = take(mb); sigv = take(mb); y[0] = take(mb); y[1] = take(mb); act = take(mb);
+        xt = reinterpret_cast<flow::Tagged<double>*>(take(2 * nb));
+        yt = reinterpret_cast<flow::Tagged<double>*>(take(2 * mb));
+        epoch = 0;
         part_a = take(pb); part_b = take(pb); part_c = take(pb); out = take(256);
         flags = reinterpret_cast<unsigned int*>(take(256));
         return 0;
@@ -268,18 +273,24 @@ struct Solver {
     int launches = 0;
     GraphMap local_graphs;
     GraphMap* graphs = &local_graphs;
-    FixedClusterKernel cluster_kernel = nullptr;
+    void (*flow_kernel)(FixedFlowArgs) = nullptr;
+    void (*cluster_kernel)(FixedClusterArgs) = nullptr;
     size_t cluster_smem = 0;  // > 0: the iterations run on one cluster
+    int flow_ctas = 0;        // > 0: the iterations run as one cooperative launch
     int dual_blocks = 0;      // partials the last dual step left in part_c
 
     void setup_grids() {
-        // Rule: the LP (no explicit Hessian) fits the shared memory of one cluster, which it
-        // does up to about 100,000 nonzeros. Below that line the cluster is the faster one
-        // throughout (fixed_cluster.cuh has the figures).
+        // Rule: an LP (no explicit Hessian) whose chunks fit the registers and shared memory of
+        // one cluster (256 chunks each way, some 45,000 nonzeros), else one that flow_pays.
         const size_t need = Q ? 0 : fixed_cluster_smem(*A, *AT);
-        cluster_kernel = fixed_cluster_kernel(*A, *AT, sem == Sem::Sk);
+        cluster_kernel = sem == Sem::Cuda ? &k_fixed_cluster<false> : &k_fixed_cluster<true>;
         cluster_smem = need > 0 && need <= cluster::kMaxSmem &&
                                cluster::available(reinterpret_cast<const void*>(cluster_kernel)) ? need : 0;
+        flow_ctas = 0;
+        if (!cluster_smem && !Q && flow::flow_pays(*A, *AT)) {
+            flow_kernel = sem == Sem::Cuda ? &k_fixed_flow<false> : &k_fixed_flow<true>;
+            flow_ctas = flow::resident_ctas(reinterpret_cast<const void*>(flow_kernel), kFlowThreads, 0);
+        }
         if (sem == Sem::Cuda) {
             grid_dual = tiled_grid<DualCudaEpi>(*A);
             grid_primal = tiled_grid<PrimalCudaEpi>(*AT);
@@ -289,6 +300,29 @@ struct Solver {
         }
         if (Q) grid_q = tiled_grid<StoreEpi>(*Q);
         dual_blocks = A->ntiles ? grid_dual : 0;
+    }
+
+    // k iterations as cooperative launches of up to cluster::kMaxSteps.
+    int run_flow(int k) {
+        if (w->epoch == 0) {
+            B200_TRY(cudaMemsetAsync(w->xt, 0, 16 * static_cast<size_t>(w->n), stream), "clear");
+            B200_TRY(cudaMemsetAsync(w->yt, 0, 16 * static_cast<size_t>(w->m), stream), "clear");
+            w->epoch = 2;
+        }
+        while (k > 0) {
+            const int steps = std::min(k, cluster::kMaxSteps), nx = cur ^ 1;
+            const FixedFlowArgs a{*A, *AT, w->c, w->cl, w->cu, has_steps ? w->tauv : nullptr,
+                                  has_qdiag ? w->qdiag : nullptr, w->rl, w->ru, has_steps ? w->sigv : nullptr, tau, sigma,
+                                  theta, w->x[cur], w->y[cur], w->x[nx], w->y[nx], w->x_bar, w->part_c, w->xt, w->yt,
+                                  w->epoch, steps, w->flags + 1};
+            B200_TRY(flow::launch(flow_kernel, a, flow_ctas, kFlowThreads, 0, stream), "cooperative launch");
+            ++launches;
+            w->epoch += steps + 1;
+            cur = nx;
+            k -= steps;
+        }
+        dual_blocks = flow_ctas;
+        return 0;
     }
 
     // k iterations as cluster launches of up to cluster::kMaxSteps.
@@ -363,6 +397,7 @@ struct Solver {
             return 0;
         }
         if (cluster_smem) return run_cluster(k);
+        if (flow_ctas) return run_flow(k);
         while (k > 0) {
             const int chunk = k > 64 ? 64 : k;
             const GraphKey key{stream, Q, has_qdiag ? 1 : 0, has_steps ? 1 : 0, chunk, cur, static_cast<int>(sem),

@@ -481,6 +481,7 @@ __global__ void k_halpern_restart(int n, int m, const T* __restrict__ x_t, const
 }  // namespace b200
 
 #include "pdlp_cluster.cuh"
+#include "pdlp_flow.cuh"
 
 namespace b200 {
 namespace {
@@ -1248,6 +1249,13 @@ struct Core {
     size_t adaptive_smem = 0, halpern_smem = 0;
     void (*adaptive_kernel)(AdaptiveClusterArgs<T, V>) = nullptr;
     void (*halpern_kernel)(HalpernClusterArgs<T, V>) = nullptr;
+    // Mid-size LPs: as one cooperative launch of so many CTAs (pdlp_flow.cuh); 0: not.
+    int adaptive_ctas = 0, halpern_ctas = 0;
+    DevBuf flow_blob;
+    flow::Tagged<T>*xt = nullptr, *yt = nullptr;
+    flow::Tagged<double>* sums = nullptr;
+    unsigned* count = nullptr;
+    unsigned epoch = 1, arrived = 0;   // iterations numbered, and arrivals counted, so far
     // Quadratic objective (the QP entry point): qmode kQDiag with the diagonal qd,
     // or kQGeneral with the Hessian Q and its diagonal majorant qd, whose products
     // Q x (committed point), Q x_cand and Q x_avg ride along like the A-side ones;
@@ -1298,7 +1306,7 @@ struct Core {
         return 0;
     }
 
-    void set_problem(const TileCsrT<V>& a, const TileCsrT<V>& at, const T* c_, const T* cl_, const T* cu_,
+    int set_problem(const TileCsrT<V>& a, const TileCsrT<V>& at, const T* c_, const T* cl_, const T* cu_,
                      const T* rl_, const T* ru_) {
         A = a;
         AT = at;
@@ -1321,26 +1329,50 @@ struct Core {
         grid_rcc = qmode == kQDiag ? tiled_grid<ResColsCenteredEpi<T, kQDiag>, T>(AT)
                    : qmode == kQGeneral ? tiled_grid<ResColsCenteredEpi<T, kQGeneral>, T>(AT)
                                         : tiled_grid<ResColsCenteredEpi<T>, T>(AT);
-        choose_cluster();
         for (auto g : graphs)
             if (g) cudaGraphExecDestroy(g);
         graphs.clear();
+        return choose_path();
     }
 
-    // Rule: an LP that fits one cluster's shared memory. The adaptive loop also needs one
-    // chunk per warp in the launches it stands for, so that the decision's sums keep their shape.
-    void choose_cluster() {
+    static constexpr size_t kFlowSmem = kFlowWarps * kChunkNnz * sizeof(T), kSumsSmem = 3 * kFlowBlocks * 8;
+
+    // Rule: an LP whose chunks fit the registers and shared memory of one cluster, else one
+    // that flow_pays. The adaptive loop also needs one chunk per warp in the launches it
+    // stands for, so that the decision's sums keep their shape.
+    int choose_path() {
         adaptive_smem = halpern_smem = 0;
-        if (qmode != kLp) return;
-        const bool one = A.share.chunks <= cluster::kClusterWarps && AT.share.chunks <= cluster::kClusterWarps;
-        adaptive_kernel = one ? &k_adaptive_cluster<T, V, true> : &k_adaptive_cluster<T, V, false>;
-        halpern_kernel = one ? &k_halpern_cluster<T, V, true> : &k_halpern_cluster<T, V, false>;
-        const size_t ad = adaptive_cluster_smem<T, V>(A, AT), ha = halpern_cluster_smem<T, V>(A, AT);
-        if (ad && ad <= cluster::kMaxSmem && A.ntiles <= grid_k3 * kWarps && AT.ntiles <= grid_k2 * kWarps &&
-            cluster::available(reinterpret_cast<const void*>(adaptive_kernel)))
-            adaptive_smem = ad;
-        if (ha && ha <= cluster::kMaxSmem && cluster::available(reinterpret_cast<const void*>(halpern_kernel)))
-            halpern_smem = ha;
+        adaptive_ctas = halpern_ctas = 0;
+        if (qmode != kLp) return 0;
+        const bool one_each = A.ntiles <= grid_k3 * kWarps && AT.ntiles <= grid_k2 * kWarps;
+        if (A.share.chunks <= cluster::kClusterWarps && AT.share.chunks <= cluster::kClusterWarps) {
+            adaptive_kernel = &k_adaptive_cluster<T, V>;
+            halpern_kernel = &k_halpern_cluster<T, V>;
+            const size_t ad = adaptive_cluster_smem<T, V>(A, AT), ha = halpern_cluster_smem<T, V>(A, AT);
+            if (ad && ad <= cluster::kMaxSmem && one_each && cluster::available(reinterpret_cast<const void*>(adaptive_kernel)))
+                adaptive_smem = ad;
+            if (ha && ha <= cluster::kMaxSmem && cluster::available(reinterpret_cast<const void*>(halpern_kernel)))
+                halpern_smem = ha;
+        }
+        if (!flow::flow_pays(A, AT)) return 0;
+        if (!adaptive_smem && one_each)
+            adaptive_ctas = flow::resident_ctas(reinterpret_cast<const void*>(&k_adaptive_flow<T, V>), kFlowThreads,
+                                                kFlowSmem + kSumsSmem);
+        if (!halpern_smem)
+            halpern_ctas = flow::resident_ctas(reinterpret_cast<const void*>(&k_halpern_flow<T, V>), kFlowThreads, kFlowSmem);
+        // a step's chunks in at most kFlowRounds rounds, its blocks in kFlowBlocks slots
+        const int blocks = (std::max(A.ntiles, AT.ntiles) + 7) / 8;
+        if (blocks > std::min(kFlowBlocks, adaptive_ctas * kFlowGroups * kFlowRounds)) adaptive_ctas = 0;
+        if (!(adaptive_ctas || halpern_ctas) || flow_blob.p) return 0;
+        const size_t xb = cluster::align16(sizeof(flow::Tagged<T>) * n), yb = cluster::align16(sizeof(flow::Tagged<T>) * m);
+        const size_t total = xb + yb + 2 * kSumsSmem * 2 + 256;
+        if (flow_blob.alloc_on(stream, total, "cudaMalloc numbered iterates")) return -1;
+        B200_TRY(cudaMemsetAsync(flow_blob.p, 0, total, stream), "clear");
+        xt = flow_blob.as<flow::Tagged<T>>();
+        yt = reinterpret_cast<flow::Tagged<T>*>(flow_blob.as<char>() + xb);
+        sums = reinterpret_cast<flow::Tagged<double>*>(flow_blob.as<char>() + xb + yb);
+        count = reinterpret_cast<unsigned*>(flow_blob.as<char>() + total - 256);
+        return 0;
     }
 
     // The QP's Hessian: a diagonal (diag, q null) or a general matrix (q, n x n, with
@@ -1462,6 +1494,22 @@ struct Core {
             B200_TRY(cudaGetLastError(), "window launch");
             return 0;
         }
+        if (adaptive && adaptive_ctas) {
+            for (int done = 0; done < period; done += cluster::kMaxSteps) {
+                const int steps = std::min(period - done, cluster::kMaxSteps);
+                const AdaptiveFlowArgs<T, V> a{A, AT, x, x_cand, x_sum, y, y_cand, y_sum, ax, ax_prev, ax_cand, c, cl, cu,
+                                               rl, ru, ctr ? ctr->yc : nullptr, st, res + kFail, xt, yt, sums, count, arrived, epoch,
+                                               steps};
+                B200_TRY(flow::launch(&k_adaptive_flow<T, V>, a, adaptive_ctas, kFlowThreads, kFlowSmem + kSumsSmem, stream),
+                         "cooperative launch");
+                epoch += steps;
+                arrived += static_cast<unsigned>(adaptive_ctas) * static_cast<unsigned>(steps);
+                ++launches;
+            }
+            window_end(true);
+            B200_TRY(cudaGetLastError(), "window launch");
+            return 0;
+        }
         cudaGraphExec_t exec = nullptr;
         if (*graph_slot >= 0) exec = graphs[static_cast<size_t>(*graph_slot)];
         if (!exec) {
@@ -1543,6 +1591,20 @@ struct Core {
                 const HalpernClusterArgs<T, V> a{A, AT, x, y, x_restart, y_restart, c, cl, cu, rl, ru, st, res + kFail,
                                                  done, std::min(period - done, cluster::kMaxSteps)};
                 B200_TRY(cluster::launch(halpern_kernel, a, halpern_smem, stream), "cluster launch");
+                ++launches;
+            }
+            halpern_window_end();
+            B200_TRY(cudaGetLastError(), "window launch");
+            return 0;
+        }
+        if (halpern_ctas) {
+            for (int done = 0; done < period; done += cluster::kMaxSteps) {
+                const int steps = std::min(period - done, cluster::kMaxSteps);
+                const HalpernFlowArgs<T, V> a{A, AT, x, y, x_restart, y_restart, c, cl, cu, rl, ru, st, res + kFail, xt, yt,
+                                              epoch + 1, done, steps};
+                B200_TRY(flow::launch(&k_halpern_flow<T, V>, a, halpern_ctas, kFlowThreads, kFlowSmem, stream),
+                         "cooperative launch");
+                epoch += steps + 1;
                 ++launches;
             }
             halpern_window_end();
@@ -1918,7 +1980,7 @@ int run_polished(const Scaled& sc, Core<double>& hi, const LoopParams& lp, const
         // primal feasibility problem (zero cost) from the main loop's x, dual at zero
         B200_TRY(cudaMemcpyAsync(xp, hi.x, nb, d2d, stream), "copy");
         if (!(ms.best.primal <= ps.polish_tolerance)) {
-            pol.set_problem(sc.A, sc.AT, zero_c, sc.cl, sc.cu, sc.rl, sc.ru);
+            if (pol.set_problem(sc.A, sc.AT, zero_c, sc.cl, sc.cu, sc.rl, sc.ru)) return -1;
             B200_TRY(cudaMemcpyAsync(pol.x, hi.x, nb, d2d, stream), "copy");
             B200_TRY(cudaMemsetAsync(pol.y, 0, mb, stream), "zero");
             pl.cost_norm = 0.0;
@@ -1940,7 +2002,7 @@ int run_polished(const Scaled& sc, Core<double>& hi, const LoopParams& lp, const
         // dual feasibility problem (finite bounds at zero) from the main loop's y, primal at zero
         B200_TRY(cudaMemcpyAsync(yd, hi.y, mb, d2d, stream), "copy");
         if (!(ms.best.dual <= ps.polish_tolerance) && !acc.timed_out && !acc.cancelled) {
-            pol.set_problem(sc.A, sc.AT, sc.c, cl0, cu0, rl0, ru0);
+            if (pol.set_problem(sc.A, sc.AT, sc.c, cl0, cu0, rl0, ru0)) return -1;
             B200_TRY(cudaMemsetAsync(pol.x, 0, nb, stream), "zero");
             B200_TRY(cudaMemcpyAsync(pol.y, hi.y, mb, d2d, stream), "copy");
             pl.cost_norm = lp.cost_norm;
@@ -1961,7 +2023,7 @@ int run_polished(const Scaled& sc, Core<double>& hi, const LoopParams& lp, const
         }
         pr->polish_seconds += now_s() - t_pol;
         // the pair, scored on the original problem
-        pol.set_problem(sc.A, sc.AT, sc.c, sc.cl, sc.cu, sc.rl, sc.ru);
+        if (pol.set_problem(sc.A, sc.AT, sc.c, sc.cl, sc.cu, sc.rl, sc.ru)) return -1;
         B200_TRY(cudaMemcpyAsync(pol.x, xp, nb, d2d, stream), "copy");
         B200_TRY(cudaMemcpyAsync(pol.x_restart, xp, nb, d2d, stream), "copy");
         B200_TRY(cudaMemcpyAsync(pol.y, yd, mb, d2d, stream), "copy");
@@ -2157,7 +2219,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
     hi.host = slot;
     if (hi.allocate(n, m, sc.sms)) return -1;
     if (hi.set_hessian(qd_s, hessian ? &Qs : nullptr)) return -1;
-    hi.set_problem(sc.A, sc.AT, sc.c, sc.cl, sc.cu, sc.rl, sc.ru);
+    if (hi.set_problem(sc.A, sc.AT, sc.c, sc.cl, sc.cu, sc.rl, sc.ru)) return -1;
     B200_TRY(cudaMemsetAsync(hi.x, 0, std::max<size_t>(nb, 1), stream), "zero");
     B200_TRY(cudaMemsetAsync(hi.y, 0, std::max<size_t>(mb, 1), stream), "zero");
     if (x0 && n) B200_TRY(cudaMemcpyAsync(hi.x, x0, nb, cudaMemcpyHostToDevice, stream), "upload x0");
@@ -2254,7 +2316,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
             lo.host = slot;
             if (lo.allocate(n, m, sc.sms)) return -1;
             if (lo.set_hessian(qd32, hessian ? &Q32 : nullptr)) return -1;
-            lo.set_problem(av, atv, ctr.c32, ctr.cl32, ctr.cu32, ctr.rl32, ctr.ru32);
+            if (lo.set_problem(av, atv, ctr.c32, ctr.cl32, ctr.cu32, ctr.rl32, ctr.ru32)) return -1;
             lo.ctr = &ctr;
             if (lo.run(lp, &stats)) return -1;
             refinements = lo.recenters;
@@ -2296,7 +2358,7 @@ int pdlp_solve(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessian, cons
         lo.stream = stream;
         lo.host = slot;
         if (lo.allocate(n, m, sc.sms)) return -1;
-        lo.set_problem(sc.A.with_values<float>(a32), sc.AT.with_values<float>(at32), c32, cl32, cu32, rl32, ru32);
+        if (lo.set_problem(sc.A.with_values<float>(a32), sc.AT.with_values<float>(at32), c32, cl32, cu32, rl32, ru32)) return -1;
         k_narrow<<<gv, kThreads, 0, stream>>>(n, hi.x, lo.x);
         k_narrow<<<gv, kThreads, 0, stream>>>(m, hi.y, lo.y);
         LoopParams flp = lp;

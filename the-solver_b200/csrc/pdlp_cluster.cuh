@@ -13,8 +13,7 @@
 // Measured on a B200 at 1,965 MHz, us per iteration with the window-end evaluations, three
 // (Halpern: two) graph launches -> one cluster launch per window of 64: 300 x 700 adaptive
 // 11.9 -> 4.3, Halpern 7.4 -> 2.8; 2,000 x 5,000 (25,000 nonzeros) adaptive FP64 13.4 -> 5.9,
-// FP32 13.6 -> 5.3, Halpern 8.2 -> 4.2; 4,000 x 9,000 (54,000) FP32 14.6 -> 7.2, Halpern
-// 8.6 -> 6.9. An adaptive iteration at 2,000 x 5,000 takes 8,000 cycles: the two vector
+// FP32 13.6 -> 5.3, Halpern 8.2 -> 4.2. An adaptive iteration at 2,000 x 5,000 takes 8,000 cycles: the two vector
 // exchanges 1,500 each, the columns' and rows' sums 1,600 and 2,000 (a serial chain of adds
 // and the chunk trees), the candidate 650, the sums' exchange 600, the decision 1,000.
 #pragma once
@@ -23,8 +22,6 @@
 
 namespace b200 {
 namespace {
-
-constexpr int kTreeBlocks = 256;   // leaves of the decision's tree; eight chunks each
 
 // All CTAs' chunk sums: two buffers taken in turn, since a CTA that has read the sums of an
 // iteration says so only by its sums of the next one.
@@ -36,7 +33,8 @@ struct ChunkSums {
     unsigned bytes;                // of one exchange
 };
 
-// Leaves of 8 chunks from v, summed by the tree over kTreeBlocks leaves (one warp).
+// Sums of 8 chunks from v, at most 32 of them, by the tree over 256 blocks (one warp): its
+// levels 128, 64 and 32 add zeros.
 __device__ __forceinline__ double tree_of_blocks(const double* v, int padded) {
     const int lane = threadIdx.x & 31;
     auto leaf = [&](int g) {
@@ -49,13 +47,7 @@ __device__ __forceinline__ double tree_of_blocks(const double* v, int padded) {
         for (int w = 1; w < 8; ++w) r = r + e[w];
         return r;
     };
-    double t = leaf(lane);
-    if (padded > 8 * 32) {   // levels 128, 64 and 32 of the tree; below, they add zeros
-        const double b4 = leaf(lane + 128), b2 = leaf(lane + 64), b6 = leaf(lane + 192), b1 = leaf(lane + 32),
-                     b5 = leaf(lane + 160), b3 = leaf(lane + 96), b7 = leaf(lane + 224);
-        t = ((t + b4) + (b2 + b6)) + ((b1 + b5) + (b3 + b7));
-    }
-    return warp_sum(t);
+    return warp_sum(leaf(lane));
 }
 
 template <class T, class V>
@@ -71,12 +63,12 @@ struct AdaptiveClusterArgs {
 
 inline int padded_chunks(int ntiles) { return (ntiles + 7) / 8 * 8; }
 
-// Shared memory of one CTA; 0 when there are no rows or columns, or more chunks than the
-// decision's tree has places for.
+// Shared memory of one CTA; 0 when there are no rows or columns. (A CTA has at most a chunk
+// per warp, so there are at most 32 blocks of eight.)
 template <class T, class V>
 inline size_t adaptive_cluster_smem(const TileCsrT<V>& A, const TileCsrT<V>& AT) {
     using namespace cluster;
-    if (A.ntiles == 0 || AT.ntiles == 0 || std::max(A.ntiles, AT.ntiles) > 8 * kTreeBlocks) return 0;
+    if (A.ntiles == 0 || AT.ntiles == 0) return 0;
     const size_t sums = 8ull * (padded_chunks(AT.ntiles) + 2 * padded_chunks(A.ntiles));
     return align16(kClusterWarps * kProducts * sizeof(T)) + slice_bytes(A) + slice_bytes(AT) + packed_bytes<T>(A) +
            packed_bytes<T>(AT) + send_bytes(A.share) + send_bytes(AT.share) + 2 * align16(sums) +
@@ -84,7 +76,7 @@ inline size_t adaptive_cluster_smem(const TileCsrT<V>& A, const TileCsrT<V>& AT)
            align16(8ull * A.share.rows) + 6 * align16(sizeof(T) * AT.share.rows);
 }
 
-template <class T, class V, bool ONE>
+template <class T, class V>
 __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
     k_adaptive_cluster(const __grid_constant__ AdaptiveClusterArgs<T, V> a) {
     using namespace cluster;
@@ -143,8 +135,8 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
     make_sends(R.row0, R.rows, yv, a.A.share, mem, &ys_out);
     cluster_sync();
     Chunk<T, V> rc, qc;
-    if (ONE && warp < R.chunks) rc.load(R, warp, xv.v);
-    if (ONE && warp < Q.chunks) qc.load(Q, warp, yv.v);
+    if (warp < R.chunks) rc.load(R, warp, xv.v);
+    if (warp < Q.chunks) qc.load(Q, warp, yv.v);
     const double omega = a.st->omega, eta_lo = a.st->eta_min, eta_hi = a.st->eta_max;
     double eta = a.st->eta, updates = a.st->updates, accepts = a.st->accept_count;
     double dx2 = 0.0, dy2 = 0.0, cross = 0.0, limit = a.st->eta_bar;
@@ -171,8 +163,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
         }
         if (keep) commit_columns();
         ok = exchange(ys_out, yc, yv);
-        for (int j = warp; j < Q.chunks; j += kClusterWarps) {
-            if (!ONE) qc.load(Q, j, yv.v);
+        if (warp < Q.chunks) {
             const T aty = qc.sum(Q, yv.v, sp);
             double d = 0.0;
             if (qc.owns) {
@@ -183,14 +174,13 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
                 d = dx * dx;
             }
             d = warp_sum(d);
-            if (lane == 0) sums.own[j] = d;
+            if (lane == 0) sums.own[warp] = d;
         }
         ok = exchange(xs_out, xc, xv, [&] {
             if (warp != kClusterWarps - 1 || lane >= 2) return;   // the warp with the fewest chunks
             growth[lane] = step_growth(updates + 1.0, lane == 0);
         }) && ok;
-        for (int j = warp; j < R.chunks; j += kClusterWarps) {
-            if (!ONE) rc.load(R, j, xv.v);
+        if (warp < R.chunks) {
             const T axn = rc.sum(R, xv.v, sp);
             double d = 0.0, e = 0.0;
             if (rc.owns) {
@@ -203,8 +193,8 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
             d = warp_sum(d);
             e = warp_sum(e);
             if (lane == 0) {
-                sums.own[Q.chunks + j] = d;
-                sums.own[Q.chunks + R.chunks + j] = e;
+                sums.own[Q.chunks + warp] = d;
+                sums.own[Q.chunks + R.chunks + warp] = e;
             }
         }
         __syncthreads();
@@ -287,7 +277,7 @@ inline size_t halpern_cluster_smem(const TileCsrT<V>& A, const TileCsrT<V>& AT) 
            6 * align16(sizeof(T) * AT.share.rows);
 }
 
-template <class T, class V, bool ONE>
+template <class T, class V>
 __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
     k_halpern_cluster(const __grid_constant__ HalpernClusterArgs<T, V> a) {
     using namespace cluster;
@@ -327,14 +317,13 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
     make_sends(R.row0, R.rows, yv, a.A.share, mem, &ys_out);
     cluster_sync();
     Chunk<T, V> rc, qc;
-    if (ONE && warp < R.chunks) rc.load(R, warp, xv.v);
-    if (ONE && warp < Q.chunks) qc.load(Q, warp, yv.v);
+    if (warp < R.chunks) rc.load(R, warp, xv.v);
+    if (warp < Q.chunks) qc.load(Q, warp, yv.v);
     const T tau = static_cast<T>(a.st->eta / a.st->omega), sigma = static_cast<T>(a.st->eta * a.st->omega);
     bool ok = true;
     for (int it = 0; it < a.iterations && ok; ++it) {
         const T lam = halpern_lambda<T>(a.st, a.first + it);
-        for (int j = warp; j < Q.chunks; j += kClusterWarps) {
-            if (!ONE) qc.load(Q, j, yv.v);
+        if (warp < Q.chunks) {
             const T aty = qc.sum(Q, yv.v, sp);
             if (qc.owns) {
                 const int r = qc.r;
@@ -344,8 +333,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
             }
         }
         ok = exchange(xs_out, xr, xv);
-        for (int j = warp; j < R.chunks; j += kClusterWarps) {
-            if (!ONE) rc.load(R, j, xv.v);
+        if (warp < R.chunks) {
             const T axb = rc.sum(R, xv.v, sp);
             if (rc.owns) {
                 const int r = rc.r;
