@@ -75,6 +75,26 @@ def test_cluster_equals_launches(engine, instances, shape, entry):
     assert got[0][2] == got[1][2]
 
 
+@pytest.mark.parametrize("check_every,limit", [(1, 300), (7, 9001), (4096, 8193), (4097, 8195)])
+@pytest.mark.parametrize("tolerance", [0.3, 1e-3, 1e-300])
+def test_checkpoints_in_the_kernel_equal_the_hosts(engine, instances, check_every, limit, tolerance):
+    """Without a time limit a cluster judges its checkpoints itself, over launches of 4096
+    iterations at most; a limit that never runs out leaves them to the host. The same
+    residuals and the same stop, bit for bit."""
+    inst = lp(instances, 257, 300, [3, 5, 0], seed=2)
+    A = engine.Matrix.from_instance(inst)
+    ps, ds = steps(inst)
+    norm = np.sqrt((0.9 / ps - 1).max() * (0.9 / ds - 1).max())
+    got = []
+    for seconds in (0.0, 1e9):
+        rc, x, _, r = engine.pdhg(A, inst, engine.settings(max_iterations=limit, check_every=check_every, tau=0.9 / norm,
+                                                           sigma=0.9 / norm, tolerance=tolerance, time_limit=seconds))
+        assert rc == 0
+        got.append((x, r))
+    assert np.array_equal(got[0][0], got[1][0])
+    assert got[0][1] == got[1][1]
+
+
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}x{s[1]}")
 @pytest.mark.parametrize("precision", ["FP64", "FP32_REFINE", "BF16_REFINE"])
 def test_adaptive_cluster_equals_launches(engine, instances, shape, precision):

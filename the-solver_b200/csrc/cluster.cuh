@@ -453,6 +453,27 @@ struct Chunk {
     }
 };
 
+// Chunks in whole blocks of eight, as the launches have them (at most 32 blocks: a CTA has at
+// most a chunk per warp).
+inline __host__ __device__ int padded_chunks(int ntiles) { return (ntiles + 7) / 8 * 8; }
+
+// Sums of 8 chunks from v, at most 32 of them, by the tree over 256 blocks (one warp): its
+// levels 128, 64 and 32 add zeros.
+__device__ __forceinline__ double tree_of_blocks(const double* v, int padded) {
+    const int lane = threadIdx.x & 31;
+    auto leaf = [&](int g) {
+        double e[8], r = 0.0;
+        if (8 * g >= padded) return r;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) e[w] = v[8 * g + w];
+        r = e[0];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) r = r + e[w];
+        return r;
+    };
+    return warp_sum(leaf(lane));
+}
+
 // Whether a cluster of kClusterCtas CTAs of `kernel`, each with all of the shared
 // memory, fits the current device (asked once per kernel and device, which also sets
 // the kernel's attributes).

@@ -15,6 +15,37 @@
 
 namespace b200 {
 
+// The checkpoints of a solve, taken by the kernel itself: every `every` iterations (and
+// after the last) the residuals of the current point, whose maxima all CTAs exchange and
+// judge alike (about 1.5 iterations' time), so that a solve without a time limit needs no
+// launch and no host between its windows. As five launches, a copy and a wait on the host
+// they took 40 us, and the next window's launch and setup 20 more: at 2,000 x 5,000, 1,000
+// iterations judged every 20 (the C core's loop) 5.86 ms -> 3.50, judged every 100
+// 3.35 -> 3.22. every 0: none.
+struct FixedChecks {
+    int every = 0;
+    double tolerance = 0.0, dual_limit = 0.0;   // CUDA: the tolerance; SK: primal_tol and dual_tol (1 + anorm)
+    int first = 1;          // no checkpoint of this solve before this launch
+    double* x_prev = nullptr;   // CUDA: the last checkpoint's x
+    double* activity = nullptr; // SK: A x of the last checkpoint
+    double* out = nullptr;      // [0] iterations run, [1] verdict, [2] checkpoints, [3 ..] the last one's maxima
+};
+enum Verdict { kUnmet = 0, kMet = 1, kNotFinite = 2 };
+// CUDA: the rows' 5 and the columns' 6 maxima, then the objective; SK: violation, step, scale, dual step.
+constexpr int kCheckMaxima = 11, kObjectiveSlot = 11, kCheckTotals = 12;
+
+// The gates on the combined maxima (sankhya_cuda_lp.cu:361-385, sk_solve.c:926-953).
+template <bool SK>
+__device__ __forceinline__ int judge(const double* v, const FixedChecks& k, bool first) {
+    if (SK) return v[0] <= k.tolerance && v[1] <= k.tolerance * fmax(1.0, v[2]) && v[3] <= k.dual_limit ? kMet : kUnmet;
+    const double objective = v[kObjectiveSlot];
+    if (fmax(v[0], v[5]) > 0.0 || !isfinite(objective)) return kNotFinite;
+    const double tol = k.tolerance;
+    return v[1] <= tol && !first && v[6] <= tol * fmax(1.0, v[7]) && fmax(v[2], v[8]) <= tol && fmax(v[3], v[9]) <= tol &&
+                   fmax(v[4], v[10]) / (1.0 + fabs(objective)) <= tol
+               ? kMet : kUnmet;
+}
+
 struct FixedClusterArgs {
     TileCsr A, AT;
     const double *c, *cl, *cu, *tauv, *qdiag;  // tauv / sigv / qdiag may be null
@@ -25,6 +56,7 @@ struct FixedClusterArgs {
     double* part;                   // SK: max |y_new - y| of the last iteration, one per CTA
     int iterations;
     unsigned int* fail;             // set when a wait gave up
+    FixedChecks check;
 };
 
 // Shared memory of one CTA; 0 when the problem has no rows or no columns, or a CTA would
@@ -37,12 +69,22 @@ inline size_t fixed_cluster_smem(const TileCsr& A, const TileCsr& AT) {
            cluster::packed_bytes<double>(AT) + cluster::send_bytes(A.share) + cluster::send_bytes(AT.share) +
            4 * cluster::align16(8ull * A.share.rows) + 7 * cluster::align16(8ull * AT.share.rows);
 }
+// What the checkpoints add: what all CTAs send of one, twice in turn, its barriers, and the
+// warps' maxima.
+template <bool SK>
+__host__ __device__ inline int gathered_length(const TileCsr& AT) {
+    return cluster::kClusterCtas * kCheckMaxima + (SK ? 0 : cluster::padded_chunks(AT.ntiles));
+}
+template <bool SK>
+inline size_t fixed_check_smem(const TileCsr& AT) {
+    return 2 * cluster::align16(8ull * gathered_length<SK>(AT)) + 16 + 8ull * cluster::kClusterWarps * kCheckMaxima;
+}
 
 template <bool SK>
 __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(const __grid_constant__ FixedClusterArgs a) {
     using namespace cluster;
     extern __shared__ __align__(16) char smem[];
-    __shared__ double red[kClusterWarps];
+    __shared__ double red[kClusterWarps], own[kCheckMaxima + kClusterWarps], total[kCheckTotals];
     const unsigned rank = cta_rank();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Arena mem{smem};
@@ -64,6 +106,17 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
     double* cl = mem.take<double>(a.AT.share.rows);
     double* cu = mem.take<double>(a.AT.share.rows);
     double* tau = mem.take<double>(a.AT.share.rows);
+    double* gathered[2] = {nullptr, nullptr};   // per CTA its maxima, then all column chunks' objectives
+    unsigned long long* gathered_bar = nullptr;
+    double* maxima = nullptr;
+    if (a.check.every) {
+        gathered[0] = mem.take<double>(gathered_length<SK>(a.AT));
+        gathered[1] = mem.take<double>(gathered_length<SK>(a.AT));
+        gathered_bar = mem.take<unsigned long long>(2);
+        maxima = mem.take<double>(kClusterWarps * kCheckMaxima);
+        if (threadIdx.x < 2) init_barrier(gathered_bar + threadIdx.x);
+        for (int k = threadIdx.x; !SK && k < gathered_length<SK>(a.AT); k += blockDim.x) gathered[0][k] = gathered[1][k] = 0.0;
+    }
     fill_packed(a.A, xv, a.x_bar);
     for (int r = threadIdx.x; r < R.rows; r += blockDim.x) {
         const int i = R.row0 + r;
@@ -89,8 +142,10 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
     if (warp < Q.chunks) qc.load(Q, warp, yv.v);
     double change = 0.0;
     bool ok = true;
-    for (int it = 0; it < a.iterations && ok; ++it) {
+    int it = 0, verdict = kUnmet, checks = 0;
+    for (; it < a.iterations && ok && verdict == kUnmet; ++it) {
         const bool last = it + 1 == a.iterations;
+        const bool check = a.check.every && (last || (it + 1) % a.check.every == 0);
         if (warp < R.chunks) {
             const double act = rc.sum(R, xv.v, sp);
             if (rc.owns) {
@@ -99,7 +154,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
                 const double yn = SK ? dual_step_sk(old, act, sig[r], rl[r], ru[r])
                                      : dual_step_cuda(old, act, sig[r], rl[r], ru[r]);
                 y[r] = yn;
-                if (SK && last) change = fmax(change, fabs(dsub(yn, old)));
+                if (SK && (last || check)) change = fabs(dsub(yn, old));
             }
         }
         ok = exchange(ys_out, y, yv);
@@ -115,7 +170,89 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
                 xb[r] = SK ? dsub(dmul(2.0, xn), old) : dadd(xn, dmul(a.theta, dsub(xn, old)));
             }
         }
-        ok = exchange(xs_out, xb, xv) && ok;
+        ok = exchange(xs_out, check ? x : xb, xv) && ok;
+        if (!check) continue;
+        // the point's residuals: x at all CTAs for A x, y still there for A'y
+        constexpr int kSlots = SK ? 4 : kCheckMaxima;
+        double v[kCheckMaxima], objective = 0.0;
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k) v[k] = 0.0;
+        if (warp < R.chunks) {
+            const double act = rc.sum(R, xv.v, sp);
+            if (rc.owns) {
+                const int r = rc.r;
+                if (SK) {
+                    a.check.activity[R.row0 + r] = act;
+                    if (!sk_neg_inf(rl[r])) v[0] = fmax(v[0], rl[r] - act);
+                    if (!sk_inf(ru[r])) v[0] = fmax(v[0], act - ru[r]);
+                    v[3] = change;
+                } else {
+                    CheckRowsCudaEpi::Acc acc;
+                    acc.init();
+                    CheckRowsCudaEpi{y, rl, ru, nullptr}.row(r, act, acc);
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) v[k] = acc.v[k];
+                }
+            }
+        }
+        if (warp < Q.chunks) {
+            const double g = SK ? 0.0 : qc.sum(Q, yv.v, sp);
+            if (qc.owns) {
+                const int r = qc.r;
+                if (SK) {
+                    v[1] = fabs(xb[r] - x[r]);
+                    v[2] = fabs(x[r]);
+                } else {
+                    CheckColsCudaEpi::Acc acc;
+                    acc.init();
+                    CheckColsCudaEpi{x, a.check.x_prev + Q.row0, c, a.qdiag ? a.qdiag + Q.row0 : nullptr, nullptr, cl, cu,
+                                     nullptr}.row(r, g, acc);
+                    v[5] = acc.v[0];
+                    objective = acc.v[1];
+#pragma unroll
+                    for (int k = 2; k < 7; ++k) v[4 + k] = acc.v[k];
+                }
+            }
+            if (!SK) {
+                objective = warp_sum(objective);
+                if (lane == 0) own[kSlots + warp] = objective;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[k] = fmax(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+            if (lane == 0) maxima[warp * kCheckMaxima + k] = v[k];
+        }
+        __syncthreads();
+        if (threadIdx.x < kSlots) {
+            double t = maxima[threadIdx.x];
+            for (int w = 1; w < kClusterWarps; ++w) t = fmax(t, maxima[w * kCheckMaxima + threadIdx.x]);
+            own[threadIdx.x] = t;
+        }
+        __syncthreads();
+        double* all = checks & 1 ? gathered[1] : gathered[0];
+        double* sums = all + kClusterCtas * kCheckMaxima;
+        unsigned long long* bar = gathered_bar + (checks & 1);
+        if (threadIdx.x == 0) expect_bytes(bar, 8u * (kClusterCtas * kSlots + (SK ? 0 : a.AT.ntiles)));
+        if (lane < kSlots + (SK ? 0 : Q.chunks))   // warp w sends to CTA w
+            send_one(remote(lane < kSlots ? all + static_cast<int>(rank) * kCheckMaxima + lane
+                                          : sums + static_cast<int>(rank) * a.AT.share.chunks + lane - kSlots, warp),
+                     own[lane], remote(bar, warp));
+        ok = wait_bytes(bar, static_cast<unsigned>(checks >> 1) & 1u) && ok;
+        if (threadIdx.x < kSlots) {
+            double t = all[threadIdx.x];
+            for (int w = 1; w < kClusterCtas; ++w) t = fmax(t, all[w * kCheckMaxima + threadIdx.x]);
+            total[threadIdx.x] = t;
+        }
+        if (!SK && warp == 1) {
+            const double t = tree_of_blocks(sums, padded_chunks(a.AT.ntiles));
+            if (lane == 0) total[kObjectiveSlot] = t;
+        }
+        ok = __syncthreads_and(ok);
+        verdict = judge<SK>(total, a.check, a.check.first && checks == 0);
+        ++checks;
+        if (verdict == kUnmet && !last) ok = exchange(xs_out, xb, xv) && ok;   // on: x_bar after all
     }
     if (!ok && threadIdx.x == 0) *a.fail = 1u;
     cluster_sync();
@@ -124,7 +261,14 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
         a.x_bar[Q.row0 + j] = xb[j];
     }
     for (int i = threadIdx.x; i < R.rows; i += blockDim.x) a.y_out[R.row0 + i] = y[i];
-    if (SK) {
+    if (a.check.every) {
+        if (rank == 0 && threadIdx.x < (SK ? 4 : kCheckTotals)) a.check.out[3 + threadIdx.x] = total[threadIdx.x];
+        if (rank == 0 && threadIdx.x == 0) {
+            a.check.out[0] = it;
+            a.check.out[1] = verdict;
+            a.check.out[2] = checks;
+        }
+    } else if (SK) {
         for (int o = 16; o > 0; o >>= 1) change = fmax(change, __shfl_xor_sync(0xffffffffu, change, o));
         if (lane == 0) red[warp] = change;
         __syncthreads();

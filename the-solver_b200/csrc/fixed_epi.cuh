@@ -18,6 +18,9 @@ __device__ __forceinline__ double primal_step_cuda(double x, double g, double c,
     return box_ieee(trial, lo, hi);
 }
 
+__device__ __forceinline__ bool sk_inf(double v) { return v >= 1.0e30; }
+__device__ __forceinline__ bool sk_neg_inf(double v) { return v <= -1.0e30; }
+
 // c/src/sk_solve.c:901-906, :908-923
 __device__ __forceinline__ double dual_step_sk(double y, double act, double s, double lo, double hi) {
     const double trial = dadd(y, dmul(s, act));
@@ -123,9 +126,10 @@ struct CheckColsCudaEpi {
         const double xj = x[j], lo = cl[j], hi = cu[j], cj = c[j];
         const double qxj = qx ? qx[j] : 0.0;
         if (!isfinite(xj) || !isfinite(aty) || !isfinite(qxj)) acc.max(0, 1.0);
-        double obj = cj * xj;
-        if (qdiag) obj += 0.5 * qdiag[j] * xj * xj;
-        else if (qx) obj += 0.5 * xj * qxj;
+        // the fused forms spelled out: the same bits in every kernel that takes this row
+        double obj = dmul(cj, xj);
+        if (qdiag) obj = fma(0.5 * qdiag[j] * xj, xj, obj);
+        else if (qx) obj = fma(0.5 * xj, qxj, obj);
         acc.add(1, obj);
         acc.max(2, fabs(xj - x_prev[j]));
         x_prev[j] = xj;

@@ -78,9 +78,6 @@ struct PrimalSkEpi {
     __device__ __forceinline__ void finish(Acc&, double*) const {}
 };
 
-__device__ __forceinline__ bool sk_inf(double v) { return v >= 1.0e30; }
-__device__ __forceinline__ bool sk_neg_inf(double v) { return v <= -1.0e30; }
-
 // sk checkpoint, rows of A: stores the activity; slots 0 primal violation
 // (c/src/sk_solve.c:82-95), 1 row dual infeasibility, 2 row complementarity
 // (the row half of sk_verify, c/src/sk_core.c:471-498).
@@ -276,6 +273,7 @@ struct Solver {
     void (*flow_kernel)(FixedFlowArgs) = nullptr;
     void (*cluster_kernel)(FixedClusterArgs) = nullptr;
     size_t cluster_smem = 0;  // > 0: the iterations run on one cluster
+    bool cluster_checks = false;  // and there is room for its own checkpoints
     int flow_ctas = 0;        // > 0: the iterations run as one cooperative launch
     int dual_blocks = 0;      // partials the last dual step left in part_c
 
@@ -286,6 +284,9 @@ struct Solver {
         cluster_kernel = sem == Sem::Cuda ? &k_fixed_cluster<false> : &k_fixed_cluster<true>;
         cluster_smem = need > 0 && need <= cluster::kMaxSmem &&
                                cluster::available(reinterpret_cast<const void*>(cluster_kernel)) ? need : 0;
+        const size_t with_checks = need + (sem == Sem::Cuda ? fixed_check_smem<false>(*AT) : fixed_check_smem<true>(*AT));
+        cluster_checks = cluster_smem && with_checks <= cluster::kMaxSmem;
+        if (cluster_checks) cluster_smem = with_checks;
         flow_ctas = 0;
         if (!cluster_smem && !Q && flow::flow_pays(*A, *AT)) {
             flow_kernel = sem == Sem::Cuda ? &k_fixed_flow<false> : &k_fixed_flow<true>;
@@ -328,17 +329,41 @@ struct Solver {
     // k iterations as cluster launches of up to cluster::kMaxSteps.
     int run_cluster(int k) {
         while (k > 0) {
-            const int steps = std::min(k, cluster::kMaxSteps), nx = cur ^ 1;
-            const FixedClusterArgs a{*A, *AT, w->c, w->cl, w->cu, has_steps ? w->tauv : nullptr,
-                                     has_qdiag ? w->qdiag : nullptr, w->rl, w->ru, has_steps ? w->sigv : nullptr,
-                                     tau, sigma, theta, w->x[cur], w->y[cur], w->x[nx], w->y[nx], w->x_bar, w->part_c,
-                                     steps, w->flags + 1};
-            B200_TRY(cluster::launch(cluster_kernel, a, cluster_smem, stream), "cluster launch");
-            ++launches;
-            cur = nx;
+            const int steps = std::min(k, cluster::kMaxSteps);
+            if (launch_cluster(steps, FixedChecks{})) return -1;
             k -= steps;
         }
         dual_blocks = cluster::kClusterCtas;
+        return 0;
+    }
+    int launch_cluster(int steps, const FixedChecks& check) {
+        const int nx = cur ^ 1;
+        const FixedClusterArgs a{*A, *AT, w->c, w->cl, w->cu, has_steps ? w->tauv : nullptr,
+                                 has_qdiag ? w->qdiag : nullptr, w->rl, w->ru, has_steps ? w->sigv : nullptr,
+                                 tau, sigma, theta, w->x[cur], w->y[cur], w->x[nx], w->y[nx], w->x_bar, w->part_c,
+                                 steps, w->flags + 1, check};
+        B200_TRY(cluster::launch(cluster_kernel, a, cluster_smem, stream), "cluster launch");
+        ++launches;
+        cur = nx;
+        return 0;
+    }
+
+    // Whether the solve's checkpoints can be left to the kernel: no time limit to look at
+    // between them, no per-kernel timing.
+    bool checks_itself(int every, double time_limit) const {
+        return cluster_checks && !(time_limit > 0.0) && every <= cluster::kMaxSteps && timing().level < 2;
+    }
+    // Up to `steps` iterations with checkpoints, until one is met: iterations run, verdict and
+    // maxima in host[0 ..] (Workspace::out and the flags).
+    int run_checked(int steps, FixedChecks check, double* host) {
+        check.x_prev = w->x_prev;
+        check.activity = w->act;
+        check.out = w->out;
+        const int most = cluster::kMaxSteps / check.every * check.every;
+        if (launch_cluster(std::min(steps, most), check)) return -1;
+        B200_TRY(cudaMemcpyAsync(host, w->out, 33 * sizeof(double), cudaMemcpyDeviceToHost, stream), "read checkpoint");
+        B200_TRY(cudaStreamSynchronize(stream), "checkpoint");
+        if (cluster_gave_up(host + 32)) return fail_msg("a wait inside the iteration kernel gave up");
         return 0;
     }
 
@@ -570,7 +595,39 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     bool have_prev = false;
     int final_iteration = s.max_iterations, it = 0;
     const double started = now_seconds();
-    while (it < s.max_iterations) {
+    if (sv.checks_itself(s.check_every, s.time_limit)) {
+        FixedChecks check;
+        check.every = s.check_every;
+        check.tolerance = s.tolerance;
+        EventTimer t_loop(timed, stream);
+        while (it < s.max_iterations) {
+            if (sv.run_checked(s.max_iterations - it, check, host)) return -1;
+            check.first = 0;
+            it += static_cast<int>(host[0]);
+            ts.last.checkpoints += static_cast<int>(host[2]);
+            const double* v = host + 3;
+            const double objective = v[kObjectiveSlot];
+            if (host[1] == kNotFinite) {
+                result->status = -2;
+                ts.last.kernel_launches = sv.launches;
+                return -2;
+            }
+            result->objective = objective;
+            result->maximum_row_violation = std::max(0.0, v[1]);
+            // the step is against the checkpoint before, so the first one has none
+            result->maximum_step = ts.last.checkpoints > 1 ? v[6] : std::numeric_limits<double>::infinity();
+            result->maximum_kkt_residual = std::max(v[2], v[8]);
+            result->maximum_dual_residual = std::max(v[3], v[9]);
+            result->maximum_complementarity = std::max(v[4], v[10]) / (1.0 + std::fabs(objective));
+            if (host[1] == kMet) {
+                final_iteration = it;
+                result->status = 0;
+                break;
+            }
+        }
+        ts.last.iterations = it;
+        ts.last.loop_ms = t_loop.stop();
+    } else while (it < s.max_iterations) {
         if (s.time_limit > 0.0 && (it + 1) % s.check_every == 1 && now_seconds() - started >= s.time_limit) {
             final_iteration = it;
             result->status = 2;
@@ -785,7 +842,22 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
     double dual_step = std::numeric_limits<double>::infinity();
     bool activity_is_ax = false;
     const double start = now_seconds();
-    while (it < max_it) {
+    if (!q && sv.checks_itself(check_every, time_limit)) {
+        FixedChecks check;
+        check.every = check_every;
+        check.tolerance = ptol;
+        check.dual_limit = dtol * (1.0 + anorm);
+        while (it < max_it && !converged) {
+            if (sv.run_checked(max_it - it, check, host)) return -1;
+            check.first = 0;
+            it += static_cast<int>(host[0]);
+            ts.last.checkpoints += static_cast<int>(host[2]);
+            dual_step = host[3 + 3];
+            converged = host[1] == kMet;
+            activity_is_ax = true;
+        }
+        ts.last.iterations = it;
+    } else while (it < max_it) {
         const int next = std::min((it / check_every + 1) * check_every, max_it);
         if (sv.run(next - it)) return -1;
         ts.last.iterations += next - it;

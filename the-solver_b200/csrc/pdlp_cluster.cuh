@@ -33,23 +33,6 @@ struct ChunkSums {
     unsigned bytes;                // of one exchange
 };
 
-// Sums of 8 chunks from v, at most 32 of them, by the tree over 256 blocks (one warp): its
-// levels 128, 64 and 32 add zeros.
-__device__ __forceinline__ double tree_of_blocks(const double* v, int padded) {
-    const int lane = threadIdx.x & 31;
-    auto leaf = [&](int g) {
-        double e[8], r = 0.0;
-        if (8 * g >= padded) return r;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) e[w] = v[8 * g + w];
-        r = e[0];
-#pragma unroll
-        for (int w = 1; w < 8; ++w) r = r + e[w];
-        return r;
-    };
-    return warp_sum(leaf(lane));
-}
-
 template <class T, class V>
 struct AdaptiveClusterArgs {
     TileCsrT<V> A, AT;
@@ -60,8 +43,6 @@ struct AdaptiveClusterArgs {
     double* fail;
     int iterations;
 };
-
-inline int padded_chunks(int ntiles) { return (ntiles + 7) / 8 * 8; }
 
 // Shared memory of one CTA; 0 when there are no rows or columns. (A CTA has at most a chunk
 // per warp, so there are at most 32 blocks of eight.)
