@@ -14,11 +14,14 @@
 // the device with per-LP maxima (atomic max on the bit patterns of non-negative
 // doubles, so the result does not depend on the order); an LP that passes is
 // frozen (its iterates are carried through unchanged) and the host reads only
-// the number of LPs still running. Per LP the arithmetic is exactly the
+// the number of LPs still running. Where it is faster (plan_batch), each LP runs
+// by itself on one CTA or a cluster of them instead (batch_cluster.cuh). Per LP the arithmetic is exactly the
 // single-LP loop's, so every LP's iterates equal a separate solve's bit for bit.
+#include "batch_cluster.cuh"
 #include "batch_common.cuh"
 
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 #include <limits>
 #include <map>
@@ -115,14 +118,32 @@ struct BatchRowsEpi {
     __device__ __forceinline__ void finish(Acc&, double*) const {}
 };
 
+// slots[k] = max(slots[k], v) of the lanes that are in: one atomic a warp where they share an
+// LP, as nearly all warps do (with one per element the atomics were the kernels' whole time:
+// 1.1M columns of 512 LPs, 137 us for k_steps_and_max and 162 for k_batch_cols).
+__device__ __forceinline__ void segment_max(unsigned long long* slots, int k, bool in, unsigned long long v) {
+    const unsigned lanes = __ballot_sync(0xffffffffu, in);
+    if (!lanes) return;
+    const int lead = __shfl_sync(0xffffffffu, k, __ffs(lanes) - 1);
+    if (__all_sync(0xffffffffu, !in || k == lead)) {
+        if (!in) v = 0;
+        for (int o = 16; o > 0; o >>= 1) v = max_u64(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if ((threadIdx.x & 31) == 0 && v) atomicMax(slots + lead, v);
+    } else if (in && v) {
+        atomicMax(slots + k, v);
+    }
+}
+
 __global__ void k_batch_cols(int n, const double* __restrict__ x, const double* __restrict__ x_bar,
                              const int* __restrict__ seg, const int* __restrict__ done,
                              unsigned long long* __restrict__ scale, unsigned long long* __restrict__ step) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += blockDim.x * gridDim.x) {
-        const int k = seg[j];
-        if (done[k]) continue;
-        atomic_max_nonneg(&scale[k], fabs(x[j]));
-        atomic_max_nonneg(&step[k], fabs(x_bar[j] - x[j]));
+    for (int b = blockIdx.x * blockDim.x + (threadIdx.x & ~31); b < n; b += blockDim.x * gridDim.x) {
+        const int j = b + (threadIdx.x & 31);
+        const int k = j < n ? seg[j] : 0;
+        const bool in = j < n && !done[k];
+        const double v = in ? x[j] : 0.0;
+        segment_max(scale, k, in, max_bits(fabs(v)));
+        segment_max(step, k, in, in ? max_bits(fabs(x_bar[j] - v)) : 0ull);
     }
 }
 
@@ -154,9 +175,11 @@ __global__ void k_batch_gate(int batch, int iteration, int last, double ptol, do
 
 __global__ void k_steps_and_max(int len, const double* __restrict__ mass, const int* __restrict__ seg,
                                 double* __restrict__ steps, unsigned long long* __restrict__ segmax) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < len; j += blockDim.x * gridDim.x) {
-        steps[j] = 0.9 / (1.0 + mass[j]);
-        atomic_max_nonneg(&segmax[seg[j]], mass[j]);
+    for (int b = blockIdx.x * blockDim.x + (threadIdx.x & ~31); b < len; b += blockDim.x * gridDim.x) {
+        const int j = b + (threadIdx.x & 31);
+        const double v = j < len ? mass[j] : 0.0;
+        if (j < len) steps[j] = 0.9 / (1.0 + v);
+        segment_max(segmax, j < len ? seg[j] : 0, j < len, max_bits(v));
     }
 }
 
@@ -181,6 +204,67 @@ __global__ void k_init_box(int n, const double* __restrict__ lo, const double* _
 }
 
 using batch::now_s;
+
+constexpr int kClusterWindow = 4096;   // iterations of one launch of k_batch_cluster
+
+// How the batch runs: on the launches (ctas 0) or on clusters of `ctas`, the `together` first of
+// `order` by whole clusters and the others by single CTAs.
+struct BatchPlan {
+    int ctas = 0, together = 0;
+    std::vector<int> order;
+};
+
+// Rule: the shorter time of an iteration by what was measured on a B200 (us; thousands of
+// nonzeros z, an LP's share taken by its rows and columns):
+//   a single CTA     1.8 + 1.1 z      (2.9 at 0.6, 8.5 at 6, 29 at 24, 69 at 60)
+//   2 or 4 CTAs      4.5 + 1.1 z / n  (four: 8.3 at 6, 10.9 at 24, 22.5 at 60)
+//   the launches     9.7, or 2 + 0.0155 z of the whole batch when longer (checks included)
+// and the largest LPs, longer than 0.85 of a CTA's even share, by whole clusters: 512 LPs of 50
+// to 5,000 rows 63.3 by single CTAs, 57.6 with the largest by pairs, 98.0 on the launches;
+// 296 of 500 rows 16.8, on the launches 26.3. Batches of a few LPs, where single CTAs leave the
+// others idle, stay on the launches, as does one with an LP too large for a CTA's shared memory
+// (some 18,000 rows and columns).
+BatchPlan plan_batch(const TileCsr& A, const TileCsr& AT, int batch, const int* row_seg, const int* col_seg, int nnz) {
+    BatchPlan p;
+    int rows_max = 0, cols_max = 0;
+    for (int k = 0; k < batch; ++k) {
+        rows_max = std::max(rows_max, row_seg[k + 1] - row_seg[k]);
+        cols_max = std::max(cols_max, col_seg[k + 1] - col_seg[k]);
+    }
+    for (const void* at : {static_cast<const void*>(A.val), static_cast<const void*>(A.idx), static_cast<const void*>(AT.val),
+                           static_cast<const void*>(AT.idx)})
+        if (reinterpret_cast<std::uintptr_t>(at) % 16) return p;   // the copy engine's alignment
+    const int slots = batch_clusters(1);
+    if (batch_cluster_smem(cols_max, rows_max) > kBatchClusterSmem || slots == 0 || A.ntiles == 0 || AT.ntiles == 0) return p;
+    p.order.resize(static_cast<size_t>(batch));
+    for (int k = 0; k < batch; ++k) p.order[k] = k;
+    auto size = [&](int k) { return row_seg[k + 1] - row_seg[k] + col_seg[k + 1] - col_seg[k]; };
+    std::stable_sort(p.order.begin(), p.order.end(), [&](int a, int b) { return size(a) > size(b); });
+    const double total = nnz / 1000.0, per = total / (static_cast<double>(A.rows) + AT.rows);
+    auto alone = [&](int at) { return 1.8 + 1.1 * per * size(p.order[at]); };
+    double sum = 0.0;
+    for (int k = 0; k < batch; ++k) sum += alone(k);
+    int large = 0;
+    while (large < batch && alone(large) > 0.85 * sum / slots) ++large;
+    double best = std::max(9.7, 2.0 + 0.0155 * total) / 1.1;   // so that a near tie stays where it was
+    for (int n : {1, 2, 4}) {
+        const int by_clusters = n > 1 ? large : 0;
+        if (batch_clusters(n) == 0) continue;
+        double work = 0.0, longest = 0.0;
+        for (int k = 0; k < batch; ++k) {
+            const double t = k < by_clusters ? 4.5 + (alone(k) - 1.8) / n : alone(k);
+            work += k < by_clusters ? n * t : t;
+            longest = std::max(longest, t);
+        }
+        const double t = std::max(longest, work / slots);
+        if (t < best) {
+            best = t;
+            p.ctas = n;
+            p.together = by_clusters;
+        }
+    }
+    return p;
+}
 
 }  // namespace
 
@@ -246,8 +330,8 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     const size_t kb = (static_cast<size_t>(batch) * 8 + 255) / 256 * 256;
     DevBuf blob;
     // 8 n-vectors + the column segment map, 7 m-vectors + the row segment map,
-    // 12 per-LP slots, counters
-    if (blob.alloc_on(stream, 9 * nb + 8 * mb + 12 * kb + 4096, "cudaMalloc batch workspace")) return -1;
+    // 15 per-LP slots, counters
+    if (blob.alloc_on(stream, 9 * nb + 8 * mb + 15 * kb + 4096, "cudaMalloc batch workspace")) return -1;
     char* p = blob.as<char>();
     auto take = [&](size_t b) { char* r = p; p += b; return r; };
     double *dc = reinterpret_cast<double*>(take(nb)), *dcl = reinterpret_cast<double*>(take(nb)),
@@ -269,6 +353,9 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     int* done = reinterpret_cast<int*>(take(kb));
     int* iters = reinterpret_cast<int*>(take(kb));
     double* report = reinterpret_cast<double*>(take(4 * kb));
+    int* d_row_seg = reinterpret_cast<int*>(take(kb + 256));
+    int* d_col_seg = reinterpret_cast<int*>(take(kb + 256));
+    int* d_order = reinterpret_cast<int*>(take(kb));
     unsigned int* counters = reinterpret_cast<unsigned int*>(take(256));
     const size_t n8 = sizeof(double) * static_cast<size_t>(n), m8 = sizeof(double) * static_cast<size_t>(m);
     if (n) {
@@ -302,6 +389,15 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     B200_TRY(cudaStreamSynchronize(stream), "batch setup");
     if (host_counters[1]) return fail_msg("matrix is not block-diagonal over the given segments");
 
+    const BatchPlan way = plan_batch(A, AT, batch, row_segments, col_segments, matrix->nnz);
+    const int ctas = way.ctas;
+    if (ctas) {
+        const size_t b4 = sizeof(int) * static_cast<size_t>(batch);
+        B200_TRY(cudaMemcpyAsync(d_order, way.order.data(), b4, cudaMemcpyHostToDevice, stream), "upload order");
+        B200_TRY(cudaMemcpyAsync(d_row_seg, row_segments, b4 + 4, cudaMemcpyHostToDevice, stream), "upload segments");
+        B200_TRY(cudaMemcpyAsync(d_col_seg, col_segments, b4 + 4, cudaMemcpyHostToDevice, stream), "upload segments");
+    }
+
     double* xb[2] = {xb0, xb1};
     double* yb[2] = {yb0, yb1};
     const int grid_d = tiled_grid<BatchDualEpi>(A), grid_p = tiled_grid<BatchPrimalEpi>(AT);
@@ -325,7 +421,31 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     bool timed_out = false;
     int checks = 0;
     batch::LoopEvents loop_events(timing().level >= 1, stream);
-    while (it < s.max_iterations) {
+    // On clusters: windows of whole checks, one check's with a time limit to look at.
+    BatchClusterArgs on_clusters{A, AT, dc, dcl, dcu, tau, drl, dru, sig, xb0, xbar, yb0, d_row_seg, d_col_seg, d_order,
+                                 cmax, rmax, done, iters, report, counters, counters + 2, counters + 4, way.together, batch, 0, 0, 0, 0,
+                                 s.max_iterations, s.check_every, s.primal_tol, s.dual_tol};
+    for (int k = 0; k < batch; ++k) {
+        on_clusters.rows_max = std::max(on_clusters.rows_max, row_segments[k + 1] - row_segments[k]);
+        on_clusters.cols_max = std::max(on_clusters.cols_max, col_segments[k + 1] - col_segments[k]);
+    }
+    const int window = s.time_limit > 0.0 ? s.check_every : std::max(1, kClusterWindow / s.check_every) * s.check_every;
+    while (ctas && it < s.max_iterations) {
+        on_clusters.begin = it;
+        on_clusters.end = it = static_cast<int>(std::min<long long>(static_cast<long long>(it) + window, s.max_iterations));
+        B200_TRY(cudaMemsetAsync(counters, 0, 20, stream), "zero counters");
+        B200_TRY(launch_batch_cluster(on_clusters, ctas, batch_clusters(ctas), stream), "cluster launch");
+        ++launches;
+        B200_TRY(cudaMemcpyAsync(host_counters, counters, 20, cudaMemcpyDeviceToHost, stream), "read");
+        B200_TRY(cudaStreamSynchronize(stream), "batch check");
+        if (host_counters[4]) return fail_msg("a wait inside the iteration kernel gave up");
+        if (host_counters[0] == 0) break;
+        if (s.time_limit > 0.0 && now_s() - t0 >= s.time_limit) {
+            timed_out = true;
+            break;
+        }
+    }
+    while (!ctas && it < s.max_iterations) {
         const int next = std::min((it / s.check_every + 1) * s.check_every, s.max_iterations);
         int k = next - it;
         while (k > 0) {
@@ -379,6 +499,11 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     B200_TRY(cudaMemcpyAsync(h_report.data(), report, sizeof(double) * 4 * batch, cudaMemcpyDeviceToHost, stream),
              "download");
     B200_TRY(cudaStreamSynchronize(stream), "batch download");
+    if (ctas) {
+        // the last check that an LP took
+        it = *std::max_element(h_iters.begin(), h_iters.end());
+        checks = (it + s.check_every - 1) / s.check_every;
+    }
     for (int k = 0; k < batch; ++k) {
         SankhyaB200BatchResult& r = results[k];
         r.status = h_done[k] ? 0 : (timed_out ? 2 : 1);
