@@ -288,18 +288,13 @@ __device__ __forceinline__ float load_value<float, __nv_bfloat16>(const __nv_bfl
     return __bfloat162float(__ldcs(p));
 }
 
-template <class Epi, class T, class V = T>
-__global__ void __launch_bounds__(kThreads) k_tiled(TileCsrT<V> A, const T* __restrict__ v, Epi epi) {
+// The chunks t, t + nw, ... of one warp, its products in sp.
+template <class Epi, class T, class V>
+__device__ __forceinline__ void tile_rows(const TileCsrT<V>& A, const T* __restrict__ v, const Epi& epi,
+                                          typename Epi::Acc& acc, T* sp, int t, int nw) {
     using P = RowPre<Epi>;
-    __shared__ T prod[kWarps][kChunkNnz];
-    __shared__ double red[kWarps * 8];
-    typename Epi::Acc acc;
-    acc.init();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = gridDim.x * kWarps;
-    T* sp = prod[warp];
+    const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
-    int t = blockIdx.x * kWarps + warp;
     int2 b0 = t < A.ntiles ? __ldg(A.tile + t) : make_int2(0, 0);
     int2 b1 = t < A.ntiles ? __ldg(A.tile + t + 1) : make_int2(0, 0);
     for (; t < A.ntiles; t += nw) {
@@ -376,6 +371,16 @@ __global__ void __launch_bounds__(kThreads) k_tiled(TileCsrT<V> A, const T* __re
         b0 = n0;
         b1 = n1;
     }
+}
+
+template <class Epi, class T, class V = T>
+__global__ void __launch_bounds__(kThreads) k_tiled(TileCsrT<V> A, const T* __restrict__ v, Epi epi) {
+    __shared__ T prod[kWarps][kChunkNnz];
+    __shared__ double red[kWarps * 8];
+    typename Epi::Acc acc;
+    acc.init();
+    const int warp = threadIdx.x >> 5;
+    tile_rows(A, v, epi, acc, prod[warp], blockIdx.x * kWarps + warp, gridDim.x * kWarps);
     epi.finish(acc, red);
 }
 
@@ -400,6 +405,26 @@ inline int launch_tiled(const TileCsrT<V>& A, const T* v, const Epi& epi, cudaSt
     if (A.ntiles == 0) return 0;
     k_tiled<Epi, T, V><<<grid, kThreads, 0, stream>>>(A, v, epi);
     return 0;
+}
+
+// Two independent products in one launch: the warps go on to B's chunks where A's end, so that
+// neither a second launch's start nor its last, part-filled wave is waited for.
+template <class Epi, class EpiB>
+__global__ void __launch_bounds__(kThreads) k_tiled_pair(TileCsr A, const double* __restrict__ v, Epi epi, TileCsr B,
+                                                         const double* __restrict__ w, EpiB epi_b) {
+    __shared__ double prod[kWarps][kChunkNnz];
+    __shared__ double red[kWarps * 8];
+    typename Epi::Acc acc;
+    acc.init();
+    const int warp = threadIdx.x >> 5, t = blockIdx.x * kWarps + warp, nw = gridDim.x * kWarps;
+    tile_rows(A, v, epi, acc, prod[warp], t, nw);
+    NoAcc none;
+    tile_rows(B, w, epi_b, none, prod[warp], (t + nw - A.ntiles % nw) % nw, nw);
+    epi.finish(acc, red);
+}
+template <class Epi, class EpiB>
+inline int tiled_pair_grid(const TileCsr& A, const TileCsr& B) {
+    return grid_for(reinterpret_cast<const void*>(&k_tiled_pair<Epi, EpiB>), (A.ntiles + B.ntiles + kWarps - 1) / kWarps, 0);
 }
 
 // Final fixed-order combine of per-block partials: out[k] = op_g partial[g*NS+k].

@@ -292,11 +292,12 @@ struct Solver {
             flow_kernel = sem == Sem::Cuda ? &k_fixed_flow<false> : &k_fixed_flow<true>;
             flow_ctas = flow::resident_ctas(reinterpret_cast<const void*>(flow_kernel), kFlowThreads, 0);
         }
+        const bool pair = Q && Q->ntiles;
         if (sem == Sem::Cuda) {
-            grid_dual = tiled_grid<DualCudaEpi>(*A);
+            grid_dual = pair ? tiled_pair_grid<DualCudaEpi, StoreEpi>(*A, *Q) : tiled_grid<DualCudaEpi>(*A);
             grid_primal = tiled_grid<PrimalCudaEpi>(*AT);
         } else {
-            grid_dual = tiled_grid<DualSkEpi>(*A);
+            grid_dual = pair ? tiled_pair_grid<DualSkEpi, StoreEpi>(*A, *Q) : tiled_grid<DualSkEpi>(*A);
             grid_primal = tiled_grid<PrimalSkEpi>(*AT);
         }
         if (Q) grid_q = tiled_grid<StoreEpi>(*Q);
@@ -371,19 +372,19 @@ struct Solver {
     void iterate(cudaEvent_t* ev) {
         const int nx = cur ^ 1;
         if (ev) cudaEventRecord(ev[0], stream);
-        if (sem == Sem::Cuda) {
-            launch_tiled(*A, w->x_bar,
-                         DualCudaEpi{w->y[cur], w->rl, w->ru, has_steps ? w->sigv : nullptr, sigma, w->y[nx]},
-                         stream, grid_dual);
-        } else {
-            launch_tiled(*A, w->x_bar, DualSkEpi{w->y[cur], w->rl, w->ru, w->sigv, w->y[nx], w->part_c}, stream,
-                         grid_dual);
-        }
+        // Q x needs only x: with a Hessian it shares the dual step's launch (k_tiled_pair; 100,000
+        // x 200,000, 2M nonzeros: 46.3 us an iteration as a launch of its own, 39.9 so).
+        const DualCudaEpi dual_cuda{w->y[cur], w->rl, w->ru, has_steps ? w->sigv : nullptr, sigma, w->y[nx]};
+        const DualSkEpi dual_sk{w->y[cur], w->rl, w->ru, w->sigv, w->y[nx], w->part_c};
+        if (Q && Q->ntiles && sem == Sem::Cuda)
+            k_tiled_pair<<<grid_dual, kThreads, 0, stream>>>(*A, w->x_bar, dual_cuda, *Q, w->x[cur], StoreEpi{w->qx});
+        else if (Q && Q->ntiles)
+            k_tiled_pair<<<grid_dual, kThreads, 0, stream>>>(*A, w->x_bar, dual_sk, *Q, w->x[cur], StoreEpi{w->qx});
+        else if (sem == Sem::Cuda)
+            launch_tiled(*A, w->x_bar, dual_cuda, stream, grid_dual);
+        else
+            launch_tiled(*A, w->x_bar, dual_sk, stream, grid_dual);
         if (ev) cudaEventRecord(ev[1], stream);
-        if (Q) {
-            launch_tiled(*Q, w->x[cur], StoreEpi{w->qx}, stream, grid_q);
-            ++launches;
-        }
         if (ev) cudaEventRecord(ev[2], stream);
         if (sem == Sem::Cuda) {
             launch_tiled(*AT, w->y[nx],
@@ -443,7 +444,7 @@ struct Solver {
                 launches = saved_launches;
             }
             B200_TRY(cudaGraphLaunch(it->second, stream), "graph launch");
-            launches += chunk * (Q ? 3 : 2);
+            launches += 2 * chunk;
             cur ^= (chunk & 1);
             k -= chunk;
         }
