@@ -377,9 +377,9 @@ struct Solver {
         const DualCudaEpi dual_cuda{w->y[cur], w->rl, w->ru, has_steps ? w->sigv : nullptr, sigma, w->y[nx]};
         const DualSkEpi dual_sk{w->y[cur], w->rl, w->ru, w->sigv, w->y[nx], w->part_c};
         if (Q && Q->ntiles && sem == Sem::Cuda)
-            k_tiled_pair<<<grid_dual, kThreads, 0, stream>>>(*A, w->x_bar, dual_cuda, *Q, w->x[cur], StoreEpi{w->qx});
+            launch_early(k_tiled_pair<DualCudaEpi, StoreEpi>, grid_dual, stream, *A, w->x_bar, dual_cuda, *Q, w->x[cur], StoreEpi{w->qx});
         else if (Q && Q->ntiles)
-            k_tiled_pair<<<grid_dual, kThreads, 0, stream>>>(*A, w->x_bar, dual_sk, *Q, w->x[cur], StoreEpi{w->qx});
+            launch_early(k_tiled_pair<DualSkEpi, StoreEpi>, grid_dual, stream, *A, w->x_bar, dual_sk, *Q, w->x[cur], StoreEpi{w->qx});
         else if (sem == Sem::Cuda)
             launch_tiled(*A, w->x_bar, dual_cuda, stream, grid_dual);
         else
