@@ -17,10 +17,10 @@ namespace b200 {
 
 // The checkpoints of a solve, taken by the kernel itself: every `every` iterations (and
 // after the last) the residuals of the current point, whose maxima all CTAs exchange and
-// judge alike (about 1.5 iterations' time), so that a solve without a time limit needs no
+// test alike (about 1.5 iterations' time), so that a solve without a time limit needs no
 // launch and no host between its windows. As five launches, a copy and a wait on the host
 // they took 40 us, and the next window's launch and setup 20 more: at 2,000 x 5,000, 1,000
-// iterations judged every 20 (the C core's loop) 5.86 ms -> 3.50, judged every 100
+// iterations tested every 20 (the C core's loop) 5.86 ms -> 3.50, tested every 100
 // 3.35 -> 3.22. every 0: none.
 struct FixedChecks {
     int every = 0;
@@ -36,7 +36,7 @@ constexpr int kCheckMaxima = 11, kObjectiveSlot = 11, kCheckTotals = 12;
 
 // The gates on the combined maxima (sankhya_cuda_lp.cu:361-385, sk_solve.c:926-953).
 template <bool SK>
-__device__ __forceinline__ int judge(const double* v, const FixedChecks& k, bool first) {
+__device__ __forceinline__ int gates(const double* v, const FixedChecks& k, bool first) {
     if (SK) return v[0] <= k.tolerance && v[1] <= k.tolerance * fmax(1.0, v[2]) && v[3] <= k.dual_limit ? kMet : kUnmet;
     const double objective = v[kObjectiveSlot];
     if (fmax(v[0], v[5]) > 0.0 || !isfinite(objective)) return kNotFinite;
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
             if (lane == 0) total[kObjectiveSlot] = t;
         }
         ok = __syncthreads_and(ok);
-        verdict = judge<SK>(total, a.check, a.check.first && checks == 0);
+        verdict = gates<SK>(total, a.check, a.check.first && checks == 0);
         ++checks;
         if (verdict == kUnmet && !last) ok = exchange(xs_out, xb, xv) && ok;   // on: x_bar after all
     }
