@@ -183,6 +183,13 @@ __global__ void k_steps_and_max(int len, const double* __restrict__ mass, const 
     }
 }
 
+// Nonzeros of each LP.
+__global__ void k_segment_entries(int batch, const int* __restrict__ row_seg, const int* __restrict__ ptr,
+                                  int* __restrict__ out) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < batch; k += blockDim.x * gridDim.x)
+        out[k] = ptr[row_seg[k + 1]] - ptr[row_seg[k]];
+}
+
 // Block-diagonal structure: every nonzero of row i lies in the columns of i's LP.
 __global__ void k_check_blocks(int rows, const int* __restrict__ ptr, const int* __restrict__ idx,
                                const int* __restrict__ rseg, const int* __restrict__ cseg,
@@ -214,8 +221,8 @@ struct BatchPlan {
     std::vector<int> order;
 };
 
-// Rule: the shorter time of an iteration by what was measured on a B200 (us; thousands of
-// nonzeros z, an LP's share taken by its rows and columns):
+// Rule: the shorter time of an iteration by what was measured on a B200 (us; z: an LP's
+// nonzeros, or 4 per row and column if those are more, in thousands):
 //   a single CTA     1.8 + 1.1 z      (2.9 at 0.6, 8.5 at 6, 29 at 24, 69 at 60)
 //   2 or 4 CTAs      4.5 + 1.1 z / n  (four: 8.3 at 6, 10.9 at 24, 22.5 at 60)
 //   the launches     9.7, or 2 + 0.0155 z of the whole batch when longer (checks included)
@@ -223,8 +230,9 @@ struct BatchPlan {
 // to 5,000 rows 63.3 by single CTAs, 57.6 with the largest by pairs, 98.0 on the launches;
 // 296 of 500 rows 16.8, on the launches 26.3. Batches of a few LPs, where single CTAs leave the
 // others idle, stay on the launches, as does one with an LP too large for a CTA's shared memory
-// (some 18,000 rows and columns).
-BatchPlan plan_batch(const TileCsr& A, const TileCsr& AT, int batch, const int* row_seg, const int* col_seg, int nnz) {
+// (some 19,000 rows and columns).
+BatchPlan plan_batch(const TileCsr& A, const TileCsr& AT, int batch, const int* row_seg, const int* col_seg,
+                     const std::vector<int>& entries) {
     BatchPlan p;
     int rows_max = 0, cols_max = 0;
     for (int k = 0; k < batch; ++k) {
@@ -238,10 +246,12 @@ BatchPlan plan_batch(const TileCsr& A, const TileCsr& AT, int batch, const int* 
     if (batch_cluster_smem(cols_max, rows_max) > kBatchClusterSmem || slots == 0 || A.ntiles == 0 || AT.ntiles == 0) return p;
     p.order.resize(static_cast<size_t>(batch));
     for (int k = 0; k < batch; ++k) p.order[k] = k;
-    auto size = [&](int k) { return row_seg[k + 1] - row_seg[k] + col_seg[k + 1] - col_seg[k]; };
+    auto size = [&](int k) {
+        return std::max<long long>(entries[k], 4ll * (row_seg[k + 1] - row_seg[k] + col_seg[k + 1] - col_seg[k]));
+    };
     std::stable_sort(p.order.begin(), p.order.end(), [&](int a, int b) { return size(a) > size(b); });
-    const double total = nnz / 1000.0, per = total / (static_cast<double>(A.rows) + AT.rows);
-    auto alone = [&](int at) { return 1.8 + 1.1 * per * size(p.order[at]); };
+    const double total = A.nnz / 1000.0;
+    auto alone = [&](int at) { return 1.8 + 1.1e-3 * size(p.order[at]); };
     double sum = 0.0;
     for (int k = 0; k < batch; ++k) sum += alone(k);
     int large = 0;
@@ -376,6 +386,11 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     const TileCsr& A = plan->a;
     const TileCsr& AT = plan->at;
     const int ge = elem_grid(std::max(m, n));
+    const size_t seg_bytes = sizeof(int) * (static_cast<size_t>(batch) + 1);
+    B200_TRY(cudaMemcpyAsync(d_row_seg, row_segments, seg_bytes, cudaMemcpyHostToDevice, stream), "upload segments");
+    B200_TRY(cudaMemcpyAsync(d_col_seg, col_segments, seg_bytes, cudaMemcpyHostToDevice, stream), "upload segments");
+    if (m) k_segment_entries<<<elem_grid(batch), kThreads, 0, stream>>>(batch, d_row_seg, A.ptr, d_order);
+    else B200_TRY(cudaMemsetAsync(d_order, 0, sizeof(int) * static_cast<size_t>(batch), stream), "zero entries");
     if (m) k_check_blocks<<<elem_grid(m), kThreads, 0, stream>>>(m, A.ptr, A.idx, d_rseg, d_cseg, counters + 1);
     if (m) k_abs_sums<<<elem_grid(m), kThreads, 0, stream>>>(m, A.ptr, A.val, rmass);
     if (n) k_abs_sums<<<elem_grid(n), kThreads, 0, stream>>>(n, AT.ptr, AT.val, cmass);
@@ -385,18 +400,16 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     B200_TRY(cudaGetLastError(), "batch setup");
     unsigned int* host_counters = reinterpret_cast<unsigned int*>(pinned_slot());
     if (!host_counters) return fail_msg("cudaMallocHost counters");
+    std::vector<int> entries(static_cast<size_t>(batch));
     B200_TRY(cudaMemcpyAsync(host_counters, counters, 8, cudaMemcpyDeviceToHost, stream), "read");
+    B200_TRY(cudaMemcpyAsync(entries.data(), d_order, sizeof(int) * batch, cudaMemcpyDeviceToHost, stream), "read");
     B200_TRY(cudaStreamSynchronize(stream), "batch setup");
     if (host_counters[1]) return fail_msg("matrix is not block-diagonal over the given segments");
 
-    const BatchPlan way = plan_batch(A, AT, batch, row_segments, col_segments, matrix->nnz);
+    const BatchPlan way = plan_batch(A, AT, batch, row_segments, col_segments, entries);
     const int ctas = way.ctas;
-    if (ctas) {
-        const size_t b4 = sizeof(int) * static_cast<size_t>(batch);
-        B200_TRY(cudaMemcpyAsync(d_order, way.order.data(), b4, cudaMemcpyHostToDevice, stream), "upload order");
-        B200_TRY(cudaMemcpyAsync(d_row_seg, row_segments, b4 + 4, cudaMemcpyHostToDevice, stream), "upload segments");
-        B200_TRY(cudaMemcpyAsync(d_col_seg, col_segments, b4 + 4, cudaMemcpyHostToDevice, stream), "upload segments");
-    }
+    if (ctas) B200_TRY(cudaMemcpyAsync(d_order, way.order.data(), sizeof(int) * way.order.size(), cudaMemcpyHostToDevice, stream),
+                       "upload order");
 
     double* xb[2] = {xb0, xb1};
     double* yb[2] = {yb0, yb1};
