@@ -35,6 +35,11 @@ typedef struct SankhyaB200Timing {
 SANKHYA_CUDA_API void sankhya_b200_set_timing(int level);
 SANKHYA_CUDA_API void sankhya_b200_last_timing(SankhyaB200Timing* out);
 
+/* Polls after which a wait inside an iteration kernel (for another thread block's
+   elements, or for a copy) gives up; the call then returns -1. Negative: the default,
+   some seconds. 0 lets every such wait fail. Thread-local. */
+SANKHYA_CUDA_API void sankhya_b200_set_wait_limit(int polls);
+
 /* --------------------------------------------------- sk_solve continuous hook */
 
 /* Layout-compatible copies of the reference's public model types

@@ -437,7 +437,7 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     // On clusters: windows of whole checks, one check's with a time limit to look at.
     BatchClusterArgs on_clusters{A, AT, dc, dcl, dcu, tau, drl, dru, sig, xb0, xbar, yb0, d_row_seg, d_col_seg, d_order,
                                  cmax, rmax, done, iters, report, counters, counters + 2, counters + 4, way.together, batch, 0, 0, 0, 0,
-                                 s.max_iterations, s.check_every, s.primal_tol, s.dual_tol};
+                                 s.max_iterations, s.check_every, wait_limit(cluster::kMaxTries), s.primal_tol, s.dual_tol};
     for (int k = 0; k < batch; ++k) {
         on_clusters.rows_max = std::max(on_clusters.rows_max, row_segments[k + 1] - row_segments[k]);
         on_clusters.cols_max = std::max(on_clusters.cols_max, col_segments[k + 1] - col_segments[k]);

@@ -36,6 +36,7 @@ struct BatchClusterArgs {
     int together;                           // the first of `order`, each by a whole cluster
     int batch, cols_max, rows_max;          // the largest LP's
     int begin, end, max_iterations, every;  // iterations begin .. end of the run
+    int tries;                              // polls of a wait
     double ptol, dtol;
 };
 
@@ -76,7 +77,8 @@ constexpr unsigned kPadAt = 8 * (kChunkNnz + 2), kBarAt = kPadAt + 8, kColumnsAt
                    kStageBytes = kColumnsAt + 4 * (kChunkNnz + 4);
 struct Stage {
     unsigned at, phase;
-    bool dead;   // a wait gave up
+    int tries;   // polls of a wait
+    bool dead;   // a wait gave up: the warp starts no copy and gathers nothing any more
 
     __device__ __forceinline__ void init() {
         asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(at + kBarAt) : "memory");
@@ -90,21 +92,28 @@ struct Stage {
     // Starts the copy of entries [p0, p1); the lanes have fenced what they wrote here. The blocks
     // read hold an entry each, so they lie in the arrays' memory.
     __device__ __forceinline__ void fetch(const double* val, const int* idx, int p0, int p1) const {
-        if (threadIdx.x & 31) return;
+        if ((threadIdx.x & 31) || dead) return;
         const unsigned n = p1 - p0;
         const unsigned v = 8u * (((p0 & 1u) + n + 1u) & ~1u), x = 4u * (((p0 & 3u) + n + 3u) & ~3u);
         asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(at + kBarAt), "r"(v + x) : "memory");
         bulk(at, val + (p0 & ~1), v);
         bulk(at + kColumnsAt, idx + (p0 & ~3), x);
     }
-    __device__ __forceinline__ void wait() {
+    __device__ __forceinline__ bool poll(int most) const {
         unsigned done = 0;
-        for (int tries = 0; !done && !dead && tries < cluster::kMaxTries; ++tries)
+        for (int k = 0; !done && k < most; ++k)
             asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
                          "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(at + kBarAt), "r"(phase) : "memory");
-        dead = !done;
-        phase ^= 1u;
+        return done != 0;
     }
+    // All lanes come to the same answer. A dead warp has one copy in flight at most, which lands
+    // in its own stage; drain waits for it before the CTA's shared memory goes.
+    __device__ __forceinline__ void wait() {
+        if (dead) return;
+        dead = __any_sync(0xffffffffu, !poll(tries));
+        phase ^= dead ? 0u : 1u;
+    }
+    __device__ __forceinline__ void drain() const { (void)poll(cluster::kMaxTries); }
 };
 
 // Rows [r0, r1) and entries [p0, p1) of a chunk, cut to the LP's rows.
@@ -165,10 +174,12 @@ __device__ __forceinline__ void sweep(const Rows& R, Stage& st, Cut cur, Head<P>
     const TileCsr& M = R.M;
     for (int t = R.first; t < R.end; t += R.step) {
         const Cut next = R.cut(t + R.step);
-        const int n = cur.p1 - cur.p0;
         const bool owns = cur.r0 + lane < cur.r1;
         double s = 0.0;
         if (Rows::copied(cur)) st.wait();
+        // without its copy the stage's columns are no columns of this LP: no entry is taken, and
+        // the call fails
+        const int n = st.dead ? 0 : cur.p1 - cur.p0;
         if (n > kChunkNnz) {
             double s0 = 0.0, s1 = 0.0;
             int p = cur.p0 + lane;
@@ -196,7 +207,7 @@ __device__ __forceinline__ void sweep(const Rows& R, Stage& st, Cut cur, Head<P>
                     if (32 * (g + k) + lane < n) cluster::sts(sv + 256u * (g + k), v[k]);
             }
             __syncwarp();
-            const int len = owns ? h.q1 - h.q0 : 0;
+            const int len = owns && n ? h.q1 - h.q0 : 0;
             const int own_len = len <= kShortRow ? len : 0;
             const int longest = __reduce_max_sync(full, own_len);
             const unsigned e = sp + 8 * h.q0, end = e + 8 * own_len, pad = st.at + kPadAt;
@@ -242,7 +253,7 @@ __global__ void __launch_bounds__(kLpThreads, 1) k_batch_cluster(const __grid_co
     double* xb = mem.take<double>(a.cols_max);
     double* y = mem.take<double>(a.rows_max);
     const unsigned xb_at = shared_address(xb), y_at = shared_address(y);
-    Stage stage{shared_address(mem.take<char>(kLpWarps * kStageBytes)) + warp * kStageBytes, 0u, false};
+    Stage stage{shared_address(mem.take<char>(kLpWarps * kStageBytes)) + warp * kStageBytes, 0u, a.tries, false};
     if (lane == 0) stage.init();
     bool together = all_ctas > 1;   // the largest LPs by all CTAs of the cluster, then each CTA its own
     if (together) cluster_sync();   // every CTA runs before its shared memory is written
@@ -376,7 +387,10 @@ __global__ void __launch_bounds__(kLpThreads, 1) k_batch_cluster(const __grid_co
         for (int i = t0; i < r1 - r0; i += ctas * kLpThreads) a.y[r0 + i] = y[i];
         for (int j = t0; j < c1 - c0; j += ctas * kLpThreads) a.x_bar[c0 + j] = xb[j];
     }
-    if (stage.dead) *a.failed = 1u;
+    if (stage.dead) {
+        stage.drain();
+        *a.failed = 1u;
+    }
 }
 
 // Clusters of `ctas` CTAs that run at once on the current device; 0 when none fits (asked once

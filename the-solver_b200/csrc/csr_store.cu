@@ -375,6 +375,13 @@ TimingState& timing() {
     return state;
 }
 
+static int& wait_limit_set() {
+    thread_local int polls = -1;
+    return polls;
+}
+
+int wait_limit(int usual) { return wait_limit_set() < 0 ? usual : wait_limit_set(); }
+
 // ------------------------------------------------------------ small kernels
 
 __global__ void k_fill(double* __restrict__ out, double value, int n) {
@@ -392,6 +399,8 @@ using namespace b200;
 extern "C" const char* sankhya_cuda_last_error(void) { return g_last_error; }
 
 extern "C" void sankhya_b200_set_timing(int level) { timing().level = level; }
+
+extern "C" void sankhya_b200_set_wait_limit(int polls) { wait_limit_set() = polls; }
 
 extern "C" void sankhya_b200_last_timing(SankhyaB200Timing* out) {
     if (out) *out = timing().last;

@@ -131,6 +131,10 @@ struct TimingState {
 };
 TimingState& timing();
 
+// Polls after which a wait inside an iteration kernel gives up: `usual`, or what
+// sankhya_b200_set_wait_limit set on this thread.
+int wait_limit(int usual);
+
 // ------------------------------------------------------- device arithmetic
 // Explicit round-to-nearest intrinsics: no multiply-add contraction, so the
 // elementwise updates round exactly like the reference's host C code.
