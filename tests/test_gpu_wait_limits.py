@@ -21,7 +21,7 @@ def fails_then_works(engine, call):
     engine.set_wait_limit(0)
     try:
         rc, _ = call()
-        assert rc == -1 and "gave up" in engine.last_error()
+        assert rc != 0 and "gave up" in engine.last_error()
     finally:
         engine.set_wait_limit(-1)
     rc, after = call()
@@ -46,3 +46,52 @@ def test_batch_on_ctas(engine, instances, kind):
         rc, x, y, _ = engine.batch_pdhg(A, blk, rseg, cseg, s, want_dual=True)
         return rc, (x, y)
     fails_then_works(engine, call)
+
+
+def loop_call(engine, oracle, inst, limit, time_limit=0.0, tol=1e-300):
+    """The C core's loop; returns a function for fails_then_works."""
+    import ctypes as C
+    keep = oracle._Keep()
+    model = oracle.build_sk_model(keep, inst, False)
+
+    def call():
+        opts = oracle.SkOptions(primal_tol=tol, dual_tol=tol, iteration_limit=limit, threads=1, time_limit=time_limit)
+        x, y, act = np.zeros(inst["n"]), np.zeros(inst["m"]), np.zeros(inst["m"])
+        res = engine.LoopResult()
+        rc = engine.lib().sankhya_b200_pdhg_loop(C.byref(model), C.byref(opts), engine._p(x), engine._p(y),
+                                                 engine._p(act), C.byref(res))
+        return rc, (x, y, act, res.iterations, res.dual_step, keep is None)
+    return call
+
+
+def fixed_call(engine, inst):
+    A = engine.Matrix.from_instance(inst)
+    kw = dict(max_iterations=100, check_every=40, tau=0.05, sigma=0.05, tolerance=1e-300)
+    return lambda: (lambda rc, x, _, r: (rc, (x, r["objective"])))(*engine.pdhg(A, inst, engine.settings(**kw)))
+
+
+def pdlp_call(engine, inst, **kw):
+    A = engine.Matrix.from_instance(inst)
+    s = engine.pdlp_default_settings()
+    s.max_iterations, s.eps_optimal, s.ruiz_iterations = 150, 1e-300, 5
+    for k, v in kw.items():
+        setattr(s, k, v)
+    return lambda: (lambda rc, x, y, r: (rc, (x, y)))(*engine.pdlp_solve(A, inst, s))
+
+
+def solve_call(engine, oracle, inst, entry):
+    if entry == "fixed":
+        return fixed_call(engine, inst)
+    if entry == "loop":
+        return loop_call(engine, oracle, inst, 100)
+    if entry == "halpern":
+        return pdlp_call(engine, inst, algorithm=engine.PDLP_HALPERN)
+    return pdlp_call(engine, inst, precision=getattr(engine, entry))
+
+
+ENTRIES = ["fixed", "loop", "halpern", "FP64", "FP32_REFINE", "BF16_REFINE"]
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+def test_cooperative_launch(engine, oracle, instances, entry):
+    fails_then_works(engine, solve_call(engine, oracle, instances.lp_uniform(6, 8000, 16000, 8), entry))

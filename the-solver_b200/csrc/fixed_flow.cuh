@@ -20,6 +20,7 @@ struct FixedFlowArgs {
     flow::Tagged<double>*xt, *yt;   // x_bar and y by iteration
     unsigned long long first;       // number of this launch's first iteration; its start has the one before
     int iterations;
+    int polls;                      // of a thread's waits in one iteration
     unsigned int* fail;
 };
 
@@ -38,7 +39,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fixed_flow(const __grid_con
     for (int it = 0; it < a.iterations; ++it) {
         const bool last = it + 1 == a.iterations;
         const unsigned long long tag = a.first + it;   // of this iteration's y and x_bar
-        int left = kMaxPolls;
+        int left = a.polls;
         for (int t = mine; t < a.A.ntiles; t += nw) {
             const ChunkRows c = chunk_rows(a.A, t);
             const int i = c.row;
@@ -79,8 +80,8 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fixed_flow(const __grid_con
                 if (last) a.x_bar[j] = xb;   // its reader above is through: this column's rows have moved on
             }
         }
-        if (left <= 0) {
-            *a.fail = 1u;
+        if (__any_sync(0xffffffffu, left <= 0)) {
+            if (lane == 0) *a.fail = 1u;
             break;
         }
     }

@@ -14,7 +14,9 @@
 // No element is overwritten before it has been read: a row's owner stores its next y only
 // after it has gathered x from all the columns of the row, and those columns' owners have
 // stored that x after they gathered this y (A and A' have the same entries). All CTAs are
-// resident (cooperative launch), so every wait ends; each is bounded all the same.
+// resident (cooperative launch), so every wait ends; each is bounded all the same. A warp (in
+// the adaptive loop a CTA) whose wait gave up leaves as a whole, since the sums need all lanes;
+// those that wait for its elements give up in turn.
 //
 // Row sums keep k_tiled's order, so every iterate has the same bits.
 //
@@ -31,7 +33,7 @@
 namespace b200 {
 namespace flow {
 
-constexpr int kMaxPolls = 1 << 22;    // loads of one wait, some seconds
+constexpr int kMaxPolls = 1 << 22;    // loads of a thread's waits in one iteration, some seconds
 
 // An element and the iteration it belongs to, read and written as one access.
 template <class T>

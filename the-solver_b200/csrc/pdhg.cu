@@ -316,7 +316,7 @@ struct Solver {
             const FixedFlowArgs a{*A, *AT, w->c, w->cl, w->cu, has_steps ? w->tauv : nullptr,
                                   has_qdiag ? w->qdiag : nullptr, w->rl, w->ru, has_steps ? w->sigv : nullptr, tau, sigma,
                                   theta, w->x[cur], w->y[cur], w->x[nx], w->y[nx], w->x_bar, w->part_c, w->xt, w->yt,
-                                  w->epoch, steps, w->flags + 1};
+                                  w->epoch, steps, wait_limit(flow::kMaxPolls), w->flags + 1};
             B200_TRY(flow::launch(flow_kernel, a, flow_ctas, kFlowThreads, 0, stream), "cooperative launch");
             ++launches;
             w->epoch += steps + 1;

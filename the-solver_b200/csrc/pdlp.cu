@@ -1541,7 +1541,7 @@ struct Core {
                 const int steps = std::min(period - done, cluster::kMaxSteps);
                 const AdaptiveFlowArgs<T, V> a{A, AT, x, x_cand, x_sum, y, y_cand, y_sum, ax, ax_prev, ax_cand, c, cl, cu,
                                                rl, ru, ctr ? ctr->yc : nullptr, st, res + kFail, xt, yt, sums, count, arrived, epoch,
-                                               steps};
+                                               steps, wait_limit(flow::kMaxPolls)};
                 B200_TRY(flow::launch(&k_adaptive_flow<T, V>, a, adaptive_ctas, kFlowThreads, kFlowSmem + kSumsSmem, stream),
                          "cooperative launch");
                 epoch += steps;
@@ -1643,7 +1643,7 @@ struct Core {
             for (int done = 0; done < period; done += cluster::kMaxSteps) {
                 const int steps = std::min(period - done, cluster::kMaxSteps);
                 const HalpernFlowArgs<T, V> a{A, AT, x, y, x_restart, y_restart, c, cl, cu, rl, ru, st, res + kFail, xt, yt,
-                                              epoch + 1, done, steps};
+                                              epoch + 1, done, steps, wait_limit(flow::kMaxPolls)};
                 B200_TRY(flow::launch(&k_halpern_flow<T, V>, a, halpern_ctas, kFlowThreads, kFlowSmem, stream),
                          "cooperative launch");
                 epoch += steps + 1;

@@ -41,7 +41,7 @@ struct AdaptiveFlowArgs {
     unsigned* count;               // CTAs that have published their sums, over all launches
     unsigned arrived;              // its value at the start
     unsigned first;                // number of the first iteration
-    int iterations;
+    int iterations, polls;         // polls of a thread's waits in one iteration
 };
 
 // The chunk of this warp in round q of a step.
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_adaptive_flow(const __grid_
     for (int it = 0; it < a.iterations && ok; ++it) {
         const typename TagOf<T>::type tag = a.first + it;
         const T sigma = static_cast<T>(eta * omega), tau = static_cast<T>(eta / omega);
-        int left = kMaxPolls;
+        int left = a.polls;
         for (int q = 0, t; (t = flow_chunk(q)) < (a.A.ntiles + 7) / 8 * 8; ++q) {
             if (t >= a.A.ntiles) continue;
             const int i = __ldg(a.A.tile + t).x + lane;
@@ -253,6 +253,7 @@ struct HalpernFlowArgs {
     flow::Tagged<T>*xt, *yt;
     unsigned first;        // number of the first iteration; the start has the one before
     int done, iterations;  // of the window
+    int polls;             // of a thread's waits in one iteration
 };
 
 template <class T, class V>
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_halpern_flow(const __grid_c
     for (int it = 0; it < a.iterations; ++it) {
         const typename TagOf<T>::type tag = a.first + it;
         const T lam = halpern_lambda<T>(a.st, a.done + it);
-        int left = kMaxPolls;
+        int left = a.polls;
         for (int t = mine; t < a.AT.ntiles; t += nw) {
             const ChunkRows k = chunk_rows(a.AT, t);
             const int j = k.row;
@@ -307,8 +308,8 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_halpern_flow(const __grid_c
                 a.y[i] = yn;
             }
         }
-        if (left <= 0) {
-            *a.fail = 1.0;
+        if (__any_sync(0xffffffffu, left <= 0)) {
+            if ((threadIdx.x & 31) == 0) *a.fail = 1.0;
             break;
         }
     }
