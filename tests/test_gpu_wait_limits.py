@@ -95,3 +95,9 @@ ENTRIES = ["fixed", "loop", "halpern", "FP64", "FP32_REFINE", "BF16_REFINE"]
 @pytest.mark.parametrize("entry", ENTRIES)
 def test_cooperative_launch(engine, oracle, instances, entry):
     fails_then_works(engine, solve_call(engine, oracle, instances.lp_uniform(6, 8000, 16000, 8), entry))
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("shape", [(40, 31, 3), (2000, 5000, 5)], ids=str)
+def test_cluster(engine, oracle, instances, shape, entry):
+    fails_then_works(engine, solve_call(engine, oracle, instances.lp_uniform(7, *shape), entry))

@@ -87,10 +87,10 @@ __device__ __forceinline__ void expect_bytes(unsigned long long* bar, unsigned b
     asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(
                      static_cast<unsigned>(__cvta_generic_to_shared(bar))), "r"(bytes) : "memory");
 }
-// False when the wait gave up.
-__device__ __forceinline__ bool wait_bytes(unsigned long long* bar, unsigned phase) {
-    unsigned done = 0;
-    for (int tries = 0; !done && tries < kMaxTries; ++tries)
+// False when the wait gave up after `most` polls; true at once with `skip`.
+__device__ __forceinline__ bool wait_bytes(unsigned long long* bar, unsigned phase, int most, bool skip = false) {
+    unsigned done = skip;
+    for (int tries = 0; !done && tries < most; ++tries)
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
                      "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done)
                      : "r"(static_cast<unsigned>(__cvta_generic_to_shared(bar))), "r"(phase) : "memory");
@@ -309,24 +309,43 @@ __device__ __forceinline__ void make_sends(int row0, int rows, const Packed<T>& 
     __syncthreads();
 }
 
+// The waits of one thread, one of which may give up where other threads of the CTA see the same
+// phase end. Such a thread waits once more (bounded) for what is on its way to the CTA, then
+// sends, arms and waits no more but passes every block barrier as before: an early exit would
+// leave the others there. Whoever waits for its elements gives up in turn, so the launch ends
+// after a few limits, its sums garbage, its addresses as ever. (A test of all threads, by a
+// barrier that reduces or a flag read behind one, took 1 to 2 % of a small solve.)
+struct Waits {
+    SendList &xs, &ys;
+    const int& polls;   // of a wait
+    bool gave_up = false;
+
+    // Thread 0 arms: it knows by its own waits that the phase before has ended.
+    __device__ __forceinline__ bool arms() const { return threadIdx.x == 0 && !gave_up; }
+    __device__ __forceinline__ void wait(unsigned long long* bar, unsigned phase) {
+        if (wait_bytes(bar, phase, polls, gave_up)) return;
+        (void)wait_bytes(bar, phase, kMaxTries);
+        gave_up = true;
+        xs.count = ys.count = 0;
+    }
+};
+
 // Sends the CTA's own elements to the CTAs that gather them, and waits until this CTA's
-// packed copy has all of its elements. False when the wait gave up. `meanwhile` runs while
-// the elements are on their way.
+// packed copy has all of its elements. `meanwhile` runs while the elements are on their way.
 template <class T, class F>
-__device__ __forceinline__ bool exchange(const SendList& s, const T* own, Packed<T>& in, F meanwhile) {
+__device__ __forceinline__ void exchange(Waits& w, const SendList& s, const T* own, Packed<T>& in, F meanwhile) {
     __syncthreads();   // `own` is complete
-    if (threadIdx.x == 0) expect_bytes(in.bar, in.bytes);
+    if (w.arms()) expect_bytes(in.bar, in.bytes);
     for (int k = threadIdx.x & 31; k < s.count; k += 32)
         send_one(s.at + static_cast<unsigned>(sizeof(T)) * k, own[s.src[k]], s.bar);
     meanwhile();
-    const bool done = wait_bytes(in.bar, in.phase);
+    w.wait(in.bar, in.phase);
     in.phase ^= 1u;
-    return done;
 }
 
 template <class T>
-__device__ __forceinline__ bool exchange(const SendList& s, const T* own, Packed<T>& in) {
-    return exchange(s, own, in, [] {});
+__device__ __forceinline__ void exchange(Waits& w, const SendList& s, const T* own, Packed<T>& in) {
+    exchange(w, s, own, in, [] {});
 }
 
 // Shared-memory loads that stay where they are written: the entries of a batch are all

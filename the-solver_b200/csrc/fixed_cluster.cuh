@@ -54,7 +54,7 @@ struct FixedClusterArgs {
     const double *x_in, *y_in;
     double *x_out, *y_out, *x_bar;  // x_bar: in and out
     double* part;                   // SK: max |y_new - y| of the last iteration, one per CTA
-    int iterations;
+    int iterations, polls;          // polls of a wait
     unsigned int* fail;             // set when a wait gave up
     FixedChecks check;
 };
@@ -141,9 +141,9 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
     if (warp < R.chunks) rc.load(R, warp, xv.v);
     if (warp < Q.chunks) qc.load(Q, warp, yv.v);
     double change = 0.0;
-    bool ok = true;
+    Waits waits{xs_out, ys_out, a.polls};
     int it = 0, verdict = kUnmet, checks = 0;
-    for (; it < a.iterations && ok && verdict == kUnmet; ++it) {
+    for (; it < a.iterations && verdict == kUnmet; ++it) {
         const bool last = it + 1 == a.iterations;
         const bool check = a.check.every && (last || (it + 1) % a.check.every == 0);
         if (warp < R.chunks) {
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
                 if (SK && (last || check)) change = fabs(dsub(yn, old));
             }
         }
-        ok = exchange(ys_out, y, yv);
+        exchange(waits, ys_out, y, yv);
         if (warp < Q.chunks) {
             const double g = qc.sum(Q, yv.v, sp);
             if (qc.owns) {
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
                 xb[r] = SK ? dsub(dmul(2.0, xn), old) : dadd(xn, dmul(a.theta, dsub(xn, old)));
             }
         }
-        ok = exchange(xs_out, check ? x : xb, xv) && ok;
+        exchange(waits, xs_out, check ? x : xb, xv);
         if (!check) continue;
         // the point's residuals: x at all CTAs for A x, y still there for A'y
         constexpr int kSlots = SK ? 4 : kCheckMaxima;
@@ -234,12 +234,12 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
         double* all = checks & 1 ? gathered[1] : gathered[0];
         double* sums = all + kClusterCtas * kCheckMaxima;
         unsigned long long* bar = gathered_bar + (checks & 1);
-        if (threadIdx.x == 0) expect_bytes(bar, 8u * (kClusterCtas * kSlots + (SK ? 0 : a.AT.ntiles)));
-        if (lane < kSlots + (SK ? 0 : Q.chunks))   // warp w sends to CTA w
+        if (waits.arms()) expect_bytes(bar, 8u * (kClusterCtas * kSlots + (SK ? 0 : a.AT.ntiles)));
+        if (!waits.gave_up && lane < kSlots + (SK ? 0 : Q.chunks))   // warp w sends to CTA w
             send_one(remote(lane < kSlots ? all + static_cast<int>(rank) * kCheckMaxima + lane
                                           : sums + static_cast<int>(rank) * a.AT.share.chunks + lane - kSlots, warp),
                      own[lane], remote(bar, warp));
-        ok = wait_bytes(bar, static_cast<unsigned>(checks >> 1) & 1u) && ok;
+        waits.wait(bar, static_cast<unsigned>(checks >> 1) & 1u);
         if (threadIdx.x < kSlots) {
             double t = all[threadIdx.x];
             for (int w = 1; w < kClusterCtas; ++w) t = fmax(t, all[w * kCheckMaxima + threadIdx.x]);
@@ -249,12 +249,12 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1) k_fixed_cluster(c
             const double t = tree_of_blocks(sums, padded_chunks(a.AT.ntiles));
             if (lane == 0) total[kObjectiveSlot] = t;
         }
-        ok = __syncthreads_and(ok);
+        __syncthreads();
         verdict = gates<SK>(total, a.check, a.check.first && checks == 0);
         ++checks;
-        if (verdict == kUnmet && !last) ok = exchange(xs_out, xb, xv) && ok;   // on: x_bar after all
+        if (verdict == kUnmet && !last) exchange(waits, xs_out, xb, xv);   // on: x_bar after all
     }
-    if (!ok && threadIdx.x == 0) *a.fail = 1u;
+    if (waits.gave_up) *a.fail = 1u;
     cluster_sync();
     for (int j = threadIdx.x; j < Q.rows; j += blockDim.x) {
         a.x_out[Q.row0 + j] = x[j];

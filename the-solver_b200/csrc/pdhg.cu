@@ -342,7 +342,7 @@ struct Solver {
         const FixedClusterArgs a{*A, *AT, w->c, w->cl, w->cu, has_steps ? w->tauv : nullptr,
                                  has_qdiag ? w->qdiag : nullptr, w->rl, w->ru, has_steps ? w->sigv : nullptr,
                                  tau, sigma, theta, w->x[cur], w->y[cur], w->x[nx], w->y[nx], w->x_bar, w->part_c,
-                                 steps, w->flags + 1, check};
+                                 steps, wait_limit(cluster::kMaxTries), w->flags + 1, check};
         B200_TRY(cluster::launch(cluster_kernel, a, cluster_smem, stream), "cluster launch");
         ++launches;
         cur = nx;

@@ -1528,7 +1528,7 @@ struct Core {
             for (int done = 0; done < period; done += cluster::kMaxSteps) {
                 const AdaptiveClusterArgs<T, V> a{A, AT, x, x_sum, y, y_sum, ax, ax_prev, c, cl, cu, rl, ru,
                                                   ctr ? ctr->yc : nullptr, st, res + kFail,
-                                                  std::min(period - done, cluster::kMaxSteps)};
+                                                  std::min(period - done, cluster::kMaxSteps), wait_limit(cluster::kMaxTries)};
                 B200_TRY(cluster::launch(adaptive_kernel, a, adaptive_smem, stream), "cluster launch");
                 ++launches;
             }
@@ -1631,7 +1631,8 @@ struct Core {
         if (halpern_smem) {
             for (int done = 0; done < period; done += cluster::kMaxSteps) {
                 const HalpernClusterArgs<T, V> a{A, AT, x, y, x_restart, y_restart, c, cl, cu, rl, ru, st, res + kFail,
-                                                 done, std::min(period - done, cluster::kMaxSteps)};
+                                                 done, std::min(period - done, cluster::kMaxSteps),
+                                                 wait_limit(cluster::kMaxTries)};
                 B200_TRY(cluster::launch(halpern_kernel, a, halpern_smem, stream), "cluster launch");
                 ++launches;
             }

@@ -41,7 +41,7 @@ struct AdaptiveClusterArgs {
     const double* y_center;        // centered loop, else null
     PdlpState* st;
     double* fail;
-    int iterations;
+    int iterations, polls;         // polls of a wait
 };
 
 // Shared memory of one CTA; 0 when there are no rows or columns. (A CTA has at most a chunk
@@ -121,7 +121,8 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
     const double omega = a.st->omega, eta_lo = a.st->eta_min, eta_hi = a.st->eta_max;
     double eta = a.st->eta, updates = a.st->updates, accepts = a.st->accept_count;
     double dx2 = 0.0, dy2 = 0.0, cross = 0.0, limit = a.st->eta_bar;
-    bool keep = false, ok = true;
+    bool keep = false;
+    Waits waits{xs_out, ys_out, a.polls};
     // the accepted candidate becomes the iterate (k_commit_dual's first half)
     auto commit = [&](int r) {
         y[r] = yc[r];
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
             xsum[r] += xc[r];
         }
     };
-    for (int it = 0; it < a.iterations && ok; ++it) {
+    for (int it = 0; it < a.iterations; ++it) {
         const T sigma = static_cast<T>(eta * omega), tau = static_cast<T>(eta / omega);
         for (int r = threadIdx.x; r < R.rows; r += blockDim.x) {
             if (keep) commit(r);
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
                                : dual_candidate(y[r], ax[r], axp[r], sigma, rl[r], ru[r]);
         }
         if (keep) commit_columns();
-        ok = exchange(ys_out, yc, yv);
+        exchange(waits, ys_out, yc, yv);
         if (warp < Q.chunks) {
             const T aty = qc.sum(Q, yv.v, sp);
             double d = 0.0;
@@ -157,10 +158,10 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
             d = warp_sum(d);
             if (lane == 0) sums.own[warp] = d;
         }
-        ok = exchange(xs_out, xc, xv, [&] {
+        exchange(waits, xs_out, xc, xv, [&] {
             if (warp != kClusterWarps - 1 || lane >= 2) return;   // the warp with the fewest chunks
             growth[lane] = step_growth(updates + 1.0, lane == 0);
-        }) && ok;
+        });
         if (warp < R.chunks) {
             const T axn = rc.sum(R, xv.v, sp);
             double d = 0.0, e = 0.0;
@@ -181,16 +182,16 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
         __syncthreads();
         double* all = it & 1 ? sums.all1 : sums.all0;
         unsigned long long* bar = it & 1 ? sums.bar1 : sums.bar0;
-        if (threadIdx.x == 0) expect_bytes(bar, sums.bytes);
+        if (waits.arms()) expect_bytes(bar, sums.bytes);
         const unsigned to = remote(bar, warp);   // warp w sends to CTA w
-        for (int k = lane; k < Q.chunks + 2 * R.chunks; k += 32) {
+        for (int k = lane; k < Q.chunks + 2 * R.chunks && !waits.gave_up; k += 32) {
             const int at = k < Q.chunks ? static_cast<int>(rank) * a.AT.share.chunks + k
                            : k < Q.chunks + R.chunks
                                ? sums.cols + static_cast<int>(rank) * a.A.share.chunks + k - Q.chunks
                                : sums.cols + sums.rows + static_cast<int>(rank) * a.A.share.chunks + k - Q.chunks - R.chunks;
             send_one(remote(all + at, warp), sums.own[k], to);
         }
-        ok = wait_bytes(bar, static_cast<unsigned>(it >> 1) & 1u) && ok;
+        waits.wait(bar, static_cast<unsigned>(it >> 1) & 1u);
         if (warp < 3) {
             const double t = warp == 0 ? tree_of_blocks(all, sums.cols)
                                        : tree_of_blocks(all + sums.cols + (warp - 1) * sums.rows, sums.rows);
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
         st->accept_count = accepts;
         st->accepted = 0.0;   // committed above
     }
-    if (!ok && threadIdx.x == 0) *a.fail = 1.0;
+    if (waits.gave_up) *a.fail = 1.0;
 }
 
 template <class T, class V>
@@ -247,6 +248,7 @@ struct HalpernClusterArgs {
     const PdlpState* st;
     double* fail;
     int first, iterations;   // of the window
+    int polls;               // of a wait
 };
 
 template <class T, class V>
@@ -301,8 +303,8 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
     if (warp < R.chunks) rc.load(R, warp, xv.v);
     if (warp < Q.chunks) qc.load(Q, warp, yv.v);
     const T tau = static_cast<T>(a.st->eta / a.st->omega), sigma = static_cast<T>(a.st->eta * a.st->omega);
-    bool ok = true;
-    for (int it = 0; it < a.iterations && ok; ++it) {
+    Waits waits{xs_out, ys_out, a.polls};
+    for (int it = 0; it < a.iterations; ++it) {
         const T lam = halpern_lambda<T>(a.st, a.first + it);
         if (warp < Q.chunks) {
             const T aty = qc.sum(Q, yv.v, sp);
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
                 x[r] = halpern_step(lam, p, x0[r]);
             }
         }
-        ok = exchange(xs_out, xr, xv);
+        exchange(waits, xs_out, xr, xv);
         if (warp < R.chunks) {
             const T axb = rc.sum(R, xv.v, sp);
             if (rc.owns) {
@@ -321,11 +323,11 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
                 y[r] = halpern_step(lam, dual_reflected(y[r], axb, sigma, rl[r], ru[r]), y0[r]);
             }
         }
-        ok = exchange(ys_out, y, yv) && ok;
+        exchange(waits, ys_out, y, yv);
     }
     for (int r = threadIdx.x; r < R.rows; r += blockDim.x) a.y[R.row0 + r] = y[r];
     for (int r = threadIdx.x; r < Q.rows; r += blockDim.x) a.x[Q.row0 + r] = x[r];
-    if (!ok && threadIdx.x == 0) *a.fail = 1.0;
+    if (waits.gave_up) *a.fail = 1.0;
     cluster_sync();
 }
 
