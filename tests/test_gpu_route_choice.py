@@ -1,0 +1,50 @@
+"""Which path a solve takes, seen by the launches it reports, at the edges of the rules that
+choose it; and that products of a mid-size matrix are not slower than a larger one's."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def lp_with_row(instances, m, n, per_col, row_len=0, seed=0):
+    """Uniform columns, and row m // 2 with row_len further entries."""
+    rng = np.random.default_rng(seed)
+    col = np.repeat(np.arange(n), per_col)
+    row = rng.integers(0, m, n * per_col)
+    if row_len:
+        col = np.concatenate([col, rng.choice(n, row_len, replace=False)])
+        row = np.concatenate([row, np.full(row_len, m // 2)])
+    key = np.unique(row.astype(np.int64) * n + col)
+    ptr, idx, val = instances._csr_from_entries(m, key // n, key % n, rng.standard_normal(key.shape[0]))
+    return instances._finish_lp(rng, m, n, ptr, idx, val)
+
+
+def pair_us(engine, A, n, m):
+    """Least time of A x and A'y by turns."""
+    x, y = torch.randn(n, dtype=torch.float64, device="cuda"), torch.randn(m, dtype=torch.float64, device="cuda")
+    x2, y2, L, h = torch.empty_like(x), torch.empty_like(y), engine.lib(), C.byref(A.handle)
+    best = np.inf
+    for _ in range(12):
+        torch.cuda.synchronize()
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        for _ in range(100):
+            assert L.sankhya_cuda_spmv_device_f64(h, x.data_ptr(), y2.data_ptr()) == 0
+            assert L.sankhya_cuda_spmv_transpose_device_f64(h, y.data_ptr(), x2.data_ptr()) == 0
+        t1.record()
+        torch.cuda.synchronize()
+        best = min(best, t0.elapsed_time(t1) * 10)
+    return best
+
+
+def test_products_of_a_mid_size_matrix_are_not_slower_than_a_larger_ones(engine, instances):
+    """Four sizes of 60 to 260 thread blocks a product against one of 340 (they took twice its
+    time when the next product's blocks were let in as each began)."""
+    larger = lp_with_row(instances, 40000, 70000, 10)
+    limit = 1.3 * pair_us(engine, engine.Matrix.from_instance(larger), 70000, 40000)
+    for m, n, per_col in [(8000, 16000, 8), (15000, 30000, 8), (25000, 45000, 8), (30000, 65000, 8)]:
+        inst = lp_with_row(instances, m, n, per_col)
+        assert pair_us(engine, engine.Matrix.from_instance(inst), n, m) < limit, (m, n)

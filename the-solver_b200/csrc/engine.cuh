@@ -295,11 +295,13 @@ __device__ __forceinline__ float load_value<float, __nv_bfloat16>(const __nv_bfl
 // Before a product: what does not depend on the kernel before it in the stream, whose blocks may
 // still be running (launch_early): the first chunk on its way to L2. After the wait that kernel is
 // complete and its writes are visible to ordinary loads, so the gathered vector is read by those
-// and not by the read-only path. A grid of up to kEarlyBlocks lets the next one in at once, since
-// both fit on the chip; a larger one only as its blocks leave (let in at once, the next one's
-// blocks take the places that its own last blocks need: 50,021 x 100,003, A x and A'y, 26.0 us,
-// so 16.2).
-constexpr int kEarlyBlocks = 2 * 148;
+// and not by the read-only path. A grid of up to kEarlyBlocks lets the next one in at once; a
+// larger one only as its blocks leave, since blocks let in at once do not spread over the chip as
+// those of a launch of its own. A x and A'y, us for both, at once / as the blocks leave / launched
+// one after the other: 13 and 20 blocks 6.9 / 6.7 / 10.3 (a restarted QP's iteration there 16.2 /
+// 17.6 / 17.6), 33 and 43 blocks 7.3 / 7.1 / 11.2, 63 10.3 / 7.9 / 12.3, 118 14.3 / 8.3 / 12.3, 157
+// 24.9 / 10.3 / 13.8, 254 26.8 / 11.0 / 14.7.
+constexpr int kEarlyBlocks = 24;
 template <class V>
 __device__ __forceinline__ void start_early(const TileCsrT<V>& A, int t) {
     if (gridDim.x <= kEarlyBlocks) asm volatile("griddepcontrol.launch_dependents;");
