@@ -48,3 +48,45 @@ def test_products_of_a_mid_size_matrix_are_not_slower_than_a_larger_ones(engine,
     for m, n, per_col in [(8000, 16000, 8), (15000, 30000, 8), (25000, 45000, 8), (30000, 65000, 8)]:
         inst = lp_with_row(instances, m, n, per_col)
         assert pair_us(engine, engine.Matrix.from_instance(inst), n, m) < limit, (m, n)
+
+
+def rows_of(instances, m, n, short, longer, share, seed=0):
+    """Rows of `short` entries, a share of them of `longer`."""
+    rng = np.random.default_rng(seed)
+    deg = np.where(rng.random(m) < share, longer, short)
+    key = np.unique(np.repeat(np.arange(m), deg).astype(np.int64) * n + rng.integers(0, n, deg.sum()))
+    ptr, idx, val = instances._csr_from_entries(m, key // n, key % n, rng.standard_normal(key.shape[0]))
+    return instances._finish_lp(rng, m, n, ptr, idx, val)
+
+
+def launches_of(engine, inst, iterations, **kw):
+    A = engine.Matrix.from_instance(inst)
+    engine.set_timing(1)
+    try:
+        rc, *_ = engine.pdhg(A, inst, engine.settings(max_iterations=iterations, check_every=iterations, tau=1e-3, sigma=1e-3,
+                                                      tolerance=1e-300, **kw))
+        assert rc == 0, engine.last_error()
+        return engine.last_timing()["kernel_launches"]
+    finally:
+        engine.set_timing(0)
+
+
+# (cooperative launch or not, instance): where it loses time, the launches stay
+SIZES = {
+    "mid-size": (True, lambda i: lp_with_row(i, 8000, 16000, 8)),
+    "a row of 700": (True, lambda i: lp_with_row(i, 8000, 16000, 8, 700)),
+    "a dense row": (False, lambda i: lp_with_row(i, 20000, 40000, 5, 40000)),
+    "a dense row, 5,000 x 12,000": (False, lambda i: lp_with_row(i, 5000, 12000, 5, 12000)),
+    "one chunk a warp, rows of 45": (True, lambda i: lp_with_row(i, 12000, 27000, 20)),
+    "two chunks a warp, rows of 40": (False, lambda i: rows_of(i, 40000, 60000, 6, 40, 0.4)),
+    "a fifth in rows of 100": (True, lambda i: rows_of(i, 100000, 100000, 8, 100, 0.02)),
+    "most elements": (True, lambda i: lp_with_row(i, 250000, 300000, 4)),
+    "too many elements": (False, lambda i: lp_with_row(i, 300000, 500000, 3)),
+}
+
+
+@pytest.mark.parametrize("name", SIZES)
+def test_cooperative_launch_where_it_pays(engine, instances, name):
+    cooperative, make = SIZES[name]
+    launches = launches_of(engine, make(instances), 60)
+    assert launches < 60 if cooperative else launches >= 120

@@ -59,7 +59,7 @@ std::vector<int> build_tiles(int rows, const int* ptr) {
     return tiles;
 }
 
-Share largest_share(const std::vector<int>& tiles) {
+Share largest_share(const std::vector<int>& tiles, const int* ptr) {
     Share s;
     const int nt = static_cast<int>(tiles.size()) / 2 - 1;
     s.chunks = (nt + cluster::kClusterCtas - 1) / cluster::kClusterCtas;
@@ -68,7 +68,11 @@ Share largest_share(const std::vector<int>& tiles) {
         s.rows = std::max(s.rows, tiles[2 * t1] - tiles[2 * t0]);
         s.nnz = std::max(s.nnz, tiles[2 * t1 + 1] - tiles[2 * t0 + 1]);
     }
-    for (int t = 0; t < nt; ++t) s.long_rows += tiles[2 * t + 3] - tiles[2 * t + 1] > kChunkNnz;
+    for (int r = 0; r < tiles[2 * nt]; ++r) {
+        const int len = ptr[r + 1] - ptr[r];
+        s.longest = std::max(s.longest, len);
+        if (len > kShortRow) s.tree += len;
+    }
     return s;
 }
 
@@ -194,7 +198,7 @@ int make_plan(const SankhyaCudaCSR* m, const int* h_ptr, const int* h_idx, const
     plan->a.val = a_val;
     plan->a.ntiles = static_cast<int>(tiles_a.size()) / 2 - 1;
     plan->a.tile = reinterpret_cast<const int2*>(plan->d_tile_a);
-    plan->a.share = largest_share(tiles_a);
+    plan->a.share = largest_share(tiles_a, h_ptr);
     plan->at.rows = cols;
     plan->at.cols = rows;
     plan->at.nnz = nnz;
@@ -203,7 +207,7 @@ int make_plan(const SankhyaCudaCSR* m, const int* h_ptr, const int* h_idx, const
     plan->at.val = plan->d_at_val;
     plan->at.ntiles = static_cast<int>(tiles_at.size()) / 2 - 1;
     plan->at.tile = reinterpret_cast<const int2*>(plan->d_tile_at);
-    plan->at.share = largest_share(tiles_at);
+    plan->at.share = largest_share(tiles_at, at_ptr.data());
     *out = std::move(plan);
     return 0;
 }

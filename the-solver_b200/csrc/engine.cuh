@@ -56,11 +56,13 @@ int device_transpose(int rows, int cols, int nnz, const int* ptr, const int* idx
 
 // Largest part of a CSR any CTA holds when the chunks of its schedule are split
 // evenly and in order over the CTAs of one cluster (cluster.cuh); chunks 0: unknown.
+// And what the whole matrix's rows are like.
 struct Share {
     int rows = 0, nnz = 0, chunks = 0;
-    int long_rows = 0;   // rows beyond kChunkNnz entries in the whole matrix
+    int longest = 0;   // entries of the longest row
+    int tree = 0;      // entries in rows beyond kShortRow, which a warp sums together
 };
-Share largest_share(const std::vector<int>& tiles);
+Share largest_share(const std::vector<int>& tiles, const int* row_offsets);
 
 // A CSR with its warp-chunk schedule; T is the value type (double, or float
 // for the FP32 inner iterations of the refined PDLP).

@@ -288,9 +288,10 @@ struct Solver {
         cluster_checks = cluster_smem && with_checks <= cluster::kMaxSmem;
         if (cluster_checks) cluster_smem = with_checks;
         flow_ctas = 0;
-        if (!cluster_smem && !Q && flow::flow_pays(*A, *AT)) {
+        if (!cluster_smem && !Q) {
             flow_kernel = sem == Sem::Cuda ? &k_fixed_flow<false> : &k_fixed_flow<true>;
             flow_ctas = flow::resident_ctas(reinterpret_cast<const void*>(flow_kernel), kFlowThreads, 0);
+            if (!flow::flow_pays(*A, *AT, flow_ctas * kFlowWarps)) flow_ctas = 0;
         }
         const bool pair = Q && Q->ntiles;
         if (sem == Sem::Cuda) {
@@ -736,9 +737,9 @@ struct OwnedPair {
         std::vector<int> ta = build_tiles(rows, rp.data());
         if (tiles.alloc_on(s, ta.size() * 4, "cudaMalloc tiles")) return -1;
         B200_TRY(cudaMemcpyAsync(tiles.p, ta.data(), tiles.bytes, cudaMemcpyHostToDevice, s), "upload tiles");
-        a = TileCsr{rows, cols, nnz, static_cast<int>(ta.size()) / 2 - 1, largest_share(ta), ptr.as<int>(),
+        a = TileCsr{rows, cols, nnz, static_cast<int>(ta.size()) / 2 - 1, largest_share(ta, rp.data()), ptr.as<int>(),
                     idx.as<int>(), val.as<double>(), tiles.as<int2>()};
-        at = TileCsr{cols, rows, nnz, static_cast<int>(tb.size()) / 2 - 1, largest_share(tb), tptr.as<int>(),
+        at = TileCsr{cols, rows, nnz, static_cast<int>(tb.size()) / 2 - 1, largest_share(tb, p), tptr.as<int>(),
                      tidx.as<int>(), tval.as<double>(), ttiles.as<int2>()};
         return 0;
     }

@@ -1396,12 +1396,13 @@ struct Core {
             if (ha && ha <= cluster::kMaxSmem && cluster::available(reinterpret_cast<const void*>(halpern_kernel)))
                 halpern_smem = ha;
         }
-        if (!flow::flow_pays(A, AT)) return 0;
         if (!adaptive_smem && one_each)
             adaptive_ctas = flow::resident_ctas(reinterpret_cast<const void*>(&k_adaptive_flow<T, V>), kFlowThreads,
                                                 kFlowSmem + kSumsSmem);
         if (!halpern_smem)
             halpern_ctas = flow::resident_ctas(reinterpret_cast<const void*>(&k_halpern_flow<T, V>), kFlowThreads, kFlowSmem);
+        if (!flow::flow_pays(A, AT, adaptive_ctas * kFlowWarps, true)) adaptive_ctas = 0;
+        if (!flow::flow_pays(A, AT, halpern_ctas * kFlowWarps)) halpern_ctas = 0;
         // a step's chunks in at most kFlowRounds rounds, its blocks in kFlowBlocks slots
         const int blocks = (std::max(A.ntiles, AT.ntiles) + 7) / 8;
         if (blocks > std::min(kFlowBlocks, adaptive_ctas * kFlowGroups * kFlowRounds)) adaptive_ctas = 0;
