@@ -90,3 +90,25 @@ def test_cooperative_launch_where_it_pays(engine, instances, name):
     cooperative, make = SIZES[name]
     launches = launches_of(engine, make(instances), 60)
     assert launches < 60 if cooperative else launches >= 120
+
+
+@pytest.mark.parametrize("m,n,per_col,every,limit,one_launch_a_window", [
+    (2000, 5000, 5, 3, 1e6, False), (2000, 5000, 5, 4, 1e6, True), (2000, 5000, 5, 3, 0.0, True),
+    (130000, 180000, 4, 9, 0.0, False), (130000, 180000, 4, 10, 0.0, True), (100000, 150000, 4, 1, 0.0, True)])
+def test_short_windows_stay_on_the_launches(engine, instances, m, n, per_col, every, limit, one_launch_a_window):
+    """Iterations between checkpoints that the host judges; the same point either way."""
+    inst = lp_with_row(instances, m, n, per_col)
+    A = engine.Matrix.from_instance(inst)
+    got = []
+    for level in (1, 2):
+        engine.set_timing(level)
+        try:
+            rc, x, _, r = engine.pdhg(A, inst, engine.settings(max_iterations=5 * every, check_every=every, tau=1e-3, sigma=1e-3,
+                                                               tolerance=1e-300, time_limit=limit))
+            assert rc == 0, engine.last_error()
+            got.append((x, r, engine.last_timing()["kernel_launches"]))
+        finally:
+            engine.set_timing(0)
+    assert np.array_equal(got[0][0], got[1][0]) and got[0][1] == got[1][1]
+    checks = 5 * 4   # launches of the checkpoints the host judges
+    assert got[0][2] <= checks + 5 if one_launch_a_window else got[0][2] == checks + 2 * 5 * every

@@ -305,6 +305,16 @@ struct Solver {
         dual_blocks = A->ntiles ? grid_dual : 0;
     }
 
+    // A solve whose checkpoints the host judges starts its kernel anew after every `every`
+    // iterations, and few of them do not make up for the start: 12 us more than the launches for
+    // the cluster at 2,000 x 5,000 (it loads the matrices; check_every 1: 50 us from check to
+    // check, so 62; 2: 62 and 62; 5: 81 and 74), 25 to 50 us for the numbered copies of 500,000
+    // rows and columns (1: 108 and 134; 5: 255 and 267; 20: 797 and 753), none below 300,000.
+    void windows_of(int every, double time_limit) {
+        if (cluster_smem && every < 4 && !checks_itself(every, time_limit)) cluster_smem = 0;
+        if (flow_ctas && every < 10 && A->rows + A->cols > 300000) flow_ctas = 0;
+    }
+
     // k iterations as cooperative launches of up to cluster::kMaxSteps.
     int run_flow(int k) {
         if (w->epoch == 0) {
@@ -353,7 +363,7 @@ struct Solver {
     // Whether the solve's checkpoints can be left to the kernel: no time limit to look at
     // between them, no per-kernel timing.
     bool checks_itself(int every, double time_limit) const {
-        return cluster_checks && !(time_limit > 0.0) && every <= cluster::kMaxSteps && timing().level < 2;
+        return cluster_smem && cluster_checks && !(time_limit > 0.0) && every <= cluster::kMaxSteps && timing().level < 2;
     }
     // Up to `steps` iterations with checkpoints, until one is met: iterations run, verdict and
     // maxima in host[0 ..] (Workspace::out and the flags).
@@ -588,6 +598,7 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     sv.sigma = s.sigma;
     sv.theta = s.theta;
     sv.setup_grids();
+    sv.windows_of(s.check_every, s.time_limit);
     const int grid_rows = tiled_grid<CheckRowsCudaEpi>(plan->a);
     const int grid_cols = tiled_grid<CheckColsCudaEpi>(plan->at);
     const int nb_rows = plan->a.ntiles ? grid_rows : 0, nb_cols = plan->at.ntiles ? grid_cols : 0;
