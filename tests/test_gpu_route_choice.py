@@ -112,3 +112,16 @@ def test_short_windows_stay_on_the_launches(engine, instances, m, n, per_col, ev
     assert np.array_equal(got[0][0], got[1][0]) and got[0][1] == got[1][1]
     checks = 5 * 4   # launches of the checkpoints the host judges
     assert got[0][2] <= checks + 5 if one_launch_a_window else got[0][2] == checks + 2 * 5 * every
+
+
+def test_anchored_windows_of_one_iteration_stay_on_the_launches(engine, instances):
+    inst = lp_with_row(instances, 200, 300, 3)
+    A = engine.Matrix.from_instance(inst)
+    launches = []
+    for period in (1, 2):
+        s = engine.pdlp_default_settings()
+        s.max_iterations, s.restart_period, s.algorithm, s.eps_optimal = 20 * period, period, engine.PDLP_HALPERN, 1e-300
+        rc, *_ = engine.pdlp_solve(A, inst, s)
+        assert rc == 0, engine.last_error()
+        launches.append(engine.last_timing()["kernel_launches"])
+    assert launches[0] > launches[1]   # two launches an iteration, then one a window; 20 windows each
