@@ -40,6 +40,10 @@ SANKHYA_CUDA_API void sankhya_b200_last_timing(SankhyaB200Timing* out);
    some seconds. 0 lets every such wait fail. Thread-local. */
 SANKHYA_CUDA_API void sankhya_b200_set_wait_limit(int polls);
 
+/* Solves keep up to 1 GiB per device of the memory they worked in for the next one.
+   This gives back what is idle; destroying the last matrix handle all but 64 MiB. */
+SANKHYA_CUDA_API void sankhya_b200_release_memory(void);
+
 /* --------------------------------------------------- sk_solve continuous hook */
 
 /* Layout-compatible copies of the reference's public model types

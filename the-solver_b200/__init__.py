@@ -39,7 +39,7 @@ EXTENSION_SYMBOLS = (
     "sankhya_b200_gnn_destroy", "sankhya_b200_gnn_parameter_count", "sankhya_b200_gnn_get_parameters",
     "sankhya_b200_gnn_set_parameters", "sankhya_b200_gnn_predict", "sankhya_b200_gnn_gradient",
     "sankhya_b200_gnn_train_step", "sankhya_b200_csr_transpose", "sankhya_b200_polish_default_settings",
-    "sankhya_b200_pdlp_solve_polished", "sankhya_b200_set_wait_limit",
+    "sankhya_b200_pdlp_solve_polished", "sankhya_b200_set_wait_limit", "sankhya_b200_release_memory",
 )
 
 _lib = None
@@ -202,6 +202,8 @@ def _declare(L):
     L.sankhya_b200_set_timing.restype = None
     L.sankhya_b200_set_wait_limit.argtypes = [C.c_int]
     L.sankhya_b200_set_wait_limit.restype = None
+    L.sankhya_b200_release_memory.argtypes = []
+    L.sankhya_b200_release_memory.restype = None
     L.sankhya_b200_last_timing.argtypes = [P(Timing)]
     L.sankhya_b200_last_timing.restype = None
     L.sankhya_b200_pdhg_loop.argtypes = [C.c_void_p, C.c_void_p, dptr, dptr, dptr, P(LoopResult)]
@@ -354,6 +356,10 @@ def set_timing(level: int):
 
 def set_wait_limit(polls: int):
     lib().sankhya_b200_set_wait_limit(int(polls))
+
+
+def release_memory():
+    lib().sankhya_b200_release_memory()
 
 
 def last_timing() -> dict:

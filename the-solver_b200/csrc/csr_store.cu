@@ -144,7 +144,7 @@ Plan::~Plan() {
 
 static int upload(void** dst, const void* src, size_t bytes, const char* what) {
     if (bytes == 0) { *dst = nullptr; return 0; }
-    cudaError_t e = cudaMalloc(dst, bytes);
+    cudaError_t e = device_malloc(dst, bytes);
     if (e != cudaSuccess) { *dst = nullptr; return fail_cuda(what, e); }
     e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail_cuda(what, e);
@@ -164,10 +164,10 @@ int make_plan(const SankhyaCudaCSR* m, const int* h_ptr, const int* h_idx, const
     // A^T) lists its row indices ascending, the order of a counting sort over the
     // rows of A.
     const size_t nnz_alloc = static_cast<size_t>(nnz > 0 ? nnz : 1);
-    B200_TRY(cudaMalloc(reinterpret_cast<void**>(&plan->d_at_ptr), (static_cast<size_t>(cols) + 1) * sizeof(int)),
+    B200_TRY(device_malloc(reinterpret_cast<void**>(&plan->d_at_ptr), (static_cast<size_t>(cols) + 1) * sizeof(int)),
              "cudaMalloc A^T offsets");
-    B200_TRY(cudaMalloc(reinterpret_cast<void**>(&plan->d_at_idx), nnz_alloc * sizeof(int)), "cudaMalloc A^T indices");
-    B200_TRY(cudaMalloc(reinterpret_cast<void**>(&plan->d_at_val), nnz_alloc * sizeof(double)), "cudaMalloc A^T values");
+    B200_TRY(device_malloc(reinterpret_cast<void**>(&plan->d_at_idx), nnz_alloc * sizeof(int)), "cudaMalloc A^T indices");
+    B200_TRY(device_malloc(reinterpret_cast<void**>(&plan->d_at_val), nnz_alloc * sizeof(double)), "cudaMalloc A^T values");
     if (device_transpose(rows, cols, nnz, static_cast<const int*>(m->device_row_offsets),
                          static_cast<const int*>(m->device_column_indices), static_cast<const double*>(m->device_values),
                          plan->d_at_ptr, plan->d_at_idx, plan->d_at_val, nullptr))
@@ -225,15 +225,14 @@ void register_plan(const void* key, std::shared_ptr<Plan> plan) {
     registry()[key] = std::move(plan);
 }
 
-void unregister_plan(const void* key) {
+bool unregister_plan(const void* key) {
     std::shared_ptr<Plan> doomed;
-    {
-        std::lock_guard<std::mutex> lock(g_registry_mutex);
-        auto it = registry().find(key);
-        if (it == registry().end()) return;
-        doomed = std::move(it->second);
-        registry().erase(it);
-    }
+    std::lock_guard<std::mutex> lock(g_registry_mutex);
+    auto it = registry().find(key);
+    if (it == registry().end()) return false;
+    doomed = std::move(it->second);
+    registry().erase(it);
+    return registry().empty();
 }
 
 // The registered plan of m when it describes the same arrays (offsets, indices,
@@ -338,13 +337,29 @@ int grid_for(const void* kernel, int ntiles, int dynamic_smem) {
     return std::max(1, std::min(ntiles, resident));
 }
 
+static std::mutex g_pool_mutex;
+static cudaMemPool_t pools[64] = {};
+
+void trim_pools(unsigned long long keep) {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    for (cudaMemPool_t pool : pools)
+        if (pool) (void)cudaMemPoolTrimTo(pool, keep);
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    (void)cudaGetLastError();
+    cudaDeviceSynchronize();   // frees enqueued by all threads' last calls
+    trim_pools(0);
+    return cudaMalloc(p, bytes);
+}
+
 cudaMemPool_t solve_pool() {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
     static bool asked[64] = {};
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
-    std::lock_guard<std::mutex> lock(mu);
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
     if (!asked[device]) {
         asked[device] = true;
         cudaMemPoolProps props{};
@@ -406,16 +421,27 @@ extern "C" void sankhya_b200_set_timing(int level) { timing().level = level; }
 
 extern "C" void sankhya_b200_set_wait_limit(int polls) { wait_limit_set() = polls; }
 
+extern "C" void sankhya_b200_release_memory(void) {
+    int devices = 0;
+    if (cudaGetDeviceCount(&devices) != cudaSuccess || devices == 0) return;
+    cudaStreamSynchronize(engine_stream());
+    trim_pools(0);
+}
+
 extern "C" void sankhya_b200_last_timing(SankhyaB200Timing* out) {
     if (out) *out = timing().last;
 }
 
 extern "C" void sankhya_cuda_csr_destroy(SankhyaCudaCSR* matrix) {
     if (matrix == nullptr) return;
-    if (matrix->device_row_offsets) unregister_plan(matrix->device_row_offsets);
+    const bool last = matrix->device_row_offsets && unregister_plan(matrix->device_row_offsets);
     cudaFree(matrix->device_row_offsets);
     cudaFree(matrix->device_column_indices);
     cudaFree(matrix->device_values);
+    if (last) {
+        cudaStreamSynchronize(engine_stream());   // or the last call's frees are not seen
+        trim_pools(kPoolRest);
+    }
     matrix->rows = matrix->cols = matrix->nnz = 0;
     matrix->device_row_offsets = nullptr;
     matrix->device_column_indices = nullptr;

@@ -120,7 +120,7 @@ int get_plan(const SankhyaCudaCSR* m, std::shared_ptr<Plan>* out);
 // plan lives on another device than the current one.
 int find_plan(const SankhyaCudaCSR* m, std::shared_ptr<Plan>* out);
 void register_plan(const void* key, std::shared_ptr<Plan> plan);
-void unregister_plan(const void* key);
+bool unregister_plan(const void* key);   // whether it was the last
 
 // ------------------------------------------------------------- streams/timing
 
@@ -507,8 +507,13 @@ inline int elem_grid(int n) {
 
 // Device memory that is kept between solves, at most kPoolBytes of it idle per device: a
 // pool of this library's own with stream-ordered allocation. Null where the device has none.
-constexpr unsigned long long kPoolBytes = 1ull << 30;
+// What is idle goes back when an allocation here would fail otherwise, by
+// sankhya_b200_release_memory, and, but for kPoolRest, with the last matrix handle (all of it would cost
+// a program that makes and drops a handle per small solve 0.5 ms of 1.9 a time).
+constexpr unsigned long long kPoolBytes = 1ull << 30, kPoolRest = 64ull << 20;
 cudaMemPool_t solve_pool();
+void trim_pools(unsigned long long keep);
+cudaError_t device_malloc(void** p, size_t bytes);   // cudaMalloc, once more after trim_pools
 
 // A pinned host slot of kPinnedSlot doubles for small results, one per thread; null when
 // it cannot be had.
@@ -539,7 +544,7 @@ struct DevBuf {
         bytes = b;
         pooled = false;
         if (b == 0) return 0;
-        cudaError_t e = cudaMalloc(&p, b);
+        cudaError_t e = device_malloc(&p, b);
         if (e != cudaSuccess) { p = nullptr; return fail_cuda(what, e); }
         return 0;
     }
