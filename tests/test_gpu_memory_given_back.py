@@ -64,3 +64,16 @@ assert kept >= 64 * MB, kept / MB   # or this shows nothing
 assert before - free() <= 8 * MB, (before - free()) / MB
 solve(A, inst)
 """)
+
+
+def test_a_matrix_holds_no_numbered_copies_on_the_launches():
+    """900,000 rows and columns are beyond the cooperative launch: a fixed-step solve's cached
+    workspace is 16 vectors of 8 bytes, without the 16 bytes more each that the launch numbers."""
+    run("""
+A = E.Matrix.from_instance(inst)
+before = free()
+assert E.pdhg(A, inst, E.settings(max_iterations=5, check_every=5, tau=1e-3, sigma=1e-3, tolerance=1e-300))[0] == 0
+kept = before - free()
+vectors = 8 * (10 * 600000 + 6 * 300000)
+assert vectors <= kept <= vectors + 8 * MB, kept / MB
+""")

@@ -188,7 +188,7 @@ enum class Sem { Cuda, Sk };
 
 // Device state of one solve; one allocation carved into aligned vectors.
 struct Workspace {
-    DevBuf blob;
+    DevBuf blob, numbered;
     double *c = nullptr, *rl = nullptr, *ru = nullptr, *cl = nullptr, *cu = nullptr;
     double *qdiag = nullptr, *tauv = nullptr, *sigv = nullptr;
     double *x[2] = {nullptr, nullptr}, *y[2] = {nullptr, nullptr};
@@ -206,7 +206,7 @@ struct Workspace {
         const size_t nb = (static_cast<size_t>(n) * 8 + 255) / 256 * 256;
         const size_t mb = (static_cast<size_t>(m) * 8 + 255) / 256 * 256;
         const size_t pb = (static_cast<size_t>(max_grid) * 8 * 8 + 255) / 256 * 256;
-        const size_t total = 10 * nb + 6 * mb + 2 * nb + 2 * mb + 3 * pb + 512;
+        const size_t total = 10 * nb + 6 * mb + 3 * pb + 512;
         const char* what = "cudaMalloc PDHG workspace";
         if (on ? blob.alloc_on(*on, total, what) : blob.alloc(total, what)) return -1;
         char* p = blob.as<char>();
@@ -214,11 +214,19 @@ struct Workspace {
         c = take(nb); cl = take(nb); cu = take(nb); qdiag = take(nb); tauv = take(nb);
         x[0] = take(nb); x[1] = take(nb); x_bar = take(nb); qx = take(nb); x_prev = take(nb);
         rl = take(mb); ru = take(mb); sigv = take(mb); y[0] = take(mb); y[1] = take(mb); act = take(mb);
-        xt = reinterpret_cast<flow::Tagged<double>*>(take(2 * nb));
-        yt = reinterpret_cast<flow::Tagged<double>*>(take(2 * mb));
-        epoch = 0;
         part_a = take(pb); part_b = take(pb); part_c = take(pb); out = take(256);
         flags = reinterpret_cast<unsigned int*>(take(256));
+        return 0;
+    }
+    // The numbered copies, 16 bytes a row and column, for a solve that takes the cooperative launch.
+    int allocate_numbered(const cudaStream_t* on) {
+        if (numbered.p) return 0;
+        const size_t xb = (16 * static_cast<size_t>(n) + 255) / 256 * 256, total = xb + 16 * static_cast<size_t>(m);
+        const char* what = "cudaMalloc numbered iterates";
+        if (on ? numbered.alloc_on(*on, total, what) : numbered.alloc(total, what)) return -1;
+        xt = numbered.as<flow::Tagged<double>>();
+        yt = reinterpret_cast<flow::Tagged<double>*>(numbered.as<char>() + xb);
+        epoch = 0;
         return 0;
     }
 };
@@ -535,6 +543,7 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     // The plan's cached workspace and graphs, unless another thread holds them.
     std::unique_lock<std::mutex> lock(plan->workspace_mutex, std::try_to_lock);
     std::shared_ptr<FixedCache> cache;
+    const cudaStream_t* pool_stream = lock.owns_lock() ? nullptr : &stream;
     if (lock.owns_lock()) {
         cache = std::static_pointer_cast<FixedCache>(plan->solve_cache);
         if (!cache || cache->w.n != cols || cache->w.m != rows) {
@@ -545,7 +554,7 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
         }
     } else {
         cache = std::make_shared<FixedCache>();
-        if (cache->w.allocate(cols, rows, sms * 8, &stream)) return -1;
+        if (cache->w.allocate(cols, rows, sms * 8, pool_stream)) return -1;
     }
     Workspace* w = &cache->w;
 
@@ -599,6 +608,7 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     sv.theta = s.theta;
     sv.setup_grids();
     sv.windows_of(s.check_every, s.time_limit);
+    if (sv.flow_ctas && w->allocate_numbered(pool_stream)) return -1;
     const int grid_rows = tiled_grid<CheckRowsCudaEpi>(plan->a);
     const int grid_cols = tiled_grid<CheckColsCudaEpi>(plan->at);
     const int nb_rows = plan->a.ntiles ? grid_rows : 0, nb_cols = plan->at.ntiles ? grid_cols : 0;
@@ -842,6 +852,7 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
     sv.has_qdiag = q && diagonal;
     sv.has_steps = true;
     sv.setup_grids();
+    if (sv.flow_ctas && w.allocate_numbered(&stream)) return -1;
     const int grid_rows = tiled_grid<CheckRowsSkEpi>(ap.a);
     const int grid_cols = tiled_grid<CheckColsSkEpi>(ap.at);
     const int nb_rows = ap.a.ntiles ? grid_rows : 0, nb_cols = ap.at.ntiles ? grid_cols : 0;
