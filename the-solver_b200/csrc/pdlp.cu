@@ -370,9 +370,16 @@ __device__ __forceinline__ T dual_reflected(T y, T axb, T sigma, T rl, T ru) {
     const T v = y + sigma * axb;
     return T(2) * (v - sigma * clampf<T>(v / sigma, rl, ru)) - y;
 }
+// lam reflected + (1 - lam) anchor. The fused form is spelled out, one for either side, as the
+// launches' kernels had been compiled: left to the compiler, the product that goes into the
+// fused sum differed from kernel to kernel, and with it the iterates' last bits.
 template <class T>
-__device__ __forceinline__ T halpern_step(T lam, T reflected, T anchor) {
-    return lam * reflected + (T(1) - lam) * anchor;
+__device__ __forceinline__ T primal_halpern_step(T lam, T reflected, T anchor) {
+    return fma(lam, reflected, dmul(T(1) - lam, anchor));
+}
+template <class T>
+__device__ __forceinline__ T dual_halpern_step(T lam, T reflected, T anchor) {
+    return fma(T(1) - lam, anchor, dmul(lam, reflected));
 }
 
 template <class T>
@@ -391,7 +398,7 @@ struct PrimalHalpernEpi {
         const T xj = x[j];
         const T xr = primal_reflected(xj, aty, tau, c[j], cl[j], cu[j]);
         x_bar[j] = xr;
-        x[j] = halpern_step(halpern_lambda<T>(st, q), xr, x0[j]);
+        x[j] = primal_halpern_step(halpern_lambda<T>(st, q), xr, x0[j]);
     }
     __device__ __forceinline__ void finish(Acc&, double*) const {}
 };
@@ -408,7 +415,7 @@ struct DualHalpernEpi {
     __device__ __forceinline__ void row(int i, T axb, Acc&) const {
         const T sigma = static_cast<T>(st->eta * st->omega);
         const T yr = dual_reflected(y[i], axb, sigma, rl[i], ru[i]);
-        y[i] = halpern_step(halpern_lambda<T>(st, q), yr, y0[i]);
+        y[i] = dual_halpern_step(halpern_lambda<T>(st, q), yr, y0[i]);
     }
     __device__ __forceinline__ void finish(Acc&, double*) const {}
 };

@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
                 const int r = qc.r;
                 const T p = primal_reflected(x[r], aty, tau, c[r], cl[r], cu[r]);
                 xr[r] = p;
-                x[r] = halpern_step(lam, p, x0[r]);
+                x[r] = primal_halpern_step(lam, p, x0[r]);
             }
         }
         exchange(waits, xs_out, xr, xv);
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(cluster::kClusterThreads, 1)
             const T axb = rc.sum(R, xv.v, sp);
             if (rc.owns) {
                 const int r = rc.r;
-                y[r] = halpern_step(lam, dual_reflected(y[r], axb, sigma, rl[r], ru[r]), y0[r]);
+                y[r] = dual_halpern_step(lam, dual_reflected(y[r], axb, sigma, rl[r], ru[r]), y0[r]);
             }
         }
         exchange(waits, ys_out, y, yv);

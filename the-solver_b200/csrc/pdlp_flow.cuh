@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_halpern_flow(const __grid_c
             if (k.owns) {
                 const T p = primal_reflected(x, aty, tau, c, lo, hi);
                 store_tagged(a.xt + j, p, tag);
-                a.x[j] = halpern_step(lam, p, x0);
+                a.x[j] = primal_halpern_step(lam, p, x0);
             }
         }
         for (int t = mine; t < a.A.ntiles; t += nw) {
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_halpern_flow(const __grid_c
             }
             const T axb = chunk_sum(a.A, k, a.xt, tag, sp, &left);
             if (k.owns) {
-                const T yn = halpern_step(lam, dual_reflected(y, axb, sigma, lo, hi), y0);
+                const T yn = dual_halpern_step(lam, dual_reflected(y, axb, sigma, lo, hi), y0);
                 store_tagged(a.yt + i, yn, tag);
                 a.y[i] = yn;
             }
