@@ -9,6 +9,7 @@
 #include "flow.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <unordered_map>
@@ -104,6 +105,24 @@ bool cluster::available(const void* kernel) {
     cache.push_back({kernel, device, ok});
     return ok;
 }
+
+constexpr int kDevices = 64;
+static std::atomic<int> g_in_flight[kDevices];
+static int& in_flight_here(int device) {
+    thread_local int depth[kDevices] = {};
+    return depth[device];
+}
+
+void flow::InFlight::enter() {
+    int device = 0;
+    if (device_ >= 0 || cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kDevices) return;
+    device_ = device;
+    if (in_flight_here(device)++ == 0) ++g_in_flight[device];
+}
+flow::InFlight::~InFlight() {
+    if (device_ >= 0 && --in_flight_here(device_) == 0) --g_in_flight[device_];
+}
+int flow::InFlight::others() const { return device_ < 0 ? 0 : g_in_flight[device_].load() - 1; }
 
 int flow::resident_ctas(const void* kernel, int threads, size_t smem) {
     struct Entry { const void* k; int device, ctas; };

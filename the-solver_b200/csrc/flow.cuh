@@ -215,6 +215,29 @@ inline bool flow_pays(const TileCsrT<V>& A, const TileCsrT<V>& AT, int warps, bo
     return few_long(A) && few_long(AT) && (adaptive ? A.nnz <= 1000000 && elements <= 250000 : A.nnz <= 3000000 && elements <= 600000);
 }
 
+// A cooperative launch takes every SM, so solves of several threads take turns, where the launches
+// fill the chip together. ms for eight solves of 1,000 iterations from as many threads, launches /
+// this: 8,000 x 16,000 16.6 / 34.0, 30,000 x 60,000 46.6 / 56.2; from two 9.4 / 9.0 and 17.0 / 14.5,
+// and with more than a chunk a warp (50,000 x 100,000) 25.2 / 27.4. So a solve that could take it is
+// counted while in flight, and a window goes to the launches when two others are, or one and
+// there is more than a chunk a warp. (Either way gives the same bits.)
+class InFlight {
+public:
+    InFlight() = default;
+    InFlight(const InFlight&) = delete;
+    InFlight& operator=(const InFlight&) = delete;
+    ~InFlight();
+    void enter();   // once per object; counts a thread's nested solves as one
+    template <class V>
+    bool crowded(const TileCsrT<V>& A, const TileCsrT<V>& AT, int warps) const {
+        return others() >= (std::max(A.ntiles, AT.ntiles) <= warps ? 2 : 1);
+    }
+
+private:
+    int others() const;
+    int device_ = -1;
+};
+
 // CTAs of `threads` threads the current device holds at a time with one per SM, 0 where
 // the kernel cannot be launched cooperatively (asked once per kernel and device).
 int resident_ctas(const void* kernel, int threads, size_t smem);

@@ -283,6 +283,7 @@ struct Solver {
     size_t cluster_smem = 0;  // > 0: the iterations run on one cluster
     bool cluster_checks = false;  // and there is room for its own checkpoints
     int flow_ctas = 0;        // > 0: the iterations run as one cooperative launch
+    flow::InFlight in_flight;
     int dual_blocks = 0;      // partials the last dual step left in part_c
 
     void setup_grids() {
@@ -442,7 +443,8 @@ struct Solver {
             return 0;
         }
         if (cluster_smem) return run_cluster(k);
-        if (flow_ctas) return run_flow(k);
+        if (flow_ctas && !in_flight.crowded(*A, *AT, flow_ctas * kFlowWarps)) return run_flow(k);
+        dual_blocks = A->ntiles ? grid_dual : 0;
         while (k > 0) {
             const int chunk = k > 64 ? 64 : k;
             const GraphKey key{stream, Q, has_qdiag ? 1 : 0, has_steps ? 1 : 0, chunk, cur, static_cast<int>(sem),
@@ -608,7 +610,10 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     sv.theta = s.theta;
     sv.setup_grids();
     sv.windows_of(s.check_every, s.time_limit);
-    if (sv.flow_ctas && w->allocate_numbered(pool_stream)) return -1;
+    if (sv.flow_ctas) {
+        sv.in_flight.enter();
+        if (w->allocate_numbered(pool_stream)) return -1;
+    }
     const int grid_rows = tiled_grid<CheckRowsCudaEpi>(plan->a);
     const int grid_cols = tiled_grid<CheckColsCudaEpi>(plan->at);
     const int nb_rows = plan->a.ntiles ? grid_rows : 0, nb_cols = plan->at.ntiles ? grid_cols : 0;
@@ -852,7 +857,10 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
     sv.has_qdiag = q && diagonal;
     sv.has_steps = true;
     sv.setup_grids();
-    if (sv.flow_ctas && w.allocate_numbered(&stream)) return -1;
+    if (sv.flow_ctas) {
+        sv.in_flight.enter();
+        if (w.allocate_numbered(&stream)) return -1;
+    }
     const int grid_rows = tiled_grid<CheckRowsSkEpi>(ap.a);
     const int grid_cols = tiled_grid<CheckColsSkEpi>(ap.at);
     const int nb_rows = ap.a.ntiles ? grid_rows : 0, nb_cols = ap.at.ntiles ? grid_cols : 0;

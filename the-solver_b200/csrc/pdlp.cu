@@ -1304,6 +1304,7 @@ struct Core {
     flow::Tagged<T>*xt = nullptr, *yt = nullptr;
     flow::Tagged<double>* sums = nullptr;
     unsigned* count = nullptr;
+    flow::InFlight in_flight;
     unsigned epoch = 1, arrived = 0;   // iterations numbered, and arrivals counted, so far
     // Quadratic objective (the QP entry point): qmode kQDiag with the diagonal qd,
     // or kQGeneral with the Hessian Q and its diagonal majorant qd, whose products
@@ -1413,7 +1414,9 @@ struct Core {
         // a step's chunks in at most kFlowRounds rounds, its blocks in kFlowBlocks slots
         const int blocks = (std::max(A.ntiles, AT.ntiles) + 7) / 8;
         if (blocks > std::min(kFlowBlocks, adaptive_ctas * kFlowGroups * kFlowRounds)) adaptive_ctas = 0;
-        if (!(adaptive_ctas || halpern_ctas) || flow_blob.p) return 0;
+        if (!(adaptive_ctas || halpern_ctas)) return 0;
+        in_flight.enter();
+        if (flow_blob.p) return 0;
         const size_t xb = cluster::align16(sizeof(flow::Tagged<T>) * n), yb = cluster::align16(sizeof(flow::Tagged<T>) * m);
         const size_t total = xb + yb + 2 * kSumsSmem * 2 + 256;
         if (flow_blob.alloc_on(stream, total, "cudaMalloc numbered iterates")) return -1;
@@ -1544,7 +1547,7 @@ struct Core {
             B200_TRY(cudaGetLastError(), "window launch");
             return 0;
         }
-        if (adaptive && adaptive_ctas) {
+        if (adaptive && adaptive_ctas && !in_flight.crowded(A, AT, adaptive_ctas * kFlowWarps)) {
             for (int done = 0; done < period; done += cluster::kMaxSteps) {
                 const int steps = std::min(period - done, cluster::kMaxSteps);
                 const AdaptiveFlowArgs<T, V> a{A, AT, x, x_cand, x_sum, y, y_cand, y_sum, ax, ax_prev, ax_cand, c, cl, cu,
@@ -1648,7 +1651,7 @@ struct Core {
             B200_TRY(cudaGetLastError(), "window launch");
             return 0;
         }
-        if (halpern_ctas) {
+        if (halpern_ctas && !in_flight.crowded(A, AT, halpern_ctas * kFlowWarps)) {
             for (int done = 0; done < period; done += cluster::kMaxSteps) {
                 const int steps = std::min(period - done, cluster::kMaxSteps);
                 const HalpernFlowArgs<T, V> a{A, AT, x, y, x_restart, y_restart, c, cl, cu, rl, ru, st, res + kFail, xt, yt,
