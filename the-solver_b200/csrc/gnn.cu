@@ -16,11 +16,10 @@
 // the input gradients (K = 16, 64 or 128; N = 64 or 128) on the 5th-generation
 // tensor cores, tcgen05.mma with a TMEM accumulator (tc_gemm.cuh), and so are
 // the weight gradients of the 128-wide layers, which reduce over all nodes in
-// fixed node slices; the 16-wide input layers' weight gradients and any operand
-// that is not 16-byte aligned take mma.sync m16n8k16 kernels. They are HBM-bound
-// streams of the activations, not tensor-throughput-bound. Aggregations are fp32
-// gathers over the stored A and A' (warp per node, 64 channels, entries in stored
-// order). Every reduction
+// fixed node slices; the 16-wide input layers' weight gradients take an mma.sync
+// m16n8k16 kernel. They are HBM-bound streams of the activations, not
+// tensor-throughput-bound. Aggregations are fp32 gathers over the stored A and A'
+// (warp per node, 64 channels, entries in stored order). Every reduction
 // (weight gradients split over K, bias sums, head sums, loss) has a fixed order,
 // so a training run is reproducible bit for bit.
 #include "batch_common.cuh"
@@ -45,30 +44,10 @@ using batch::slot_value;
 constexpr int kH = 64;          // hidden width
 constexpr int kF = 16;          // input features per node
 constexpr int kX = 2 * kH;      // row width of a layer input [H | aggregation]
-constexpr int kGemmThreads = 128;
 constexpr int kRedBlocks = 296; // partial sums per reduction (2 per SM)
 constexpr int kInputSlices = 296; // partial sums of an input layer's gradients (2 per SM)
 
 // ----------------------------------------------------------------- GEMM
-
-template <class TB>
-struct Gemm {
-    int M, N, K;                  // C[M x N] = A[M x K] B[K x N]
-    const float* A;
-    long long sam, sak;           // element (m, k) at A[m sam + k sak]
-    const TB* B;
-    long long sbk, sbn;           // element (k, n) at B[k sbk + n sbn]
-    float* C;
-    long long scm, scn, scz;      // element (m, n) of K-slice z at C[z scz + m scm + n scn]
-    int kchunk;                   // K extent of one grid.z slice
-    const float* bias;            // per output column, or null
-    int relu;
-};
-
-__device__ __forceinline__ __nv_bfloat16 to_bf16(float v) { return __float2bfloat16_rn(v); }
-__device__ __forceinline__ __nv_bfloat16 to_bf16(__nv_bfloat16 v) { return v; }
-
-__device__ __forceinline__ unsigned ld_pair(const __nv_bfloat16* p) { return *reinterpret_cast<const unsigned*>(p); }
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
                                          unsigned b1) {
@@ -77,87 +56,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1
         "{%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// Stages a 64 x 32 tile, element (r, k) = src[(r0 + r) sr + (k0 + k) sk] (zero
-// outside r0 + r < rlim, k0 + k < kend), into dst[r][k] as bf16. When k is the
-// contiguous index, a warp reads 32 consecutive k of one row. Otherwise each
-// thread takes two consecutive k of one row (lanes 0-7: eight consecutive rows,
-// lane bits 3-4: the k pair), so the global reads fill whole sectors and the
-// 4-byte shared stores of a warp fall in 32 different banks (row stride 20 words).
-template <class T>
-__device__ __forceinline__ void stage_tile(__nv_bfloat16 (*dst)[40], const T* src, long long sr, long long sk, int r0,
-                                           int rlim, int k0, int kend) {
-    if (sk == 1) {
-        for (int i = threadIdx.x; i < 64 * 32; i += kGemmThreads) {
-            const int r = i >> 5, k = i & 31;
-            const int gr = r0 + r, gk = k0 + k;
-            dst[r][k] = (gr < rlim && gk < kend) ? to_bf16(src[gr * sr + gk]) : to_bf16(0.f);
-        }
-    } else {
-        for (int q = threadIdx.x; q < 64 * 16; q += kGemmThreads) {
-            const int r = (q & 7) + 8 * ((q >> 5) & 7);
-            const int k = 2 * (((q >> 3) & 3) + 4 * (q >> 8));
-            const int gr = r0 + r, gk = k0 + k;
-            const bool live = gr < rlim;
-            __nv_bfloat162 v;
-            v.x = (live && gk < kend) ? to_bf16(src[gr * sr + gk * sk]) : to_bf16(0.f);
-            v.y = (live && gk + 1 < kend) ? to_bf16(src[gr * sr + (gk + 1) * sk]) : to_bf16(0.f);
-            *reinterpret_cast<__nv_bfloat162*>(&dst[r][k]) = v;
-        }
-    }
-}
-
-// One block = a 64 x 64 tile of C (4 warps x 16 rows, 8 n8 tiles each); K in
-// steps of 32 staged as bf16 in shared memory (A row-major, B transposed so both
-// fragments are pairs of consecutive k).
-template <class TB>
-__global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16(Gemm<TB> g) {
-    __shared__ __align__(16) __nv_bfloat16 As[64][40];
-    __shared__ __align__(16) __nv_bfloat16 Bt[64][40];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
-    const int kb = blockIdx.z * g.kchunk;
-    const int ke = min(g.K, kb + g.kchunk);
-    float acc[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
-    const int g4 = lane >> 2, t4 = lane & 3;
-    for (int k0 = kb; k0 < ke; k0 += 32) {
-        stage_tile(As, g.A, g.sam, g.sak, m0, g.M, k0, ke);
-        stage_tile(Bt, g.B, g.sbn, g.sbk, n0, g.N, k0, ke);
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 32; kk += 16) {
-            const int r = warp * 16 + g4;
-            const unsigned a0 = ld_pair(&As[r][kk + 2 * t4]), a1 = ld_pair(&As[r + 8][kk + 2 * t4]);
-            const unsigned a2 = ld_pair(&As[r][kk + 2 * t4 + 8]), a3 = ld_pair(&As[r + 8][kk + 2 * t4 + 8]);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const unsigned b0 = ld_pair(&Bt[8 * j + g4][kk + 2 * t4]);
-                const unsigned b1 = ld_pair(&Bt[8 * j + g4][kk + 2 * t4 + 8]);
-                mma_bf16(acc[j], a0, a1, a2, a3, b0, b1);
-            }
-        }
-        __syncthreads();
-    }
-    float* C = g.C + blockIdx.z * g.scz;
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int row = m0 + warp * 16 + g4 + 8 * h, col = n0 + 8 * j + 2 * t4 + e;
-                if (row < g.M && col < g.N) {
-                    float v = acc[j][2 * h + e];
-                    if (g.bias) v += g.bias[col];
-                    if (g.relu) v = fmaxf(v, 0.f);
-                    C[row * g.scm + col * g.scn] = v;
-                }
-            }
 }
 
 // out[i] = sum over z of part[z stride + i]. A block covers 64 consecutive
@@ -626,6 +524,8 @@ int elem_blocks(long long count) {
     return static_cast<int>(std::max<long long>(1, std::min<long long>(b, 148LL * 16)));
 }
 
+bool unaligned(const DevBuf& b) { return reinterpret_cast<uintptr_t>(b.p) % 256 != 0; }
+
 int ensure_workspace(SankhyaB200Gnn* g, int m, int n) {
     if (g->m == m && g->n == n) return 0;
     const int R = g->settings.rounds;
@@ -639,6 +539,7 @@ int ensure_workspace(SankhyaB200Gnn* g, int m, int n) {
                             mx + nh + mh + al(4 * part_floats) + 256 + al(sizeof(FeatureSlots));
     g->m = g->n = -1;
     if (g->ws.alloc(static_cast<size_t>(total), "cudaMalloc network workspace")) return -1;
+    if (unaligned(g->ws) || unaligned(g->model)) return fail_msg("network memory is not 256-byte aligned");
     char* p = g->ws.as<char>();
     auto take = [&](long long b) { char* r = p; p += b; return r; };
     g->c = reinterpret_cast<double*>(take(nd));
@@ -675,14 +576,6 @@ int ensure_workspace(SankhyaB200Gnn* g, int m, int n) {
     return 0;
 }
 
-// The tensor-core (tcgen05) GEMM where its layout conditions hold: 16-byte
-// aligned rows of A and C (row strides multiples of 4 floats). One CTA per SM-share
-// of TMEM (512 columns per SM, N per CTA), persistent over the 128-row tiles.
-bool tc_fits(const void* a, int lda, const void* c, int ldc) {
-    return (reinterpret_cast<uintptr_t>(a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(c) & 15u) == 0 &&
-           lda % 4 == 0 && ldc % 4 == 0;
-}
-
 // CTAs per SM of a kernel with this much dynamic shared memory, asked (and the kernel's
 // attribute set) once per kernel and device.
 int resident(const void* fn, int threads, int smem) {
@@ -700,6 +593,9 @@ int resident(const void* fn, int threads, int smem) {
     return cache.back().per_sm;
 }
 
+// The tensor-core (tcgen05) GEMMs, persistent over the 128-row tiles. They read and write rows in
+// 16-byte pieces: every operand starts at a multiple of 128 bytes in an allocation whose start
+// is checked, with rows of 64 or 128 floats (16 for the input features).
 // K = 64 / 128: the cp.async-pipelined kernel, one CTA per SM (its shared memory).
 template <int N, int K, int ST>
 void gemm_tc_pipe(SankhyaB200Gnn* s, cudaStream_t st, int M, const float* A, int lda, const __nv_bfloat16* B, int sbk,
@@ -731,29 +627,16 @@ void gemm_tc(SankhyaB200Gnn* s, cudaStream_t st, int M, const float* A, int lda,
                                                      s->tc_flag.as<unsigned int>());
 }
 
-// C = A B (+ bias, relu) with A fp32 [M x K] (row-major, lda) and B bf16 [K x 64] row-major.
-void gemm_forward(SankhyaB200Gnn* s, cudaStream_t st, int M, int K, const float* A, int lda,
-                  const __nv_bfloat16* W, const float* bias, float* C, int ldc) {
-    if (M == 0) return;
-    if (tc_fits(A, lda, C, ldc) && (K == kF || K == kX)) {
-        if (K == kF) gemm_tc<kH, kF>(s, st, M, A, lda, W, kH, 1, bias, 1, C, ldc);
-        else gemm_tc<kH, kX>(s, st, M, A, lda, W, kH, 1, bias, 1, C, ldc);
-        return;
-    }
-    Gemm<__nv_bfloat16> g{M, kH, K, A, lda, 1, W, kH, 1, C, ldc, 1, 0, K, bias, 1};
-    k_gemm_bf16<__nv_bfloat16><<<dim3((M + 63) / 64, 1, 1), kGemmThreads, 0, st>>>(g);
+// C = relu(A W + bias) with A fp32 [M x K] (row-major, lda) and W bf16 [K x 64] row-major.
+template <int K>
+void gemm_forward(SankhyaB200Gnn* s, cudaStream_t st, int M, const float* A, int lda, const __nv_bfloat16* W,
+                  const float* bias, float* C, int ldc) {
+    if (M > 0) gemm_tc<kH, K>(s, st, M, A, lda, W, kH, 1, bias, 1, C, ldc);
 }
 
-// dX [M x K] = dZ [M x 64] W^T, W bf16 [K x 64] row-major; K = 128.
-void gemm_input_grad(SankhyaB200Gnn* s, cudaStream_t st, int M, const float* dz, const __nv_bfloat16* W, int K,
-                     float* dx, int ldx) {
-    if (M == 0) return;
-    if (tc_fits(dz, kH, dx, ldx) && K == kX && (reinterpret_cast<uintptr_t>(W) & 15u) == 0) {
-        gemm_tc<kX, kH>(s, st, M, dz, kH, W, 1, kH, nullptr, 0, dx, ldx);
-        return;
-    }
-    Gemm<__nv_bfloat16> g{M, K, kH, dz, kH, 1, W, 1, kH, dx, ldx, 1, 0, kH, nullptr, 0};
-    k_gemm_bf16<__nv_bfloat16><<<dim3((M + 63) / 64, (K + 63) / 64, 1), kGemmThreads, 0, st>>>(g);
+// dX [M x 128] = dZ [M x 64] W^T, W bf16 [128 x 64] row-major.
+void gemm_input_grad(SankhyaB200Gnn* s, cudaStream_t st, int M, const float* dz, const __nv_bfloat16* W, float* dx) {
+    if (M > 0) gemm_tc<kX, kH>(s, st, M, dz, kH, W, 1, kH, nullptr, 0, dx, kX);
 }
 
 // Fails the call when a tensor-core GEMM's bounded wait gave up (the flag is cleared).
@@ -831,13 +714,13 @@ int upload_instance(SankhyaB200Gnn* g, const Plan& plan, const double* c, const 
 void forward(SankhyaB200Gnn* g, const Plan& plan, cudaStream_t st) {
     const int m = plan.a.rows, n = plan.a.cols, R = g->settings.rounds;
     const Offsets& o = g->off;
-    gemm_forward(g, st, n, kF, g->fv, kF, g->params_h + o.Ev, g->params + o.bev, g->xv[0], kX);
-    gemm_forward(g, st, m, kF, g->fc, kF, g->params_h + o.Ec, g->params + o.bec, g->xc[0], kX);
+    gemm_forward<kF>(g, st, n, g->fv, kF, g->params_h + o.Ev, g->params + o.bev, g->xv[0], kX);
+    gemm_forward<kF>(g, st, m, g->fc, kF, g->params_h + o.Ec, g->params + o.bec, g->xc[0], kX);
     for (int t = 0; t < R; ++t) {
         spmm(st, plan.a, g->xv[t], kX, nullptr, g->inv_row, g->xc[t] + kH, kX, nullptr, nullptr);
-        gemm_forward(g, st, m, kX, g->xc[t], kX, g->params_h + o.Wc[t], g->params + o.bc[t], g->xc[t + 1], kX);
+        gemm_forward<kX>(g, st, m, g->xc[t], kX, g->params_h + o.Wc[t], g->params + o.bc[t], g->xc[t + 1], kX);
         spmm(st, plan.at, g->xc[t + 1], kX, nullptr, g->inv_col, g->xv[t] + kH, kX, nullptr, nullptr);
-        gemm_forward(g, st, n, kX, g->xv[t], kX, g->params_h + o.Wv[t], g->params + o.bv[t], g->xv[t + 1], kX);
+        gemm_forward<kX>(g, st, n, g->xv[t], kX, g->params_h + o.Wv[t], g->params + o.bv[t], g->xv[t + 1], kX);
     }
 }
 
@@ -873,10 +756,10 @@ void backward(SankhyaB200Gnn* g, const Plan& plan, cudaStream_t st) {
     const Offsets& o = g->off;
     for (int t = R - 1; t >= 0; --t) {
         layer_grads(g, st, n, g->xv[t], g->zv, g->grad + o.Wv[t]);
-        gemm_input_grad(g, st, n, g->zv, g->params_h + o.Wv[t], kX, g->gv, kX);
+        gemm_input_grad(g, st, n, g->zv, g->params_h + o.Wv[t], g->gv);
         spmm(st, plan.a, g->gv + kH, kX, g->inv_col, nullptr, g->zc, kH, g->gc, g->xc[t + 1]);
         layer_grads(g, st, m, g->xc[t], g->zc, g->grad + o.Wc[t]);
-        gemm_input_grad(g, st, m, g->zc, g->params_h + o.Wc[t], kX, g->gc, kX);
+        gemm_input_grad(g, st, m, g->zc, g->params_h + o.Wc[t], g->gc);
         spmm(st, plan.at, g->gc + kH, kX, g->inv_row, nullptr, g->zv, kH, g->gv, g->xv[t]);
     }
     input_grads(g, st, n, g->fv, g->zv, kH, nullptr, g->grad + o.Ev);
