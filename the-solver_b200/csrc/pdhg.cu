@@ -405,7 +405,6 @@ struct Solver {
         else
             launch_tiled(*A, w->x_bar, dual_sk, stream, grid_dual);
         if (ev) cudaEventRecord(ev[1], stream);
-        if (ev) cudaEventRecord(ev[2], stream);
         if (sem == Sem::Cuda) {
             launch_tiled(*AT, w->y[nx],
                          PrimalCudaEpi{w->x[cur], w->c, has_steps ? w->tauv : nullptr, Q ? w->qx : nullptr,
@@ -417,7 +416,7 @@ struct Solver {
                                      w->cl, w->cu, w->x[nx], w->x_bar},
                          stream, grid_primal);
         }
-        if (ev) cudaEventRecord(ev[3], stream);
+        if (ev) cudaEventRecord(ev[2], stream);
         launches += 2;
         cur = nx;
     }
@@ -427,14 +426,14 @@ struct Solver {
     int run(int k) {
         TimingState& ts = timing();
         if (ts.level >= 2) {
-            cudaEvent_t ev[4];
+            cudaEvent_t ev[3];
             for (auto& e : ev) cudaEventCreate(&e);
             for (int i = 0; i < k; ++i) {
                 iterate(ev);
-                cudaEventSynchronize(ev[3]);
+                cudaEventSynchronize(ev[2]);
                 float a = 0, b = 0;
                 cudaEventElapsedTime(&a, ev[0], ev[1]);
-                cudaEventElapsedTime(&b, ev[2], ev[3]);
+                cudaEventElapsedTime(&b, ev[1], ev[2]);
                 ts.last.dual_kernel_ms += a;
                 ts.last.primal_kernel_ms += b;
                 ts.last.per_kernel_samples += 1;
