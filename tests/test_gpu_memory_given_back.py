@@ -77,3 +77,22 @@ kept = before - free()
 vectors = 8 * (10 * 600000 + 6 * 300000)
 assert vectors <= kept <= vectors + 8 * MB, kept / MB
 """)
+
+
+def test_a_handle_may_outlive_the_threads_streams():
+    """The last handle destroyed by another thread than the one that solved, which has ended."""
+    run("""
+import threading
+T.close()
+A = E.Matrix.from_instance(inst)
+t = threading.Thread(target=solve, args=(A, inst))
+t.start()
+t.join()
+t = threading.Thread(target=A.close)
+t.start()
+t.join()
+A = E.Matrix.from_instance(tiny)
+solve(A, tiny)
+import atexit
+atexit.register(A.close)
+""")

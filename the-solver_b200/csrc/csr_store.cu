@@ -316,10 +316,22 @@ int get_plan(const SankhyaCudaCSR* m, std::shared_ptr<Plan>* out) {
 
 // ------------------------------------------------------------ stream, grid
 
+// The engine's streams of this thread while they live: a handle may be destroyed after them, at
+// the end of the program.
+static thread_local cudaStream_t* g_thread_streams = nullptr;
+
+static void sync_engine_stream() {
+    int device = 0;
+    if (g_thread_streams && cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < 64 && g_thread_streams[device])
+        cudaStreamSynchronize(g_thread_streams[device]);
+}
+
 cudaStream_t engine_stream() {
     struct PerThread {
         cudaStream_t streams[64] = {};
+        PerThread() { g_thread_streams = streams; }
         ~PerThread() {
+            g_thread_streams = nullptr;
             for (cudaStream_t s : streams)
                 if (s) cudaStreamDestroy(s);
         }
@@ -443,7 +455,7 @@ extern "C" void sankhya_b200_set_wait_limit(int polls) { wait_limit_set() = poll
 extern "C" void sankhya_b200_release_memory(void) {
     int devices = 0;
     if (cudaGetDeviceCount(&devices) != cudaSuccess || devices == 0) return;
-    cudaStreamSynchronize(engine_stream());
+    sync_engine_stream();
     trim_pools(0);
 }
 
@@ -458,7 +470,7 @@ extern "C" void sankhya_cuda_csr_destroy(SankhyaCudaCSR* matrix) {
     cudaFree(matrix->device_column_indices);
     cudaFree(matrix->device_values);
     if (last) {
-        cudaStreamSynchronize(engine_stream());   // or the last call's frees are not seen
+        sync_engine_stream();   // or the last call's frees are not seen
         trim_pools(kPoolRest);
     }
     matrix->rows = matrix->cols = matrix->nnz = 0;
