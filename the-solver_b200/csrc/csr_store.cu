@@ -381,7 +381,7 @@ cudaError_t device_malloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
     (void)cudaGetLastError();
-    cudaDeviceSynchronize();   // frees enqueued by all threads' last calls
+    sync_engine_stream();   // frees of this thread's last call
     trim_pools(0);
     return cudaMalloc(p, bytes);
 }
