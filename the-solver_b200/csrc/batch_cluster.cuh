@@ -6,8 +6,8 @@
 // and SM and reads the matrix from HBM; 512 LPs of 50 to 5,000 rows (6.6M nonzeros) 98.0 us
 // with its share of the checks, here 57.6 (148 LPs of 60,000 nonzeros 161 -> 69, 296 of 6,000
 // 26 -> 17). It is bound by the shared-memory wavefronts of the gathers and of the row sums,
-// whose order is fixed (76 % of the pipe with the copies by cp.async, which took 30 % of them;
-// the copy engine's take none), then by the chain of a chunk: 24 warps hide it best (640
+// whose order is fixed (the L1 data pipe is 62 % busy, shared memory 54 %; 74 % with the copies by
+// cp.async, whose wavefronts the copy engine saves), then by the chain of a chunk: 24 warps hide it best (640
 // threads 60.1, 896 59.2; two chunks in flight a warp needs registers that 24 warps do not
 // have: 16 warps 76.6).
 #pragma once

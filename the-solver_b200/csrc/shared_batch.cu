@@ -21,7 +21,8 @@
 // 20.0; 256 of 300 x 600 11.4 -> 10.5. The larger share came from instructions (the shuffles
 // that handed out a row's entries, under tests of whether each exists, were three quarters
 // of them), the rest from the boxes and the in-place update, which keep the working set
-// (50 MB at 256 nodes) in L2. 24 to 32 warps per SM at half of the issue slots remain.
+// (50 MB at 256 nodes) in L2. The latency of the gathers remains: 24 warps an SM at 44 % of the
+// issue slots, L1 38 to 50 % and L2 22 to 26 % busy.
 #include "batch_common.cuh"
 
 #include <algorithm>
