@@ -59,6 +59,12 @@ def rows_of(instances, m, n, short, longer, share, seed=0):
     return instances._finish_lp(rng, m, n, ptr, idx, val)
 
 
+def transposed(instances, inst):
+    rows = np.repeat(np.arange(inst["m"]), np.diff(inst["ptr"]))
+    ptr, idx, val = instances._csr_from_entries(inst["n"], inst["idx"], rows, inst["val"])
+    return instances._finish_lp(np.random.default_rng(0), inst["n"], inst["m"], ptr, idx, val)
+
+
 def launches_of(engine, inst, iterations, **kw):
     A = engine.Matrix.from_instance(inst)
     engine.set_timing(1)
@@ -82,6 +88,13 @@ SIZES = {
     "a fifth in rows of 100": (True, lambda i: rows_of(i, 100000, 100000, 8, 100, 0.02)),
     "most elements": (True, lambda i: lp_with_row(i, 250000, 300000, 4)),
     "too many elements": (False, lambda i: lp_with_row(i, 300000, 500000, 3)),
+    "wide, 120 a row": (True, lambda i: lp_with_row(i, 800, 24000, 4)),
+    "wide, 400 a row": (False, lambda i: lp_with_row(i, 800, 80000, 4)),
+    "wide, 250 a row": (False, lambda i: lp_with_row(i, 1200, 75000, 4)),
+    "tall, 180 a column": (False, lambda i: transposed(i, lp_with_row(i, 2000, 90000, 4))),
+    "a quarter in rows of 400": (True, lambda i: rows_of(i, 20000, 30000, 10, 400, 0.007)),
+    "half in rows of 400": (False, lambda i: rows_of(i, 20000, 30000, 6, 400, 0.018)),
+    "a fifth in rows beyond 32, many elements": (False, lambda i: rows_of(i, 150000, 200000, 6, 40, 0.05)),
 }
 
 

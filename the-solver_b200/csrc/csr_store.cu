@@ -73,6 +73,7 @@ Share largest_share(const std::vector<int>& tiles, const int* ptr) {
         const int len = ptr[r + 1] - ptr[r];
         s.longest = std::max(s.longest, len);
         if (len > kShortRow) s.tree += len;
+        if (len > kChunkNnz) s.streamed += len;
     }
     return s;
 }

@@ -61,6 +61,7 @@ struct Share {
     int rows = 0, nnz = 0, chunks = 0;
     int longest = 0;   // entries of the longest row
     int tree = 0;      // entries in rows beyond kShortRow, which a warp sums together
+    int streamed = 0;  // of these, in rows beyond kChunkNnz
 };
 Share largest_share(const std::vector<int>& tiles, const int* row_offsets);
 

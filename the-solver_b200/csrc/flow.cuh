@@ -194,24 +194,29 @@ __device__ __forceinline__ T chunk_sum(const TileCsrT<V>& A, const ChunkRows& c,
 //   27,000 (540,000; rows of 45) 12.7 -> 8.7, 16.4 -> 13.1, 19.7 -> 15.4. A row beyond a chunk
 //   is waited for 64 entries at a time: 15,000 x 30,000 with a row of 700 9.6 -> 8.9, 13.0 -> 10.0,
 //   17.8 -> 14.1, with one of 1,000 11.3 -> 11.4 (fixed step), and a row of 40,000 in 20,000 x 40,000
-//   207 -> 430.
+//   207 -> 430; 20,000 x 30,000 with a quarter of the entries in rows of 400 9.0 -> 7.3, half 8.9 -> 9.8.
+// - With a vector of few elements every one has many readers, and the lines of those that come
+//   early go back and forth. Nonzeros per row (or per column): 120 (800 x 24,000) 7.9 -> 5.9, 180 (2,000 x
+//   90,000) 9.5 -> 10.2, 250 (1,200 x 75,000) 8.8 -> 13.4, 400 (800 x 80,000) 9.8 -> 25.7; transposed alike.
 // - With more chunks a warp takes them one after the other, and 16 warps an SM do not hide the
 //   sums of rows beyond kShortRow (a tree per row) as the launches' 64 do: 40,000 x 60,000 with
 //   four fifths of A's entries in rows of 40 (776,000) 15.5 -> 22.2; a fifth in rows of 100, 100,000 x
-//   100,000 (979,000) 17.2 -> 14.7.
+//   100,000 (979,000) 17.2 -> 14.7. With more elements fewer of them: a quarter at 100,000 x 466,000
+//   (2.8M) 39.2 -> 43.3, a fifteenth at 120,000 x 240,000 (2.9M) 38.4 -> 35.6.
 // - Every launch writes the numbered copy anew, and its 16 bytes an element no longer stay near:
 //   250,000 x 300,000 (1.2M) 19.0 -> 18.1, 223,000 x 487,000 (1M) 18.4 -> 20.2, 496,000 x 329,000 (1.3M)
 //   21.9 -> 29.2.
 // - The adaptive loop's sums cost it more: 48,000 x 59,000 (885,000) 0.94 of the launches, from
 //   1.2M or 330,000 rows and columns on 0.96 to 1.04.
-constexpr int kLongest = 768;
+constexpr int kLongest = 768, kReaders = 150;
 template <class V>
 inline bool flow_pays(const TileCsrT<V>& A, const TileCsrT<V>& AT, int warps, bool adaptive = false) {
     if (A.ntiles == 0 || AT.ntiles == 0) return false;
     if (std::max(A.share.longest, AT.share.longest) > (A.nnz <= 400000 ? kLongest : kChunkNnz)) return false;
+    if (std::max(A.share.streamed, AT.share.streamed) > A.nnz / 3 || A.nnz / kReaders > std::min(A.rows, A.cols)) return false;
     if (std::max(A.ntiles, AT.ntiles) <= warps) return true;
-    auto few_long = [&](const TileCsrT<V>& M) { return M.ntiles <= warps || M.share.tree <= M.nnz / 4; };
-    const int elements = A.rows + A.cols;
+    const int elements = A.rows + A.cols, part = elements <= 300000 ? 4 : 10;
+    auto few_long = [&](const TileCsrT<V>& M) { return M.ntiles <= warps || M.share.tree <= M.nnz / part; };
     return few_long(A) && few_long(AT) && (adaptive ? A.nnz <= 1000000 && elements <= 250000 : A.nnz <= 3000000 && elements <= 600000);
 }
 
