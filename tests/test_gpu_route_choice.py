@@ -127,6 +127,19 @@ def test_short_windows_stay_on_the_launches(engine, instances, m, n, per_col, ev
     assert got[0][2] <= checks + 5 if one_launch_a_window else got[0][2] == checks + 2 * 5 * every
 
 
+def test_a_solve_of_few_iterations_is_a_short_window(engine, instances):
+    inst = lp_with_row(instances, 2000, 5000, 5)
+    A = engine.Matrix.from_instance(inst)
+    engine.set_timing(1)
+    try:
+        for iterations, launches in ((3, 6), (4, 1)):
+            rc, *_ = engine.pdhg(A, inst, engine.settings(max_iterations=iterations, check_every=100, tau=1e-3, sigma=1e-3,
+                                                          tolerance=1e-300, time_limit=1e6))
+            assert rc == 0 and engine.last_timing()["kernel_launches"] == launches + 4
+    finally:
+        engine.set_timing(0)
+
+
 def test_anchored_windows_of_one_iteration_stay_on_the_launches(engine, instances):
     inst = lp_with_row(instances, 200, 300, 3)
     A = engine.Matrix.from_instance(inst)

@@ -608,7 +608,7 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     sv.sigma = s.sigma;
     sv.theta = s.theta;
     sv.setup_grids();
-    sv.windows_of(s.check_every, s.time_limit);
+    sv.windows_of(std::min(s.check_every, s.max_iterations), s.time_limit);
     if (sv.flow_ctas) {
         sv.in_flight.enter();
         if (w->allocate_numbered(pool_stream)) return -1;
