@@ -46,7 +46,10 @@ using batch::slot_value;
 // Gathers a warp has in flight for one row (times 64 LPs). Every depth sums each LP in
 // stored order, so all give the same bits; the fastest for a (matrix, batch width) is
 // picked by timing (schedule 0) or fixed by the caller (schedule 1..3).
-constexpr int kAhead[3] = {3, 4, 6};
+// The first is the deepest, as it has always been: a row with most of the columns is a chain of gathers,
+// and a caller who has fixed it for one gets it (31 LPs, a row of 4,000, us per iteration: depths
+// 6, 4, 3 410, 590, 454).
+constexpr int kAhead[3] = {6, 4, 3};
 
 // The epilogues work on two LPs, k and k + 1 (k even), of one row or column: load reads
 // what they need (before the gathers), store finishes the step with the row sums.
