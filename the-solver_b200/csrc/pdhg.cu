@@ -199,14 +199,15 @@ struct Workspace {
     unsigned int* flags = nullptr;  // right behind `out`: [0] input checks, [1] a cluster wait gave up
     int n = 0, m = 0;
 
-    // From the solve pool on *on, or (null) for longer than a call.
-    int allocate(int n_, int m_, int max_grid, const cudaStream_t* on) {
+    // From the solve pool on *on, or (null) for longer than a call; with_numbered: the numbered copies in
+    // the same allocation (one of its own took 0.3 ms more on a matrix's first solve).
+    int allocate(int n_, int m_, int max_grid, const cudaStream_t* on, bool with_numbered = false) {
         n = n_;
         m = m_;
         const size_t nb = (static_cast<size_t>(n) * 8 + 255) / 256 * 256;
         const size_t mb = (static_cast<size_t>(m) * 8 + 255) / 256 * 256;
         const size_t pb = (static_cast<size_t>(max_grid) * 8 * 8 + 255) / 256 * 256;
-        const size_t total = 10 * nb + 6 * mb + 3 * pb + 512;
+        const size_t total = 10 * nb + 6 * mb + 3 * pb + 512 + (with_numbered ? 2 * (nb + mb) : 0);
         const char* what = "cudaMalloc PDHG workspace";
         if (on ? blob.alloc_on(*on, total, what) : blob.alloc(total, what)) return -1;
         char* p = blob.as<char>();
@@ -216,11 +217,15 @@ struct Workspace {
         rl = take(mb); ru = take(mb); sigv = take(mb); y[0] = take(mb); y[1] = take(mb); act = take(mb);
         part_a = take(pb); part_b = take(pb); part_c = take(pb); out = take(256);
         flags = reinterpret_cast<unsigned int*>(take(256));
+        if (with_numbered) {
+            xt = reinterpret_cast<flow::Tagged<double>*>(take(2 * nb));
+            yt = reinterpret_cast<flow::Tagged<double>*>(take(2 * mb));
+        }
         return 0;
     }
     // The numbered copies, 16 bytes a row and column, for a solve that takes the cooperative launch.
     int allocate_numbered(const cudaStream_t* on) {
-        if (numbered.p) return 0;
+        if (xt) return 0;
         const size_t xb = (16 * static_cast<size_t>(n) + 255) / 256 * 256, total = xb + 16 * static_cast<size_t>(m);
         const char* what = "cudaMalloc numbered iterates";
         if (on ? numbered.alloc_on(*on, total, what) : numbered.alloc(total, what)) return -1;
@@ -541,6 +546,15 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, plan->device);
 
+    Solver sv;
+    sv.sem = Sem::Cuda;
+    sv.stream = stream;
+    sv.A = &plan->a;
+    sv.AT = &plan->at;
+    sv.Q = qplan ? &qplan->a : nullptr;
+    sv.setup_grids();
+    sv.windows_of(std::min(s.check_every, s.max_iterations), s.time_limit);
+
     // The plan's cached workspace and graphs, unless another thread holds them.
     std::unique_lock<std::mutex> lock(plan->workspace_mutex, std::try_to_lock);
     std::shared_ptr<FixedCache> cache;
@@ -550,12 +564,12 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
         if (!cache || cache->w.n != cols || cache->w.m != rows) {
             plan->solve_cache.reset();
             cache = std::make_shared<FixedCache>();
-            if (cache->w.allocate(cols, rows, sms * 8, nullptr)) return -1;
+            if (cache->w.allocate(cols, rows, sms * 8, nullptr, sv.flow_ctas > 0)) return -1;
             plan->solve_cache = cache;
         }
     } else {
         cache = std::make_shared<FixedCache>();
-        if (cache->w.allocate(cols, rows, sms * 8, pool_stream)) return -1;
+        if (cache->w.allocate(cols, rows, sms * 8, pool_stream, sv.flow_ctas > 0)) return -1;
     }
     Workspace* w = &cache->w;
 
@@ -593,12 +607,6 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     }
     ts.last.h2d_ms = t_h2d.stop();
 
-    Solver sv;
-    sv.sem = Sem::Cuda;
-    sv.stream = stream;
-    sv.A = &plan->a;
-    sv.AT = &plan->at;
-    sv.Q = qplan ? &qplan->a : nullptr;
     sv.w = w;
     // graphs over an explicit Hessian bake in that matrix's pointers: keep them per call
     sv.graphs = hessian == nullptr ? &cache->graphs : &sv.local_graphs;
@@ -607,8 +615,6 @@ static int solve_fixed(const SankhyaCudaCSR* matrix, const SankhyaCudaCSR* hessi
     sv.tau = s.tau;
     sv.sigma = s.sigma;
     sv.theta = s.theta;
-    sv.setup_grids();
-    sv.windows_of(std::min(s.check_every, s.max_iterations), s.time_limit);
     if (sv.flow_ctas) {
         sv.in_flight.enter();
         if (w->allocate_numbered(pool_stream)) return -1;
@@ -827,7 +833,7 @@ static int sk_loop(const sk_model* m, const sk_options* o, double* x, double* y,
     const bool explicit_q = q && !diagonal;
     if (explicit_q && qp.upload_csc(n, n, q->p, q->i, q->x, stream)) return -1;
     Workspace w;
-    if (w.allocate(n, r, sms * 8, &stream)) return -1;
+    if (w.allocate(n, r, sms * 8, &stream)) return -1;   // from the pool: the numbered copies cost nothing more apart
     const size_t nb = sizeof(double) * static_cast<size_t>(n), mb = sizeof(double) * static_cast<size_t>(r);
     if (n) {
         B200_TRY(cudaMemcpyAsync(w.c, m->c, nb, cudaMemcpyHostToDevice, stream), "upload c");
