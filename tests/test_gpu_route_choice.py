@@ -151,3 +151,19 @@ def test_anchored_windows_of_one_iteration_stay_on_the_launches(engine, instance
         assert rc == 0, engine.last_error()
         launches.append(engine.last_timing()["kernel_launches"])
     assert launches[0] > launches[1]   # two launches an iteration, then one a window; 20 windows each
+
+
+@pytest.mark.parametrize("count,m,every,on_ctas", [(512, 30, 20, False), (512, 30, 100, False), (40, 60, 20, True),
+                                                   (300, 60, 20, True), (300, 250, 20, True), (296, 500, 20, True)])
+def test_batches_of_small_lps(engine, instances, count, m, every, on_ctas):
+    """Several tiny LPs a CTA take longer than two launches over all of them."""
+    lps = [lp_with_row(instances, m, 2 * m, 4, seed=k) for k in range(count)]
+    blk, rseg, cseg = engine.block_diagonal(lps)
+    s = engine.batch_default_settings()
+    s.max_iterations, s.check_every, s.primal_tol, s.dual_tol = 100, every, 1e-300, 1e-300
+    engine.set_timing(1)
+    try:
+        rc, *_ = engine.batch_pdhg(engine.Matrix.from_instance(blk), blk, rseg, cseg, s)
+        assert rc == 0 and (engine.last_timing()["kernel_launches"] < 100) == on_ctas
+    finally:
+        engine.set_timing(0)

@@ -223,16 +223,20 @@ struct BatchPlan {
 
 // Rule: the shorter time of an iteration by what was measured on a B200 (us; z: an LP's
 // nonzeros, or 4 per row and column if those are more, in thousands):
-//   a single CTA     1.8 + 1.1 z      (2.9 at 0.6, 8.5 at 6, 29 at 24, 69 at 60)
+//   a single CTA     1.8 + 1.1 z, 3 at least (3.0 at 0.4, 2.9 at 0.6, 8.5 at 6, 29 at 24, 69 at 60)
 //   2 or 4 CTAs      4.5 + 1.1 z / n  (four: 8.3 at 6, 10.9 at 24, 22.5 at 60)
-//   the launches     9.7, or 2 + 0.0155 z of the whole batch when longer (checks included)
+//   the launches     8.2 + 0.004 z of the whole batch, or 0.9 + 0.0139 z when longer, and 22 + 0.032 z a
+//                    check; 2 + 0.0155 z at least
+// those of CTAs with a check every 20 iterations, which is 0.8 of an iteration to them (512 LPs
+// of 5 to 34 rows: launches 9.1 checked every 20, 8.8 every 100; CTAs, which the model without the least
+// of 3 took, 10.7 and 10.2; 160 of 500 to 1,000 checked every 5: 26.1 and 14.3)
 // and the largest LPs, longer than 0.85 of a CTA's even share, by whole clusters: 512 LPs of 50
 // to 5,000 rows 63.3 by single CTAs, 57.6 with the largest by pairs, 98.0 on the launches;
 // 296 of 500 rows 16.8, on the launches 26.3. Batches of a few LPs, where single CTAs leave the
 // others idle, stay on the launches, as does one with an LP too large for a CTA's shared memory
 // (some 19,000 rows and columns).
 BatchPlan plan_batch(const TileCsr& A, const TileCsr& AT, int batch, const int* row_seg, const int* col_seg,
-                     const std::vector<int>& entries) {
+                     const std::vector<int>& entries, int every) {
     BatchPlan p;
     int rows_max = 0, cols_max = 0;
     for (int k = 0; k < batch; ++k) {
@@ -251,12 +255,14 @@ BatchPlan plan_batch(const TileCsr& A, const TileCsr& AT, int batch, const int* 
     };
     std::stable_sort(p.order.begin(), p.order.end(), [&](int a, int b) { return size(a) > size(b); });
     const double total = A.nnz / 1000.0;
-    auto alone = [&](int at) { return 1.8 + 1.1e-3 * size(p.order[at]); };
+    auto alone = [&](int at) { return std::max(3.0, 1.8 + 1.1e-3 * size(p.order[at])); };
     double sum = 0.0;
     for (int k = 0; k < batch; ++k) sum += alone(k);
     int large = 0;
     while (large < batch && alone(large) > 0.85 * sum / slots) ++large;
-    double best = std::max(9.7, 2.0 + 0.0155 * total) / 1.1;   // so that a near tie stays where it was
+    const double check = (22.0 + 0.032 * total) / every;
+    const double launches = std::max({8.2 + 0.004 * total + check, 0.9 + 0.0139 * total + check, 2.0 + 0.0155 * total});
+    double best = launches / 1.1 / ((1.0 + 0.8 / every) / 1.04);   // / 1.1: a near tie stays where it was
     for (int n : {1, 2, 4}) {
         const int by_clusters = n > 1 ? large : 0;
         if (batch_clusters(n) == 0) continue;
@@ -406,7 +412,7 @@ extern "C" int sankhya_b200_batch_pdhg(const SankhyaCudaCSR* matrix, int batch, 
     B200_TRY(cudaStreamSynchronize(stream), "batch setup");
     if (host_counters[1]) return fail_msg("matrix is not block-diagonal over the given segments");
 
-    const BatchPlan way = plan_batch(A, AT, batch, row_segments, col_segments, entries);
+    const BatchPlan way = plan_batch(A, AT, batch, row_segments, col_segments, entries, s.check_every);
     const int ctas = way.ctas;
     if (ctas) B200_TRY(cudaMemcpyAsync(d_order, way.order.data(), sizeof(int) * way.order.size(), cudaMemcpyHostToDevice, stream),
                        "upload order");
