@@ -624,7 +624,9 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
     } graphs_guard{&graphs};
     int cur = 0, it = 0, launches = 0;
     // In place, so that x, x_bar and y (50 MB at 256 LPs of 5,000 x 10,000) stay in L2; only
-    // the iteration before a check keeps the y it started from.
+    // the iteration before a check keeps the y it started from, and the one before that writes
+    // to the other buffer too, so that every window starts with the same one: a second graph,
+    // for the windows between, took 0.1 ms of a call to capture.
     auto iterate = [&](bool keep) {
         const int nx = keep ? cur ^ 1 : cur;
         launch_multi(shape, m, bpi, A, xbar, MultiDualEpi{yb[cur], drl, dru, sig, done, yb[nx], bpi,
@@ -649,7 +651,7 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
                 const int saved = cur;
                 cudaGraph_t graph;
                 B200_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-                for (int i = 0; i < chunk; ++i) iterate(last && i + 1 == chunk);
+                for (int i = 0; i < chunk; ++i) iterate(last && i + 2 >= chunk);
                 B200_TRY(cudaStreamEndCapture(stream, &graph), "end capture");
                 cudaGraphExec_t exec;
                 cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
@@ -660,7 +662,7 @@ extern "C" int sankhya_b200_shared_batch_pdhg(const SankhyaCudaCSR* matrix, int 
             }
             B200_TRY(cudaGraphLaunch(g->second, stream), "graph launch");
             launches += (m ? 2 : 1) * chunk;
-            if (last) cur ^= 1;
+            if (last && chunk == 1) cur ^= 1;
             k -= chunk;
         }
         it = next;
