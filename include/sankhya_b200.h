@@ -327,7 +327,7 @@ typedef struct SankhyaB200BatchSettings {
     int check_every;     /* 20, as in sk_solve                               */
     int schedule;        /* shared-matrix batch only: 0 = gather depth picked by timing
                             (cached per matrix and batch width), 1..3 = fixed depth
-                            (6, 4, 3 row entries in flight); results do not
+                            (6, 4, 3 row entries in flight; 1: 8 up to 64 LPs); results do not
                             depend on it                                      */
     double primal_tol;   /* 1e-7 */
     double dual_tol;     /* 1e-7 */

@@ -48,8 +48,10 @@ using batch::slot_value;
 // picked by timing (schedule 0) or fixed by the caller (schedule 1..3).
 // The first is the deepest, as it has always been: a row with most of the columns is a chain of gathers,
 // and a caller who has fixed it for one gets it (31 LPs, a row of 4,000, us per iteration: depths
-// 6, 4, 3 410, 590, 454).
+// 6, 4, 3 387, 558, 431). Up to 64 LPs are one group, whose rows are too few warps for their registers to
+// matter, and the first is 8 deep: 235 there, 29 where a power-law matrix of 563 x 248 took 48.
 constexpr int kAhead[3] = {6, 4, 3};
+constexpr int kFewLps = 64, kAheadFew = 8;
 
 // The epilogues work on two LPs, k and k + 1 (k even), of one row or column: load reads
 // what they need (before the gathers), store finishes the step with the row sums.
@@ -146,7 +148,7 @@ struct MultiStoreEpi {
 // entry exists took three times the instructions.
 // Off: unsigned while an element's offset fits 32 bits.
 template <class Epi, int AH, class Off>
-__global__ void __launch_bounds__(kThreads, AH <= 4 ? 4 : 3) k_multi(int rows, int groups, int bp,
+__global__ void __launch_bounds__(kThreads, AH <= 4 ? 4 : AH <= 6 ? 3 : 2) k_multi(int rows, int groups, int bp,
                                                                       const int* __restrict__ ptr,
                                                                       const int* __restrict__ idx,
                                                                       const double* __restrict__ val,
@@ -429,7 +431,10 @@ void launch_multi(int shape, int rows, int bp, const TileCsr& M, const double* v
         return;
     }
     switch (shape) {
-        case 0: launch_ahead<Epi, kAhead[0], unsigned>(rows, bp, M, v, epi, st); break;
+        case 0:
+            if (bp <= kFewLps) launch_ahead<Epi, kAheadFew, unsigned>(rows, bp, M, v, epi, st);
+            else launch_ahead<Epi, kAhead[0], unsigned>(rows, bp, M, v, epi, st);
+            break;
         case 1: launch_ahead<Epi, kAhead[1], unsigned>(rows, bp, M, v, epi, st); break;
         default: launch_ahead<Epi, kAhead[2], unsigned>(rows, bp, M, v, epi, st); break;
     }
