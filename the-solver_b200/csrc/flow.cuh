@@ -203,6 +203,11 @@ __device__ __forceinline__ T chunk_sum(const TileCsrT<V>& A, const ChunkRows& c,
 //   four fifths of A's entries in rows of 40 (776,000) 15.5 -> 22.2; a fifth in rows of 100, 100,000 x
 //   100,000 (979,000) 17.2 -> 14.7. With more elements fewer of them: a quarter at 100,000 x 466,000
 //   (2.8M) 39.2 -> 43.3, a fifteenth at 120,000 x 240,000 (2.9M) 38.4 -> 35.6.
+// - Where only one matrix has more chunks than warps, they are mostly of light rows, 32 to a chunk, and while the other
+//   has no long rows the sums stay hidden: columns of up to 82 with 0.63 of the entries, 50,000 x 80,000
+//   (443,000) 12.0 -> 9.5, 14.1 -> 11.5, 19.6 -> 17.3; 0.58, 40,000 x 120,000 (550,000) 13.6 -> 11.5.
+//   With two full rounds of chunks, 150,000 x 40,000 (355,000), 12.2 -> 14.3; with four fifths,
+//   76,000 x 30,000 (376,000), 12.5 -> 13.6.
 // - Every launch writes the numbered copy anew, and its 16 bytes an element no longer stay near:
 //   250,000 x 300,000 (1.2M) 19.0 -> 18.1, 223,000 x 487,000 (1M) 18.4 -> 20.2, 496,000 x 329,000 (1.3M)
 //   21.9 -> 29.2.
@@ -216,6 +221,9 @@ inline bool flow_pays(const TileCsrT<V>& A, const TileCsrT<V>& AT, int warps, bo
     if (std::max(A.share.streamed, AT.share.streamed) > A.nnz / 3 || A.nnz / kReaders > std::min(A.rows, A.cols)) return false;
     if (std::max(A.ntiles, AT.ntiles) <= warps) return true;
     const int elements = A.rows + A.cols, part = elements <= 300000 ? 4 : 10;
+    const TileCsrT<V>&less = A.ntiles <= AT.ntiles ? A : AT, &more = A.ntiles <= AT.ntiles ? AT : A;
+    if (less.ntiles <= warps && less.share.longest <= kShortRow && more.ntiles <= warps / 4 * 7 && more.share.tree <= A.nnz / 3 * 2)
+        return true;
     auto few_long = [&](const TileCsrT<V>& M) { return M.ntiles <= warps || M.share.tree <= M.nnz / part; };
     return few_long(A) && few_long(AT) && (adaptive ? A.nnz <= 1000000 && elements <= 250000 : A.nnz <= 3000000 && elements <= 600000);
 }
