@@ -87,6 +87,8 @@ SIZES = {
     "two rounds of light rows": (False, lambda i: rows_of(i, 150000, 40000, 1, 36, 0.04)),
     "four fifths in rows of 40": (False, lambda i: rows_of(i, 76000, 30000, 1, 40, 0.1)),
     "light rows and columns, two thirds in rows of 100": (False, lambda i: rows_of(i, 100000, 80000, 1, 100, 0.02)),
+    "long rows beside two rounds of columns": (False, lambda i: lp_with_row(i, 15000, 90000, 5)),
+    "a few long rows beside two rounds of columns": (True, lambda i: lp_with_row(i, 25000, 100000, 5)),
     "a dense row, 5,000 x 12,000": (False, lambda i: lp_with_row(i, 5000, 12000, 5, 12000)),
     "one chunk a warp, rows of 45": (True, lambda i: lp_with_row(i, 12000, 27000, 20)),
     "two chunks a warp, rows of 40": (False, lambda i: rows_of(i, 40000, 60000, 6, 40, 0.4)),

@@ -208,6 +208,8 @@ __device__ __forceinline__ T chunk_sum(const TileCsrT<V>& A, const ChunkRows& c,
 //   (443,000) 12.0 -> 9.5, 14.1 -> 11.5, 19.6 -> 17.3; 0.58, 40,000 x 120,000 (550,000) 13.6 -> 11.5.
 //   With two full rounds of chunks, 150,000 x 40,000 (355,000), 12.2 -> 14.3; with four fifths,
 //   76,000 x 30,000 (376,000), 12.5 -> 13.6.
+//   Long rows in that other matrix delay all: 15,000 x 90,000 (450,000), 0.38 in them, 11.6 -> 16.8, 15.9 -> 18.1,
+//   19.3 -> 25.3; 0.25, 30,000 x 90,000 (303,000) 10.2 -> 12.6; 0.07, 15,000 x 120,000 (360,000) 11.0 -> 10.1.
 // - Every launch writes the numbered copy anew, and its 16 bytes an element no longer stay near:
 //   250,000 x 300,000 (1.2M) 19.0 -> 18.1, 223,000 x 487,000 (1M) 18.4 -> 20.2, 496,000 x 329,000 (1.3M)
 //   21.9 -> 29.2.
@@ -224,7 +226,7 @@ inline bool flow_pays(const TileCsrT<V>& A, const TileCsrT<V>& AT, int warps, bo
     const TileCsrT<V>&less = A.ntiles <= AT.ntiles ? A : AT, &more = A.ntiles <= AT.ntiles ? AT : A;
     if (less.ntiles <= warps && less.share.longest <= kShortRow && more.ntiles <= warps / 4 * 7 && more.share.tree <= A.nnz / 3 * 2)
         return true;
-    auto few_long = [&](const TileCsrT<V>& M) { return M.ntiles <= warps || M.share.tree <= M.nnz / part; };
+    auto few_long = [&](const TileCsrT<V>& M) { return M.share.tree <= M.nnz / (M.ntiles <= warps ? 14 : part); };
     return few_long(A) && few_long(AT) && (adaptive ? A.nnz <= 1000000 && elements <= 250000 : A.nnz <= 3000000 && elements <= 600000);
 }
 
